@@ -1036,13 +1036,49 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
-// Pass B of one column: block = two 128-sample tiles of tiles_s, thread = one sample of
-// each (the limb words it loads serve both).  The marker limb planes are staged in
-// shared memory kSrChunk markers at a time.  With kLists the c planes give way to qc
-// itself (qc32), and after each chunk the block adds qc over the missing calls of its
-// 256 samples in the chunk — one segment of miss_ent, each entry (sample in block) <<
-// bits | (marker in chunk) — into per-sample int64 counters: the integer Mi the flag
-// sums give.
+// How one-column pass B divides the markers: units of kSrChunk / sub markers, `units`
+// of them per block, n_units in all, over `blocks` blocks per pair of sample tiles.
+struct SrSplitB {
+  int sub;
+  int64_t units, n_units;
+  unsigned blocks;
+};
+
+// The line: kSrBlocksB blocks per SM in all.  Fewer than that many (pair of tiles, chunk)
+// units: the chunks are divided (up to one 128-marker tile per unit) until there are;
+// more: a block takes several chunks, so that its planes' staging and its sums at the
+// end stay small beside the dense loop.
+constexpr int64_t kSrBlocksB = 24;
+
+SrSplitB sr_split_b(int64_t n_pad, int64_t m_pad) {
+  const int64_t pairs = n_pad / (2 * kRows), chunks = ceil_div(m_pad, (int64_t)kSrChunk);
+  const int64_t want = 148 * kSrBlocksB;
+  SrSplitB s;
+  s.sub = 1;
+  while (s.sub < kSrChunk / 128 && pairs * chunks * s.sub * 4 < want) s.sub *= 2;
+  s.n_units = ceil_div(m_pad, (int64_t)(kSrChunk / s.sub));
+  const int64_t blocks = std::max<int64_t>(1, std::min(s.n_units, want / pairs));
+  s.units = ceil_div(s.n_units, blocks);
+  s.blocks = (unsigned)ceil_div(s.n_units, s.units);
+  return s;
+}
+
+// Pass B of one column: block = two 128-sample tiles of tiles_s (thread = one sample of
+// each; the limb words it loads serve both) x a range of marker units.  A unit is a
+// chunk of kSrChunk markers or one of its `sub` equal parts; the unit's limb planes are
+// staged in shared memory.  With kLists the c planes give way to qc itself (qc32), and
+// the block adds qc over its part of the chunk's segment of missing calls — entries
+// (sample in block) << bits | (marker in chunk) — into per-sample int64 counters: the
+// integer Mi the flag sums give.
+//
+// Bound: integer issue (dp4a) once every SM has warps enough to hide the loads of the
+// codes.  The markers are split over blockIdx.y because a cohort's sample tiles alone do
+// not fill 148 SMs: at n = 9,001 they are 36 blocks of four warps, each walking all
+// m = 20,900 markers (331 us; 47 us split), and at n = 200,000, m = 150,000 they are 782
+// blocks, 5.3 per SM, where the SMs with six take 13 % longer (3.65 ms; 3.06 ms split).  The sums
+// are integers, so partial sums meet in sums_g / sums_m (int64 per sample, atomics) in any
+// order with the same result; the block that takes the last ticket of its sample tiles
+// runs the epilogue and leaves the sums and the ticket at zero for the next product.
 template <bool kLists>
 __global__ void __launch_bounds__(128)
     sr_pass_b_kernel(const uint8_t* __restrict__ tiles_s, int64_t n_mt, int64_t s_ld,
@@ -1051,7 +1087,10 @@ __global__ void __launch_bounds__(128)
                      const double* __restrict__ scale_w, const double* __restrict__ scale_c,
                      const int32_t* __restrict__ qc32, const uint32_t* __restrict__ miss_ent,
                      const int64_t* __restrict__ miss_seg, int64_t nch, int bits,
-                     unsigned int* __restrict__ err, double out_scale, double* __restrict__ out) {
+                     unsigned int* __restrict__ err, SrSplitB split,
+                     unsigned long long* __restrict__ sums_g,
+                     unsigned long long* __restrict__ sums_m, unsigned int* __restrict__ tickets,
+                     double out_scale, double* __restrict__ out) {
   constexpr int kPlanes = kLists ? 3 : 6;
   __shared__ __align__(16) int8_t sp[kPlanes][kSrChunk];
   __shared__ __align__(16) int32_t sq[kLists ? kSrChunk : 4];
@@ -1067,32 +1106,42 @@ __global__ void __launch_bounds__(128)
     mi_s[r] = 0ull;
     mi_s[kRows + r] = 0ull;
   }
-  for (int64_t mt0 = 0; mt0 < n_mt; mt0 += kSrChunk / 128) {
+  const int64_t tiles_per_unit = (kSrChunk / 128) / split.sub;
+  const int64_t u_end = min((int64_t)(blockIdx.y + 1) * split.units, split.n_units);
+  for (int64_t unit = (int64_t)blockIdx.y * split.units; unit < u_end; ++unit) {
+    const int64_t chunk = unit / split.sub;
+    const int part = (int)(unit - chunk * split.sub);
+    const int64_t mt0 = unit * tiles_per_unit;
     const int64_t base = mt0 * 128;
-    const int64_t len = m_pad - base < kSrChunk ? m_pad - base : (int64_t)kSrChunk;
-    int64_t e0 = 0, e1 = 0;  // kLists: this chunk's segment
+    const int64_t cbase = chunk * kSrChunk;  // kLists: the segment's positions count from here
+    const int len = (int)max((int64_t)0, min(m_pad - base, tiles_per_unit * 128));
+    const int clen = (int)min(m_pad - cbase, (int64_t)kSrChunk);
+    int64_t e0 = 0, e1 = 0;  // kLists: this unit's part of the chunk's segment
     if constexpr (kLists) {
-      const int64_t* sg = miss_seg + (int64_t)blockIdx.x * nch + mt0 / (kSrChunk / 128);
-      e0 = sg[0];
-      e1 = sg[1];
+      const int64_t* sg = miss_seg + (int64_t)blockIdx.x * nch + chunk;
+      // the last chunk may have fewer parts than sub
+      const int64_t left = split.n_units - chunk * split.sub;
+      const int64_t parts = left < split.sub ? left : split.sub;
+      const int64_t s0 = sg[0], cnt = sg[1] - sg[0];
+      e0 = s0 + cnt * part / parts;
+      e1 = s0 + cnt * (part + 1) / parts;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < kPlanes * (kSrChunk / 16); t += 128) {
       const int pl = t / (kSrChunk / 16), k = t % (kSrChunk / 16);
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (16 * k < len)
-        v = __ldg(reinterpret_cast<const uint4*>(planes + (int64_t)pl * m_pad + base) + k);
-      reinterpret_cast<uint4*>(sp[pl])[k] = v;
+        reinterpret_cast<uint4*>(sp[pl])[k] =
+            __ldg(reinterpret_cast<const uint4*>(planes + (int64_t)pl * m_pad + base) + k);
     }
     if constexpr (kLists) {
       for (int t = threadIdx.x; t < kSrChunk / 4; t += 128) {
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (4 * t < len) v = __ldg(reinterpret_cast<const uint4*>(qc32 + base) + t);
+        if (4 * t < clen) v = __ldg(reinterpret_cast<const uint4*>(qc32 + cbase) + t);
         reinterpret_cast<uint4*>(sq)[t] = v;
       }
     }
     __syncthreads();
-    const int64_t mt_end = mt0 + kSrChunk / 128 < n_mt ? mt0 + kSrChunk / 128 : n_mt;
+    const int64_t mt_end = mt0 + len / 128;
 #pragma unroll 2
     for (int64_t mt = mt0; mt < mt_end; ++mt) {
       uint32_t words[2][8];
@@ -1151,23 +1200,56 @@ __global__ void __launch_bounds__(128)
       }
     }
     if constexpr (kLists) {
-      add_slice(miss_ent, e0, e1, threadIdx.x, 128, bits, 2u * kRows, (uint32_t)len, mi_s, err,
+      add_slice(miss_ent, e0, e1, threadIdx.x, 128, bits, 2u * kRows, (uint32_t)clen, mi_s, err,
                 [&](uint32_t mk) { return (long long)sq[mk]; });
     }
   }
   if constexpr (kLists) __syncthreads();
+  // this block's integer sums per sample: G (formed with -g) and Mi
+  long long g[2], mi[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    g[h] = 65536LL * acc[h][0] + 256LL * acc[h][1] + (long long)acc[h][2];
+    if constexpr (kLists)
+      mi[h] = (long long)mi_s[h * kRows + r];
+    else
+      mi[h] = 65536LL * acc[h][kPlanes - 3] + 256LL * acc[h][kPlanes - 2] +
+              (long long)acc[h][kPlanes - 1];
+  }
+  if (gridDim.y > 1) {
+    __shared__ int last_s;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t i = (st0 + h) * 128 + r;
+      atomicAdd(&sums_g[i], (unsigned long long)g[h]);
+      atomicAdd(&sums_m[i], (unsigned long long)mi[h]);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const bool last = atomicAdd(&tickets[blockIdx.x], 1u) == gridDim.y - 1;
+      if (last) tickets[blockIdx.x] = 0u;
+      last_s = last ? 1 : 0;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t i = (st0 + h) * 128 + r;
+      g[h] = (long long)__ldcg(&sums_g[i]);
+      mi[h] = (long long)__ldcg(&sums_m[i]);
+      sums_g[i] = 0ull;
+      sums_m[i] = 0ull;
+    }
+  }
   const double S = (double)(long long)sum_c[0];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    // the genotype sums were formed with -g; Mi is the same integer either way
-    const double G =
-        -(65536.0 * (double)acc[h][0] + 256.0 * (double)acc[h][1] + (double)acc[h][2]);
-    double Mi;
-    if constexpr (kLists)
-      Mi = (double)(long long)mi_s[h * kRows + r];
-    else
-      Mi = 65536.0 * (double)acc[h][kPlanes - 3] + 256.0 * (double)acc[h][kPlanes - 2] +
-           (double)acc[h][kPlanes - 1];
+    // both integers are below 2^53: exact in FP64, as the limb sums of the tensor-core
+    // epilogue are
+    const double G = -(double)g[h];
+    const double Mi = (double)mi[h];
     out[(st0 + h) * 128 + r] = __dmul_rn(
         out_scale, __dsub_rn(__dmul_rn(scale_w[0], G), __dmul_rn(scale_c[0], S - Mi)));
   }
@@ -1230,6 +1312,7 @@ struct TcPlan {
   // sums over them
   MissLists miss;
   DevBuf sr_qc;
+  DevBuf sr_sums;  // pass B's sums over its marker splits and its tickets: zero between products
 };
 
 // The missing-call lists cost about two products' time to build (four passes over the
@@ -1698,18 +1781,29 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
         u, h->m_pad, h->inv_s, h->two_p, sc.amax_w, sc.amax_c, sc.scale_w, sc.scale_c, planes_b,
         qc32, sc.sum_c);
     // two sample tiles per block (n_pad is a multiple of 512: an even tile count)
-    const unsigned grid_b = (unsigned)(h->n_pad / (2 * kRows));
+    const SrSplitB split = sr_split_b(h->n_pad, h->m_pad);
+    const unsigned pairs = (unsigned)(h->n_pad / (2 * kRows));
+    const dim3 grid_b(pairs, split.blocks);
+    if (split.blocks > 1 && !p->sr_sums.ptr) {
+      const size_t bytes = (size_t)h->n_pad * 16 + (size_t)pairs * 4;
+      SG_TRY(p->sr_sums.reserve(bytes));
+      SG_CUDA(cudaMemsetAsync(p->sr_sums.ptr, 0, bytes, st));
+    }
+    unsigned long long* sums = p->sr_sums.as<unsigned long long>();
+    unsigned int* tickets = reinterpret_cast<unsigned int*>(sums + 2 * h->n_pad);
     const double out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
     double* out = kp + (int64_t)cols[0] * h->n_pad;
     if (lists)
       sr_pass_b_kernel<true><<<grid_b, kRows, 0, st>>>(
           p->tiles_s.as<uint8_t>(), h->m_pad / kRows, p->s_ld, planes_b, h->m_pad, sc.sum_c,
           sc.scale_w, sc.scale_c, qc32, p->miss.b_ent.as<uint32_t>(), p->miss.b_seg.as<int64_t>(),
-          p->miss.b_nch, p->miss.b_bits, sc.err, out_scale, out);
+          p->miss.b_nch, p->miss.b_bits, sc.err, split, sums, sums + h->n_pad, tickets, out_scale,
+          out);
     else
       sr_pass_b_kernel<false><<<grid_b, kRows, 0, st>>>(
           p->tiles_s.as<uint8_t>(), h->m_pad / kRows, p->s_ld, planes_b, h->m_pad, sc.sum_c,
-          sc.scale_w, sc.scale_c, nullptr, nullptr, nullptr, 0, 0, nullptr, out_scale, out);
+          sc.scale_w, sc.scale_c, nullptr, nullptr, nullptr, 0, 0, nullptr, split, sums,
+          sums + h->n_pad, tickets, out_scale, out);
     SG_CHECK_LAUNCH();
     count_launches(6);
     SG_TRY(mark(&t1));
