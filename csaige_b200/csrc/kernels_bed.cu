@@ -16,6 +16,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int64_t kSmemRowMax = 200 * 1024;  // stage raw rows up to this size in shared memory
+constexpr int64_t kSmemHalf = 112 * 1024;    // shared memory of one of two blocks on an SM
 
 // Counts over a word of 16 codes; valid = even bits of the real samples.
 __device__ __forceinline__ void count_word(uint32_t w, uint32_t valid, long long& alt,
@@ -53,8 +54,8 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 // row, at most two, are copied byte by byte, so no load leaves the row.  Several
 // independent chunk loads per thread are in flight at once.  Returns row_s + off.
 // row_s holds round_up(bpm + 16, 16) bytes, 16-byte aligned.
-__device__ __forceinline__ const uint8_t* stage_row(const uint8_t* row, int64_t bpm,
-                                                    uint8_t* row_s) {
+__device__ __forceinline__ const uint8_t* copy_row(const uint8_t* row, int64_t bpm,
+                                                   uint8_t* row_s) {
   const int off = (int)(reinterpret_cast<uintptr_t>(row) & 15u);
   const uint4* base = reinterpret_cast<const uint4*>(row - off);
   const int64_t n16 = (off + bpm + 15) / 16;
@@ -70,8 +71,15 @@ __device__ __forceinline__ const uint8_t* stage_row(const uint8_t* row, int64_t 
       }
     }
   }
-  __syncthreads();
   return row_s + off;
+}
+
+// copy_row by the whole block, then the barrier that makes the row readable.
+__device__ __forceinline__ const uint8_t* stage_row(const uint8_t* row, int64_t bpm,
+                                                    uint8_t* row_s) {
+  const uint8_t* p = copy_row(row, bpm, row_s);
+  __syncthreads();
+  return p;
 }
 
 // The codes of samples sidx[0 .. kn) (kn <= 16) of a raw row as one PLINK-order
@@ -102,64 +110,206 @@ __device__ __forceinline__ uint32_t gather_word(const uint8_t* src, const int32_
   return word;
 }
 
-template <bool kIdentity>
-__global__ void __launch_bounds__(kThreads)
-    bed_gather_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
-                      const int64_t* __restrict__ src_rows, const int32_t* __restrict__ sidx,
-                      int64_t n, uint32_t* __restrict__ out, int64_t wpr,
-                      int64_t* __restrict__ counts, int use_smem) {
-  extern __shared__ __align__(16) uint8_t row_s[];
-  __shared__ long long red[2][kThreads / 32];
-  const int64_t r = blockIdx.x;
-  const uint8_t* row = bed + 3 + src_rows[r] * bpm;
-  const uint8_t* src = use_smem ? stage_row(row, bpm, row_s) : row;
-  const bool sidx16 = (reinterpret_cast<uintptr_t>(sidx) & 15u) == 0;
-  long long alt = 0, miss = 0;
-  const int64_t n_words_real = (n + 15) / 16;
-  const int64_t n_words = out ? wpr : n_words_real;
-  for (int64_t j = threadIdx.x; j < n_words; j += blockDim.x) {
-    // Padding samples are coded 11 (genotype 0, not missing): every vector the
-    // products read is zero there, so they contribute nothing to any sum.
-    uint32_t w = 0xFFFFFFFFu;
-    if (j < n_words_real) {
-      const int64_t k0 = j * 16;
-      const int kn = (n - k0) < 16 ? (int)(n - k0) : 16;
-      uint32_t word = 0;
-      if (kIdentity) {
-        // bytes 4j .. 4j+3 of the raw row hold exactly these samples
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int64_t bi = 4 * j + b;
-          const uint32_t byte = bi < bpm ? (uint32_t)src[bi] : 0u;
-          word |= byte << (8 * b);
-        }
-      } else {
-        word = gather_word(src, sidx + k0, kn, kn == 16 && sidx16);
-      }
-      const uint32_t keep = kn >= 16 ? 0xFFFFFFFFu : ((1u << (2 * kn)) - 1u);
-      count_word(word, keep & 0x55555555u, alt, miss);
-      // padding samples are coded 11, then the word is re-laid out
-      w = to_device_layout((word & keep) | ~keep);
-    }
-    if (out) out[r * wpr + j] = w;
-  }
-  if (!counts) return;
+// A row's counts from its threads' counts: kGroup threads (one warp, or the whole block
+// of kThreads) share a row; thread 0 of the group writes.
+template <int kGroup>
+__device__ __forceinline__ void store_counts(long long alt, long long miss, int64_t* out) {
   alt = warp_sum_ll(alt);
   miss = warp_sum_ll(miss);
+  const int lane = threadIdx.x & 31;
+  if constexpr (kGroup == 32) {
+    if (lane == 0) {
+      out[0] = alt;
+      out[1] = miss;
+    }
+  } else {
+    __shared__ long long red[2][kGroup / 32];
+    const int wid = threadIdx.x >> 5;
+    if (lane == 0) {
+      red[0][wid] = alt;
+      red[1][wid] = miss;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      long long a = 0, mm = 0;
+      for (int k = 0; k < kGroup / 32; ++k) {
+        a += red[0][k];
+        mm += red[1][k];
+      }
+      out[0] = a;
+      out[1] = mm;
+    }
+  }
+}
+
+// All samples in .fam order: word j of a packed row is bytes 4j .. 4j+3 of the raw row,
+// whose start (3 + row bpm) is not aligned, so a word is cut out of the two aligned words
+// around it.  The aligned word in front starts at most 3 bytes before the row, still inside
+// the .bed (the header is 3 bytes); the words near the row's end, whose aligned words
+// would reach past it, are read byte by byte.  kGroup threads per row: a warp for short
+// rows, the block for long ones.
+// Bound: issue, about 20 instructions per 16 samples, three of them population counts
+// at half rate, beside DRAM.  The counts come from three sums over the code bits (both
+// planes together, the low plane, and their product).  40,000 rows of 200,000 samples:
+// counts 1.35 ms with a byte per load, 64-bit counters and every word handled as if it
+// were the last; now 0.48 ms with a block per row, 0.39 ms with a warp (5.1 TB/s).
+template <int kGroup, bool kOut, bool kCounts>
+__global__ void __launch_bounds__(kThreads)
+    bed_rows_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
+                    const int64_t* __restrict__ src_rows, int64_t n_rows, int64_t n,
+                    uint32_t* __restrict__ out, int64_t wpr, int64_t* __restrict__ counts) {
+  const int64_t r = (int64_t)blockIdx.x * (kThreads / kGroup) + threadIdx.x / kGroup;
+  if (r >= n_rows) return;  // whole warps (kGroup 32) or, never, whole blocks
+  const uint8_t* row = bed + 3 + src_rows[r] * bpm;
+  const int off = (int)(reinterpret_cast<uintptr_t>(row) & 3u);
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(row - off);
+  uint32_t* dst = kOut ? out + r * wpr : nullptr;
+  // words of 16 samples whose two aligned words end inside the row (n < 2^31: n_words < 2^27)
+  const int n_words = (int)(kOut ? wpr : (n + 15) / 16);
+  const int64_t safe = bpm + off >= 8 ? (bpm + off - 8) / 4 + 1 : 0;
+  const int n_fast = (int)(safe < n / 16 ? safe : n / 16);
+  uint32_t both = 0, low = 0, prod = 0;  // over the fast words: set bits, low bits, 11 codes
+  int j = threadIdx.x % kGroup;
+  const int first = j;
+#pragma unroll 8
+  for (; j < n_fast; j += kGroup) {
+    const uint32_t w = __funnelshift_r(__ldg(base + j), __ldg(base + j + 1), 8 * off);
+    if (kCounts) {
+      const uint32_t lo = w & 0x55555555u;
+      both += __popc(w);
+      low += __popc(lo);
+      prod += __popc(lo & (w >> 1));
+    }
+    if (kOut) dst[j] = to_device_layout(w);
+  }
+  long long alt = 0, miss = 0;
+  if (kCounts) {
+    // per code: 00 two alternative alleles, 10 (high bit alone) one, 01 missing
+    const int fast = n_fast > first ? (n_fast - first + kGroup - 1) / kGroup : 0;
+    const long long high = (long long)both - low;
+    alt = 32LL * fast - 2LL * low - high + (long long)prod;
+    miss = (long long)low - (long long)prod;
+  }
+  for (; j < n_words; j += kGroup) {
+    // Padding samples are coded 11 (genotype 0, not missing): every vector the
+    // products read is zero there, so they contribute nothing to any sum.
+    const int64_t left = n - 16 * (int64_t)j;
+    uint32_t w = 0xFFFFFFFFu;
+    if (left > 0) {
+      uint32_t word = 0;
+      for (int b = 0; b < 4; ++b) {
+        const int64_t bi = 4 * (int64_t)j + b;
+        if (bi < bpm) word |= (uint32_t)row[bi] << (8 * b);
+      }
+      const uint32_t keep = left >= 16 ? 0xFFFFFFFFu : ((1u << (2 * (int)left)) - 1u);
+      if (kCounts) count_word(word, keep & 0x55555555u, alt, miss);
+      w = to_device_layout((word & keep) | ~keep);
+    }
+    if (kOut) dst[j] = w;
+  }
+  if (kCounts) store_counts<kGroup>(alt, miss, counts + 2 * r);
+}
+
+// A sample subset, kRows raw rows per block staged in shared memory (kRows = 0: one row,
+// read from global memory, for rows too long to stage): each thread loads the 16 sample
+// indices of a packed word once and gathers that word from every staged row.  Bound: the
+// index loads (64 bytes from L2 per 4-byte word and row with a row per block) and the bank
+// conflicts of the byte gathers.  40,000 rows of 60,013 of 150,001 samples: 2.10 ms with a
+// row per block, 1.59 ms with three.  (Lane = sample with two ballots per 32 samples has no
+// bank conflicts but took 2.37 ms: the votes bound it.)
+constexpr int kSubsetThreads = 512;
+
+template <int kRows>
+__global__ void __launch_bounds__(kSubsetThreads, 2)
+    bed_subset_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
+                      const int64_t* __restrict__ src_rows, int64_t n_rows,
+                      const int32_t* __restrict__ sidx, int64_t n, uint32_t* __restrict__ out,
+                      int64_t wpr, int64_t* __restrict__ counts) {
+  constexpr int R = kRows ? kRows : 1;
+  extern __shared__ __align__(16) uint8_t row_s[];
+  __shared__ int red[2 * R][kSubsetThreads / 32];
+  const int64_t r0 = (int64_t)blockIdx.x * R;
+  const int nr = n_rows - r0 < R ? (int)(n_rows - r0) : R;
+  const int64_t stride = (bpm + 31) / 16 * 16;  // round_up(bpm + 16, 16)
+  const uint8_t* src[R];
+  const uint8_t* raw[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) raw[q] = bed + 3 + src_rows[r0 + (q < nr ? q : 0)] * bpm;
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+    src[q] = kRows ? copy_row(raw[q], bpm, row_s + q * stride) : raw[q];
+  if (kRows) __syncthreads();
+  const bool vec = (reinterpret_cast<uintptr_t>(sidx) & 15u) == 0;
+  const int64_t n_real = (n + 15) / 16;
+  const int64_t n_words = out ? wpr : n_real;
+  int alt[R], miss[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) alt[q] = miss[q] = 0;
+  for (int64_t j = threadIdx.x; j < n_words; j += kSubsetThreads) {
+    uint32_t w[R];
+    if (j < n_real) {
+      const int64_t k0 = 16 * j;
+      const int kn = n - k0 < 16 ? (int)(n - k0) : 16;
+#pragma unroll
+      for (int q = 0; q < R; ++q) w[q] = 0u;
+      if (vec && kn == 16) {
+        const int4* s4 = reinterpret_cast<const int4*>(sidx + k0);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int4 v = __ldg(s4 + g);
+          const int32_t ss[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int at = ss[e] >> 2, sh = (ss[e] & 3) * 2;
+#pragma unroll
+            for (int q = 0; q < R; ++q)
+              w[q] |= (((uint32_t)src[q][at] >> sh) & 3u) << (2 * (4 * g + e));
+          }
+        }
+      } else {
+        for (int k = 0; k < kn; ++k) {
+          const int32_t s = sidx[k0 + k];
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+            w[q] |= (((uint32_t)src[q][s >> 2] >> ((s & 3) * 2)) & 3u) << (2 * k);
+        }
+      }
+      const uint32_t keep = kn >= 16 ? 0xFFFFFFFFu : ((1u << (2 * kn)) - 1u);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        long long a = 0, mm = 0;
+        count_word(w[q], keep & 0x55555555u, a, mm);
+        alt[q] += (int)a;
+        miss[q] += (int)mm;
+        w[q] = to_device_layout((w[q] & keep) | ~keep);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < R; ++q) w[q] = 0xFFFFFFFFu;
+    }
+    if (out) {
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (q < nr) out[(r0 + q) * wpr + j] = w[q];
+    }
+  }
+  if (!counts) return;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    red[0][wid] = alt;
-    red[1][wid] = miss;
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    // a warp's counts (at most n / 8) fit in 32 bits, a row's need not
+    const int a = __reduce_add_sync(0xffffffffu, alt[q]);
+    const int mm = __reduce_add_sync(0xffffffffu, miss[q]);
+    if (lane == 0) {
+      red[2 * q][wid] = a;
+      red[2 * q + 1][wid] = mm;
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    long long a = 0, mm = 0;
-    for (int k = 0; k < kThreads / 32; ++k) {
-      a += red[0][k];
-      mm += red[1][k];
-    }
-    counts[2 * r] = a;
-    counts[2 * r + 1] = mm;
+  if (threadIdx.x < 2 * nr) {
+    long long s = 0;
+    for (int k = 0; k < kSubsetThreads / 32; ++k) s += red[threadIdx.x][k];
+    counts[2 * r0 + threadIdx.x] = s;
   }
 }
 
@@ -328,21 +478,51 @@ cudaError_t launch_bed_gather(const uint8_t* bed, int64_t bpm, const int64_t* sr
                               int64_t n_rows, const int32_t* sample_idx, int64_t n,
                               uint32_t* geno_out, int64_t words_per_row, int64_t* counts,
                               cudaStream_t st) {
-  if (n_rows <= 0) return cudaSuccess;
-  const int use_smem = bpm <= kSmemRowMax ? 1 : 0;
-  const size_t smem = use_smem ? (size_t)round_up(bpm + 16, 16) : 0;
+  if (n_rows <= 0 || (!geno_out && !counts)) return cudaSuccess;
   if (sample_idx) {
-    auto k = bed_gather_kernel<false>;
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    k<<<(unsigned)n_rows, kThreads, smem, st>>>(bed, bpm, src_rows, sample_idx, n, geno_out,
-                                                words_per_row, counts, use_smem);
+    // as many rows per block as half an SM's shared memory holds (two blocks of 16 warps
+    // per SM, so that one stages while the other gathers), at most four; a row beyond
+    // that, up to kSmemRowMax, has the SM to itself
+    const int64_t stride = round_up(bpm + 16, 16);
+    const int64_t fit = kSmemHalf / stride;
+    const int rows = bpm > kSmemRowMax ? 0 : (fit >= 4 ? 4 : (fit >= 2 ? (int)fit : 1));
+    auto go = [&](auto kern, int per) -> cudaError_t {
+      const size_t smem = rows ? (size_t)(stride * rows) : 0;
+      if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (e != cudaSuccess) return e;
+      }
+      kern<<<(unsigned)ceil_div(n_rows, (int64_t)per), kSubsetThreads, smem, st>>>(
+          bed, bpm, src_rows, n_rows, sample_idx, n, geno_out, words_per_row, counts);
+      return cudaGetLastError();
+    };
+    cudaError_t e = rows == 4   ? go(bed_subset_kernel<4>, 4)
+                    : rows == 3 ? go(bed_subset_kernel<3>, 3)
+                    : rows == 2 ? go(bed_subset_kernel<2>, 2)
+                    : rows == 1 ? go(bed_subset_kernel<1>, 1)
+                                : go(bed_subset_kernel<0>, 1);
+    count_launches(1);
+    return e;
+  }
+  // identity subset: a warp per row when the rows are short or enough for the chip, else
+  // the block (256 threads on a row of 1,250 words leave a fifth of their steps empty and
+  // add a block reduction: 100,000 rows of 20,000 samples 319 us, with warps 126 us; few
+  // long rows would leave SMs idle; long rows that are also written: 40,000 rows of 200,000
+  // samples 0.69 ms with blocks, 0.78 ms with warps)
+  const bool shortrow = bpm <= 2048 || (n_rows >= 148 * 16 && (!geno_out || bpm <= 16 * 1024));
+  const unsigned grid = (unsigned)(shortrow ? ceil_div(n_rows, (int64_t)(kThreads / 32)) : n_rows);
+  auto go = [&](auto kern) {
+    kern<<<grid, kThreads, 0, st>>>(bed, bpm, src_rows, n_rows, n, geno_out, words_per_row, counts);
+  };
+  if (shortrow) {
+    if (geno_out && counts) go(bed_rows_kernel<32, true, true>);
+    else if (geno_out) go(bed_rows_kernel<32, true, false>);
+    else go(bed_rows_kernel<32, false, true>);
   } else {
-    // identity subset: no staging needed, bytes are read in order
-    bed_gather_kernel<true><<<(unsigned)n_rows, kThreads, 0, st>>>(
-        bed, bpm, src_rows, nullptr, n, geno_out, words_per_row, counts, 0);
+    if (geno_out && counts) go(bed_rows_kernel<kThreads, true, true>);
+    else if (geno_out) go(bed_rows_kernel<kThreads, true, false>);
+    else go(bed_rows_kernel<kThreads, false, true>);
   }
   count_launches(1);
   return cudaGetLastError();

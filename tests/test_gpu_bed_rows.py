@@ -40,6 +40,15 @@ def test_counts_of_all_samples(n, m):
         assert all(np.array_equal(a, b) for a, b in zip(got, want)), shift
 
 
+@pytest.mark.parametrize("n", [8197, 70001])
+def test_counts_of_many_long_rows(n):
+    # enough rows for a warp each (2,368 and more) although they are long
+    bed = _bed(n, 2370, n)
+    want = O.marker_stats(bed, n, 2370, None)
+    got = _stats_at(bed, 1, n, 2370, None)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
 # rows staged per block: 4 (short rows), 3, 2, 1 (half and whole SM), 0 (read in place)
 @pytest.mark.parametrize("n_fam", [50, 20003, 120001, 150001, 200003, 300001, 500003, 830003])
 @pytest.mark.parametrize("m", [1, 6])
