@@ -8,8 +8,7 @@
 namespace saige {
 namespace {
 
-constexpr int kG = 32;        // Gram tile (32 x 32 outputs per block)
-constexpr int kGThreads = 256;
+constexpr int kG = 32;  // Gram: rows per stage; the chunks of rows are counted in 32 x 32 tiles
 
 int gram_chunks(int64_t n, int a, int b) {
   const int tiles = ((a + kG - 1) / kG) * ((b + kG - 1) / kG);
@@ -18,39 +17,102 @@ int gram_chunks(int64_t n, int a, int b) {
   return (int)std::max<int64_t>(1, std::min(by_rows, want));
 }
 
-// Block (chunk x, tile y): rows [x*chunk, (x+1)*chunk) of the 32 x 32 output tile y.
-__global__ void __launch_bounds__(kGThreads)
+// 16 bytes global -> shared (cp.async); bytes past `valid` (0, 8 or 16) are zero.
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, int valid) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(valid)
+               : "memory");
+}
+
+// Block (chunk x, tile y): the sums over rows [x*chunk, (x+1)*chunk) of output tile y,
+// 8R x 8R entries, 8 x 8 threads of R x R.  Each entry is one chain of fused multiply-adds
+// in row order (a start's coefficients are sensitive to the last bit, so neither the
+// chains nor the chunks may depend on the tile), which sets the pace: 32 rows are staged
+// column by column while the ones before them are multiplied (cp.async, 8 / R buffers; column
+// pitch 34 doubles: the eight columns that a quarter warp reads lie in different banks),
+// and two rows are read per 16-byte load.
+// Bound: the FP64 pipe for many rows and columns (R = 4: 16 chains per thread), the
+// latency of the chains and of the stages' loads for few (R = 2, four times the blocks).  With 32 x 32 tiles of 256
+// threads, unstaged loads and five 8-byte shared loads per four multiply-adds: 302 us at
+// n = 200,000 (bases of up to about 120 columns, mean of a fit's ten) and 123 us at n = 2,000;
+// now 158 and 29 us.
+constexpr int kGramPitch = kG + 2;
+
+template <int R>
+__global__ void __launch_bounds__(64)
     gram_kernel(const double* __restrict__ A, int a, const double* __restrict__ B, int b,
                 int64_t n, int64_t ld, int64_t chunk, double* __restrict__ partial) {
-  __shared__ double as[kG][kG + 1], bs[kG][kG + 1];
-  const int tiles_b = (b + kG - 1) / kG;
-  const int ta = blockIdx.y / tiles_b, tb = blockIdx.y % tiles_b;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // ty 0..7
+  constexpr int kTile = 8 * R, kStages = 8 / R;
+  __shared__ __align__(16) double as[kStages][kTile][kGramPitch], bs[kStages][kTile][kGramPitch];
+  const int tiles_b = (b + kTile - 1) / kTile;
+  const int i0 = (blockIdx.y / tiles_b) * kTile, j0 = (blockIdx.y % tiles_b) * kTile;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   const int64_t lo = (int64_t)blockIdx.x * chunk;
   const int64_t hi = lo + chunk < n ? lo + chunk : n;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int64_t r0 = lo; r0 < hi; r0 += kG) {
-    const int64_t row = r0 + tx;
+  // stage rows r0 .. r0+31 of the tile's columns, 16 pieces of two rows per column; rows
+  // past hi and columns past the end are zero.  A thread takes piece pc of the columns
+  // c0 + 4k of both operands: their addresses differ by a constant.
+  const int pc = threadIdx.x & 15, c0 = threadIdx.x >> 4;
+  const double* const pa = A + (int64_t)(i0 + c0) * ld + 2 * pc;
+  const double* const pb = B + (int64_t)(j0 + c0) * ld + 2 * pc;
+  const int na = a - i0 - c0, nb = b - j0 - c0;  // column 4k exists when 4k < na (nb)
+  auto stage = [&](int buf, int64_t r0) {
+    const int64_t left = hi - (r0 + 2 * pc);
+    const int rows = left >= 2 ? 16 : (left == 1 ? 8 : 0);
 #pragma unroll
-    for (int k = ty; k < kG; k += 8) {
-      const int ca = ta * kG + k, cb = tb * kG + k;
-      as[tx][k] = (ca < a && row < hi) ? A[(int64_t)ca * ld + row] : 0.0;
-      bs[tx][k] = (cb < b && row < hi) ? B[(int64_t)cb * ld + row] : 0.0;
+    for (int k = 0; k < 2 * R; ++k) {
+      const bool in = 4 * k < na && rows > 0;
+      cp_async16_zfill(&as[buf][c0 + 4 * k][2 * pc], in ? pa + 4 * k * ld + r0 : A, in ? rows : 0);
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int r = 0; r < kG; ++r) {
-      const double bv = bs[r][tx];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] += as[r][ty + 8 * k] * bv;
+    for (int k = 0; k < 2 * R; ++k) {
+      const bool in = 4 * k < nb && rows > 0;
+      cp_async16_zfill(&bs[buf][c0 + 4 * k][2 * pc], in ? pb + 4 * k * ld + r0 : A, in ? rows : 0);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[R][R];
+#pragma unroll
+  for (int k = 0; k < R; ++k)
+#pragma unroll
+    for (int l = 0; l < R; ++l) acc[k][l] = 0.0;
+  // kStages - 1 stages ahead; an empty group where there is no further stage keeps the
+  // count of groups in flight the same
+  auto ahead = [&](int buf, int64_t r0) {
+    if (r0 < hi) stage(buf, r0);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < kStages - 1; ++k) ahead(k, lo + k * kG);
+  int buf = 0;
+  for (int64_t r0 = lo; r0 < hi; r0 += kG, buf = buf + 1 == kStages ? 0 : buf + 1) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();  // stage r0 has landed, and every thread is done with the one before
+    ahead(buf == 0 ? kStages - 1 : buf - 1, r0 + (kStages - 1) * kG);
+#pragma unroll
+    for (int r = 0; r < kG; r += 2) {
+      double2 x[R], y[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) x[k] = *reinterpret_cast<const double2*>(&as[buf][ty + 8 * k][r]);
+#pragma unroll
+      for (int l = 0; l < R; ++l) y[l] = *reinterpret_cast<const double2*>(&bs[buf][tx + 8 * l][r]);
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+#pragma unroll
+        for (int l = 0; l < R; ++l) acc[k][l] = fma(x[k].x, y[l].x, acc[k][l]);
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+#pragma unroll
+        for (int l = 0; l < R; ++l) acc[k][l] = fma(x[k].y, y[l].y, acc[k][l]);
+    }
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int i = ta * kG + ty + 8 * k, j = tb * kG + tx;
-    if (i < a && j < b) partial[((int64_t)i * b + j) * gridDim.x + blockIdx.x] = acc[k];
-  }
+  for (int k = 0; k < R; ++k)
+#pragma unroll
+    for (int l = 0; l < R; ++l) {
+      const int i = i0 + ty + 8 * k, j = j0 + tx + 8 * l;
+      if (i < a && j < b) partial[((int64_t)i * b + j) * gridDim.x + blockIdx.x] = acc[k][l];
+    }
 }
 
 // out[e] = sum over chunks, in chunk order.
@@ -233,9 +295,14 @@ cudaError_t gram(const double* A, int a, const double* B, int b, int64_t n, int6
                  double* partial, double* out, cudaStream_t st) {
   const int nch = gram_chunks(n, a, b);
   const int64_t chunk = round_up(ceil_div(n, nch), kG);
-  const int tiles = ((a + kG - 1) / kG) * ((b + kG - 1) / kG);
-  gram_kernel<<<dim3((unsigned)nch, (unsigned)tiles), kGThreads, 0, st>>>(A, a, B, b, n, ld, chunk,
-                                                                           partial);
+  // 32 x 32 tiles while they give every SM two blocks, else 16 x 16
+  const int64_t tiles4 = ceil_div(a, 32) * ceil_div(b, 32);
+  if (tiles4 * nch >= 296)
+    gram_kernel<4><<<dim3((unsigned)nch, (unsigned)tiles4), 64, 0, st>>>(A, a, B, b, n, ld, chunk,
+                                                                          partial);
+  else
+    gram_kernel<2><<<dim3((unsigned)nch, (unsigned)(ceil_div(a, 16) * ceil_div(b, 16))), 64, 0, st>>>(
+        A, a, B, b, n, ld, chunk, partial);
   const int64_t count = (int64_t)a * b;
   gram_reduce<<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(partial, nch, count, out);
   count_launches(2);
