@@ -375,9 +375,14 @@ Status bed_gather_dev(const uint8_t* bed_dev, int64_t n_fam, const std::vector<i
 // ---------------------------------------------------------------------------
 static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
                                const int32_t* active, cudaStream_t st) {
-  SG_TRY(h->v32.reserve((size_t)h->n_pad * sizeof(float)));
-  SG_TRY(h->u32.reserve((size_t)h->m_pad * sizeof(float)));
-  SG_TRY(h->ypart.reserve((size_t)h->n_splits * h->n_pad * sizeof(float)));
+  std::vector<int> act;
+  for (int c = 0; c < q; ++c)
+    if (!active || active[c] == kColActive) act.push_back(c);
+  // the active columns in groups of up to kFp32Cols that share one decode of the codes
+  const size_t group = std::min<size_t>(std::max<size_t>(act.size(), 1), kFp32Cols);
+  SG_TRY(h->v32.reserve(group * h->n_pad * sizeof(float)));
+  SG_TRY(h->u32.reserve(group * h->m_pad * sizeof(float)));
+  SG_TRY(h->ypart.reserve(std::min<size_t>(group, kFp32ColsB) * h->n_splits * h->n_pad * sizeof(float)));
   const float scale = 1.0f / (float)(h->masked ? h->m_active : h->m_eff);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->profiling) {
@@ -385,23 +390,32 @@ static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
     SG_CUDA(cudaEventCreate(&e1));
     SG_CUDA(cudaEventRecord(e0, st));
   }
-  int64_t done = 0;
-  for (int c = 0; c < q; ++c) {
-    if (active && active[c] != kColActive) continue;
-    const double* vc = v + (int64_t)c * h->n_pad;
-    double* oc = kp + (int64_t)c * h->n_pad;
-    SG_CUDA(launch_to_f32(vc, h->n, h->n_pad, h->v32.as<float>(), st));
-    SG_CUDA(launch_fp32_zt(h->geno, h->wpr, h->zlut, h->m_pad, h->v32.as<float>(),
-                           h->u32.as<float>(), st));
-    if (h->masked) SG_CUDA(mask_rows_f32(h->u32.as<float>(), h->excl.as<uint8_t>(), h->m, st));
-    SG_CUDA(launch_fp32_z(h->geno, h->wpr, h->zlut, h->m_pad, h->u32.as<float>(),
-                          h->ypart.as<float>(), h->n_splits, st));
-    SG_CUDA(launch_fp32_finish(h->ypart.as<float>(), h->n_splits, h->n_pad, h->n, scale, oc, st));
-    h->n_kv += 1;
-    ++done;
+  for (size_t c0 = 0; c0 < act.size(); c0 += kFp32Cols) {
+    const int nc = (int)std::min<size_t>(kFp32Cols, act.size() - c0);
+    Fp32Cols cols{};
+    for (int k = 0; k < nc; ++k) {
+      cols.v[k] = v + (int64_t)act[c0 + k] * h->n_pad;
+      cols.out[k] = kp + (int64_t)act[c0 + k] * h->n_pad;
+    }
+    float* u = h->u32.as<float>();
+    SG_CUDA(launch_to_f32(cols, nc, h->n, h->n_pad, h->v32.as<float>(), st));
+    SG_CUDA(launch_fp32_zt(h->geno, h->wpr, h->zlut, h->m_pad, h->v32.as<float>(), nc, u, st));
+    if (h->masked)
+      for (int k = 0; k < nc; ++k)
+        SG_CUDA(mask_rows_f32(u + (size_t)k * h->m_pad, h->excl.as<uint8_t>(), h->m, st));
+    for (int k = 0; k < nc; k += kFp32ColsB) {
+      const int nb = std::min(kFp32ColsB, nc - k);
+      Fp32Cols part{};
+      for (int j = 0; j < nb; ++j) part.out[j] = cols.out[k + j];
+      SG_CUDA(launch_fp32_z(h->geno, h->wpr, h->zlut, h->m_pad, u + (size_t)k * h->m_pad, nb,
+                            h->ypart.as<float>(), h->n_splits, st));
+      SG_CUDA(launch_fp32_finish(h->ypart.as<float>(), h->n_splits, h->n_pad, h->n, scale, part, nb,
+                                 st));
+    }
+    h->n_kv += nc;
   }
   h->n_kv_launches += 1;
-  h->stats.fp32_launches += done;
+  h->stats.fp32_launches += (int64_t)act.size();
   if (h->profiling) {
     SG_CUDA(cudaEventRecord(e1, st));
     SG_CUDA(cudaEventSynchronize(e1));

@@ -55,19 +55,27 @@ cudaError_t launch_gen_bed(const void* layout, uint8_t* bed, int64_t bytes_per_m
                            int64_t m, cudaStream_t st);
 
 // ---- FP32 GRM product (saige-rs arithmetic) --------------------------------
+// One to kFp32Cols columns per call (pass B and the finish: to kFp32ColsB); the planes of v32 (n_pad floats, in the kernels' own
+// order), u (m_pad) and ypart (n_splits x n_pad) of column c follow those of column c - 1.
+constexpr int kFp32Cols = 8;
+constexpr int kFp32ColsB = 4;
+struct Fp32Cols {
+  const double* v[kFp32Cols];
+  double* out[kFp32Cols];
+};
 // u[m] = sum_i z(code_mi) v32[i]       (pass A, f32)
 cudaError_t launch_fp32_zt(const uint32_t* geno, int64_t words_per_row, const float4* zlut,
-                           int64_t m_pad, const float* v32, float* u, cudaStream_t st);
+                           int64_t m_pad, const float* v32, int cols, float* u, cudaStream_t st);
 // ypart[s][i] = sum_{m in split s} z(code_mi) u[m]   (pass B, f32)
 cudaError_t launch_fp32_z(const uint32_t* geno, int64_t words_per_row, const float4* zlut,
-                          int64_t m_pad, const float* u, float* ypart, int n_splits,
+                          int64_t m_pad, const float* u, int cols, float* ypart, int n_splits,
                           cudaStream_t st);
 int fp32_z_splits(int64_t n_pad, int64_t m_pad);
 // out[i] = (double)((sum_s ypart[s][i]) * scale)  (f32 arithmetic)
 cudaError_t launch_fp32_finish(const float* ypart, int n_splits, int64_t n_pad, int64_t n,
-                               float scale, double* out, cudaStream_t st);
-// v32[i] = (float)v[i] for i < n, 0 for n <= i < n_pad
-cudaError_t launch_to_f32(const double* v, int64_t n, int64_t n_pad, float* v32,
+                               float scale, const Fp32Cols& cols, int n_cols, cudaStream_t st);
+// v32 <- (float)v[i] for i < n, 0 for n <= i < n_pad
+cudaError_t launch_to_f32(const Fp32Cols& cols, int n_cols, int64_t n, int64_t n_pad, float* v32,
                           cudaStream_t st);
 
 }  // namespace saige

@@ -112,15 +112,16 @@ Status matvec_noalloc(saige_grm* h, const double* v, double* out, int64_t n, int
   float* ypart = reinterpret_cast<float*>(static_cast<unsigned char*>(base) + v_bytes + u_bytes);
   const float scale = 1.0f / (float)h->m_eff;
   for (int c = 0; c < nrhs; ++c) {
-    const double* vc = v + (int64_t)c * n;
-    double* oc = out + (int64_t)c * n;
+    Fp32Cols cols{};
+    cols.v[0] = v + (int64_t)c * n;
+    cols.out[0] = out + (int64_t)c * n;
     // to_f32 writes all n_pad entries (zeros past n); pass A writes all m_pad
     // entries of u; pass B writes every split's plane for the sample windows that
     // the finish kernel reads.
-    SG_CUDA(launch_to_f32(vc, n, h->n_pad, v32, st));
-    SG_CUDA(launch_fp32_zt(h->geno, h->wpr, h->zlut, h->m_pad, v32, u32, st));
-    SG_CUDA(launch_fp32_z(h->geno, h->wpr, h->zlut, h->m_pad, u32, ypart, h->n_splits, st));
-    SG_CUDA(launch_fp32_finish(ypart, h->n_splits, h->n_pad, n, scale, oc, st));
+    SG_CUDA(launch_to_f32(cols, 1, n, h->n_pad, v32, st));
+    SG_CUDA(launch_fp32_zt(h->geno, h->wpr, h->zlut, h->m_pad, v32, 1, u32, st));
+    SG_CUDA(launch_fp32_z(h->geno, h->wpr, h->zlut, h->m_pad, u32, 1, ypart, h->n_splits, st));
+    SG_CUDA(launch_fp32_finish(ypart, h->n_splits, h->n_pad, n, scale, cols, 1, st));
   }
   h->n_kv += nrhs;
   h->n_kv_launches += 1;
