@@ -472,6 +472,7 @@ Status pcg_scratch(saige_grm* h, int q, PcgScratch& s) {
 
 Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   const int q = run.q;
+  const int64_t kv0 = h->n_kv, launches0 = h->n_kv_launches;
   const int64_t n = h->n, ld = h->n_pad;
   PcgScratch s;
   const int ne = run.extra_in && run.extra_out ? run.n_extra : 0;
@@ -570,6 +571,7 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
     if (run.max_iter <= 0 && state[(size_t)c] == kColActive) run.state[(size_t)c] = kColMaxIter;
     run.total_iters += run.iters[(size_t)c];
   }
+  if (run.count_columns) h->n_kv_launches = launches0 + (h->n_kv - kv0);
   return Status();
 }
 

@@ -201,6 +201,8 @@ struct PcgRun {
   double* keep_p = nullptr;
   double* keep_kp = nullptr;
   int keep_cols = 0, keep_cap = 0, kept = 0;
+  // count a product of k columns as k launches (solves that stand for k of one column)
+  bool count_columns = false;
   std::vector<int32_t> iters, state;
   std::vector<double> resid;
   int64_t total_iters = 0;
