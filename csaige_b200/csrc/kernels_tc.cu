@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gptr(P.MISC()));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gptr(P.MISC() + 8u));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // warp: uniform over the warp, and known to be
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tile = blockIdx.x;
 
   if (threadIdx.x == 0) {
@@ -296,18 +297,23 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     // The whole warp takes each filled operand slot from its unpack group through
-    // a named barrier and lane 0 issues the stage's MMAs.  The issuing thread
-    // performs no memory access while its MMAs are in flight: on sm_100 such an
-    // access waits for all of them to complete, which would drain the tensor
-    // pipe at every stage.  One commit per stage releases both the load slot
-    // and the operand slot.
+    // a named barrier and one elected lane issues the stage's MMAs.  The lane comes from
+    // elect.sync, in a branch that is otherwise uniform over the warp: the compiler then
+    // keeps descriptors and addresses in uniform registers, which tcgen05.mma reads.
+    // Under a branch on the lane number each MMA first moved its operands there, 47 cycles
+    // per MMA alone (measured with N = 32; 16 cycles elected) and 79 instead of 65 cycles
+    // with N = 128 beside the unpack's TMEM stores, where the tensor pipe needs 64.
+    // The issuing thread performs no memory access while its MMAs are in flight: on
+    // sm_100 such an access waits for all of them to complete, which would drain the tensor
+    // pipe at every stage.
     // Ring positions advance incrementally: no division in the loop.
     const uint32_t idesc = i8_idesc(a.ng);
+    const int flag_lane = elected_lane() ^ 1;  // not the issuing lane
     int t = 0, s = 0, ab = 0;  // sub-stage within the load stage, load slot, operand slot
-    // (lane 0) the last load stage and sub-stage whose LDONE / ADONE was committed
+    // the last load stage and sub-stage whose LDONE / ADONE was committed
     int j_done = -1, k_done = -1;
     // One named-barrier handoff per batch of hb sub-stages (slots ab .. ab + hb - 1,
-    // barrier 1 + ab / hb): the warp waits once, then lane 0 issues the whole batch.
+    // barrier 1 + ab / hb): the warp waits once, then one lane issues the whole batch.
     for (int k = 0; k < a.nk;) {
       if (lane == 1) {
         trace_mark(a, k, 6);  // MMA warp reaches the stage
@@ -316,38 +322,33 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
       }
       named_bar_sync(1 + (ab >> (kHb - 1)), kHandoffThreads);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 1) trace_mark(a, k, 4);  // MMA may issue
       // After an abort no further MMA is issued (the handoffs still run, in step with
-      // the unpack groups).  Lane 1 reads the flag: lane 0, which has MMAs in flight,
-      // makes no memory access.
-      const int aborted = __shfl_sync(0xffffffffu, lane == 1 ? *abort_flag : 0, 1);
+      // the unpack groups).  The flag is read by a lane that has no MMAs in flight.
+      const bool aborted = __any_sync(0xffffffffu, lane == flag_lane && *abort_flag);
       const int k_batch = k;
+      if (lane == flag_lane) trace_mark(a, k, 4);  // MMA may issue
 #pragma unroll
       for (int j = 0; j < kHb; ++j, ++k) {
         if (kHb > 1 && k >= a.nk) break;
-        if (lane == 0 && !aborted) {
-          // genotype and missing-flag MMAs alternate (two independent accumulators
-          // pipeline; grouping each accumulator's MMAs measured 15-40 % slower), and
-          // each sub-stage is committed as soon as its MMAs are issued, so that its
-          // operand and load slots free up one sub-stage earlier than a batch commit
+        if (!aborted) {
+          // genotype and missing-flag MMAs alternate (two independent accumulators)
           const uint64_t bg = sw128_desc(P.B_g(s, t));
           const uint64_t bm = kPassB ? sw128_desc(P.B_m(s, t)) : bg;
           const uint32_t ag = tmem_a + (uint32_t)ab * kSlotCols, am = ag + 32u;
+          const bool stage_end = t == a.sub - 1 || k == a.nk - 1;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kKt / 32; ++kk) {
-            // K advance of 32 int8: 8 TMEM columns of A, 32 bytes (2 x 16 B) along a B row
-            const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-            mma_i8_ts(tmem_g, ag + 8u * kk, bg + 2u * kk, idesc, acc);
-            mma_i8_ts(tmem_m, am + 8u * kk, bm + 2u * kk, idesc, acc);
+            for (int kk = 0; kk < kKt / 32; ++kk) {
+              // K advance of 32 int8: 8 TMEM columns of A, 32 bytes (2 x 16 B) along a B row
+              const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
+              mma_i8_ts(tmem_g, ag + 8u * kk, bg + 2u * kk, idesc, acc);
+              mma_i8_ts(tmem_m, am + 8u * kk, bm + 2u * kk, idesc, acc);
+            }
+            if (!kMerged) mma_commit(P.ADONE(ab));
+            if (stage_end) mma_commit(P.LDONE(s));
           }
-          if (!kMerged) {
-            mma_commit(P.ADONE(ab));
-            k_done = k;
-          }
-          if (t == a.sub - 1 || k == a.nk - 1) {
-            mma_commit(P.LDONE(s));
-            j_done = k / a.sub;
-          }
+          if (!kMerged) k_done = k;
+          if (stage_end) j_done = k / a.sub;
         }
         if (++t == a.sub) {
           t = 0;
@@ -356,9 +357,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
         if (++ab == a.sa) ab = 0;
       }
       __syncwarp();
-      if (lane == 1) trace_mark(a, k_batch, 5);  // MMAs issued
+      if (lane == flag_lane) trace_mark(a, k_batch, 5);  // MMAs issued
     }
-    if (lane == 0) {
+    if (elect_one()) {
       mma_commit(P.ACCF());
       // A commit's mbarrier arrival is performed when its MMAs complete, in no set order
       // with the other commits: the epilogue's wait on ACCF does not cover the last

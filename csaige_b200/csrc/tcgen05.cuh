@@ -148,6 +148,24 @@ __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// True in one lane of a converged warp, always the same one (elect.sync).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
+// The lane that elect_one picks.
+__device__ __forceinline__ int elected_lane() {
+  uint32_t lane;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync %0|p, 0xffffffff;\n\t}" : "=r"(lane));
+  return (int)lane;
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    bar)
