@@ -24,18 +24,22 @@
 // Both use the device word layout of the row-major copy (entry 4j+i of a
 // 16-entry word at bit 16(j>>1) + 2(j&1) + 4i), built once per GRM.
 //
-// Pipeline (one CTA per 128-row tile, K swept in 128-entry stages):
-//   warp 0      bulk-copies the stage's code tile and its vector-limb tile(s)
+// Pipeline (one persistent CTA per SM; the launch's sub-stages of 128 rows x 128 K entries
+// are numbered tile by tile and divided evenly over the CTAs, so a CTA walks a run of
+// segments, each a tile or a part of one):
+//   warp 0      bulk-copies the sub-stages' code tiles and their vector-limb tile(s)
 //               (written beforehand in the 128-byte-swizzled K-major layout)
-//               into a shared-memory load ring;
-//   warps 2-9   two groups of four warps take alternate stages; each thread
+//               into a shared-memory load ring, running ahead over segments;
+//   warps 2-17  four groups of four warps take sub-stages in turn; each thread
 //               expands its row's 128 codes into 128 int8 genotypes and 128
 //               int8 missing flags with byte permutes and stores them straight
 //               into a TMEM operand slot (tcgen05.st): the A operand never
 //               touches shared memory;
 //   warp 1      issues tcgen05.mma kind::i8 with A from TMEM and B (limbs)
-//               from shared memory, and commits each stage to mbarriers;
-//   warps 2-9   finally run the FP64 epilogue from the TMEM accumulators.
+//               from shared memory, and commits each sub-stage to mbarriers;
+//   warps 2-17  run the epilogue of each segment from the TMEM accumulators: FP64 and
+//               the output for a whole tile; the integer sums of a part of a tile meet
+//               in global memory, and the CTA that adds the last part finishes the tile.
 // Every mbarrier wait is bounded; a wait that runs out sets an error word the
 // host reads back (SAIGE_TIMEOUT).
 #include <cuda.h>
@@ -63,10 +67,11 @@ using namespace tcx;
 constexpr int kRows = 128;                    // MMA M: rows of a CTA tile
 constexpr int kKt = 128;                      // K entries per pipeline stage
 constexpr uint32_t kTileBytes = kRows * kKt / 4;  // 4 KB of 2-bit codes
-constexpr int kMaxSA = 6;                     // TMEM operand slots at most
+constexpr int kGroups = 4;                     // unpack groups of four warps
+constexpr int kMaxSA = kGroups;               // TMEM operand slots at most
 constexpr int kMaxSL = 24;                    // load-ring stages at most
-constexpr int kUnpackWarps = 8;
-constexpr int kThreads = 64 + 32 * kUnpackWarps;  // producer warp, MMA warp, 8 unpack warps
+constexpr int kUnpackThreads = 128 * kGroups;
+constexpr int kThreads = 64 + kUnpackThreads;  // producer warp, MMA warp, unpack warps
 constexpr size_t kSmemBudget = 227 * 1024;
 constexpr uint32_t kTmemCols = 512;           // the whole TMEM (one CTA per SM)
 constexpr uint32_t kSlotCols = 64;            // per slot: 32 columns of genotypes + 32 of flags
@@ -76,12 +81,18 @@ constexpr double kQ = 127.0 * 65536.0;
 struct TcArgs {
   int ng;                   // B tile rows (= MMA N), multiple of 16
   int r;                    // right-hand sides in this launch
-  int nk;                   // pipeline stages over K
+  int nk;                   // sub-stages over K of a tile
+  // work division (TcWork): whole tiles per CTA, then the sub-stages of the tiles left over
+  int whole, extra;         // CTA c takes tiles c + i grid, i < whole (+ 1 for c < extra)
+  int tail_tile;            // first tile that CTAs share
+  int64_t tail_units;       // sub-stages of the shared tiles
   int sub;                  // 128-entry sub-stages per load stage (1, 2 or 4)
   int sl;                   // load-ring depth in load stages (>= 2)
-  int sa;                   // TMEM operand slots, one per sub-stage (a multiple of 2 hb)
-  int hb;                   // sub-stages per handoff to the MMA warp (1 or 2)
-  int merged;               // 1: one commit per batch (hb == sub == 2, sa == 4, sl >= 3)
+  int sa;                   // TMEM operand slots, one per sub-stage (2 .. kGroups)
+  // sums of tiles that several CTAs share: per slot (TcSplit) 2 x r x 128 int64, and the
+  // sub-stages added so far; all zero between launches
+  unsigned long long* part;
+  unsigned int* part_done;
   const uint8_t* tiles;     // this pass's code tiles, tile t at (t*tile_ld + k)*4 KB
   int64_t tile_ld;          // tiles from one output tile's row of tiles to the next (>= nk)
   const uint8_t* img_g;     // nk x ng x 128 bytes
@@ -103,9 +114,10 @@ struct TcArgs {
 constexpr int kTraceStages = 64;
 constexpr int kTraceSlots = 8;
 
-// Records %globaltimer for CTA 0, stage k, event slot e when tracing is on.
+// Records %globaltimer for CTA 0, sub-stage k, event slot e (kTrace builds of the kernel).
+template <bool kTrace>
 __device__ __forceinline__ void trace_mark(const TcArgs& a, int k, int e) {
-  if (a.trace && blockIdx.x == 0 && k < kTraceStages) {
+  if (kTrace && blockIdx.x == 0 && k < kTraceStages) {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     a.trace[k * kTraceSlots + e] = t;
@@ -133,21 +145,63 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t tmem_d, uint32_t tmem_a, uint
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z));
 }
 
-// Named barriers 1..sa hand operand slot ab from its unpack group (four warps,
-// bar.arrive) to the MMA warp (bar.sync).
-constexpr int kHandoffThreads = 32 + 32 * (kUnpackWarps / 2);
+constexpr int kEpi = 4;  // columns per step of the epilogue (12 limb columns)
+constexpr int kUnpackWarps = kUnpackThreads / 32;
 
-// 32 consecutive TMEM columns of this thread's lane <- v[0..31].
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+// CTA c's share of the shared tiles' sub-stages: [units c / grid, units (c + 1) / grid).
+__host__ __device__ __forceinline__ int64_t unit_begin(int64_t units, int c, int grid) {
+  return units * c / grid;
+}
+
+// One CTA's run of segments: its whole tiles, then its share of the tiles left over.
+struct Segments {
+  int64_t u, end;
+  int i, n_whole, nk, tail_tile;
+  int tile, k0, k1;
+  __device__ Segments(const TcArgs& a)
+      : u(unit_begin(a.tail_units, blockIdx.x, gridDim.x)),
+        end(unit_begin(a.tail_units, blockIdx.x + 1, gridDim.x)),
+        i(0),
+        n_whole(a.whole + ((int)blockIdx.x < a.extra ? 1 : 0)),
+        nk(a.nk),
+        tail_tile(a.tail_tile) {}
+  // the next segment: sub-stages [k0, k1) of `tile`
+  __device__ bool next() {
+    if (i < n_whole) {
+      tile = (int)(blockIdx.x + (unsigned)i * gridDim.x);
+      k0 = 0;
+      k1 = nk;
+      ++i;
+      return true;
+    }
+    if (u >= end) return false;
+    const int q = (int)(u / nk);
+    tile = tail_tile + q;
+    k0 = (int)(u - (int64_t)q * nk);
+    const int64_t left = end - u;
+    k1 = left < nk - k0 ? k0 + (int)left : nk;
+    u += k1 - k0;
+    return true;
+  }
+};
+
+// Slot of a tile that several CTAs share: the first CTA (>= 1) whose share begins inside it,
+// less one.
+__device__ __forceinline__ int part_slot(const TcArgs& a, int tile) {
+  const int64_t first = (int64_t)(tile - a.tail_tile) * a.nk;
+  int c = (int)(first * gridDim.x / a.tail_units);
+  while (unit_begin(a.tail_units, c, gridDim.x) <= first) ++c;
+  return c - 1;
+}
+
+// 16 consecutive TMEM columns of this thread's lane <- v[0..15].
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-      "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, "
-      "%29, %30, %31, %32};" ::"r"(taddr),
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15, %16};" ::"r"(taddr),
       "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
       "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
-      "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]),
-      "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]),
-      "r"(v[29]), "r"(v[30]), "r"(v[31])
+      "r"(v[15])
       : "memory");
 }
 
@@ -158,12 +212,16 @@ constexpr uint32_t kLutM = 0x00000100u;
 // Shared-memory plan (1024-byte aligned):
 //   load ring  sl x [codes sub x 4 KB | B_g sub x ng*128 | B_m sub x ng*128 (pass B)]
 //   barriers   FULL[sl] (load stage landed), LDONE[sl] (its MMAs complete),
-//              ADONE[sa] (MMAs reading operand slot complete), ACCF
-//   misc       TMEM address, abort flag
+//              AFULL[kGroups] (a group's sub-stage is in its operand slot: one arrival per
+//              warp), ADONE[kGroups] (its MMAs complete), ACCF (a segment's MMAs complete),
+//              AFREE (its accumulators read: one arrival per unpack warp), PSUM and PLAST
+//              (the sums of a shared tile: added by every warp, its count taken)
+//   misc       TMEM address, abort flag, last-part flag
+// Every wait between roles is a bounded wait on an mbarrier: a role that gives up raises the
+// abort flag and leaves its loop, the others see the flag in their next wait, and nobody
+// waits for an arrival that does not come.
 // A load stage carries `sub` consecutive 128-entry sub-stages in one
-// transaction-counted mbarrier phase: a CTA completes only about one such
-// phase per ~550 cycles on sm_100, so 4 KB phases would cap a CTA near
-// 15 GB/s; 16 KB and more per phase reach HBM speed.
+// transaction-counted mbarrier phase (fewer at the end of a segment).
 // TMEM: accumulators G at columns [0, ng), Mi at [ng, 2 ng); operand slots of
 // 64 columns (one sub-stage) from column a0 = round_up(2 ng, 32).
 struct SmemPlan {
@@ -178,9 +236,13 @@ struct SmemPlan {
   }
   __device__ uint32_t FULL(int s) const { return bars + 8u * s; }
   __device__ uint32_t LDONE(int s) const { return bars + 8u * (kMaxSL + s); }
-  __device__ uint32_t ADONE(int a) const { return bars + 8u * (2 * kMaxSL + a); }
-  __device__ uint32_t ACCF() const { return bars + 8u * (2 * kMaxSL + kMaxSA); }
-  __device__ uint32_t MISC() const { return ACCF() + 8u; }
+  __device__ uint32_t AFULL(int g) const { return bars + 8u * (2 * kMaxSL + g); }
+  __device__ uint32_t ADONE(int g) const { return bars + 8u * (2 * kMaxSL + kGroups + g); }
+  __device__ uint32_t ACCF() const { return bars + 8u * (2 * kMaxSL + 2 * kGroups); }
+  __device__ uint32_t AFREE() const { return ACCF() + 8u; }
+  __device__ uint32_t PSUM() const { return ACCF() + 16u; }
+  __device__ uint32_t PLAST() const { return ACCF() + 24u; }
+  __device__ uint32_t MISC() const { return ACCF() + 32u; }
 };
 
 __host__ __device__ constexpr uint32_t round1k(uint32_t x) { return (x + 1023u) & ~1023u; }
@@ -213,14 +275,21 @@ __device__ __forceinline__ void expand_word(uint32_t w, uint32_t* g, uint32_t* m
   m[3] = __byte_perm(kLutM, 0u, hi2);
 }
 
-// kHb: sub-stages per handoff (a.hb), a template parameter so that the batch loops
-// unroll to straight-line code.  kMerged (with kHb == 2 and two sub-stages per load
-// stage): one commit per batch, on the load stage's LDONE barrier, frees both the load
-// slot and the batch's two operand slots.  A tcgen05.commit leaves the tensor pipe idle
-// for ~200 cycles (measured: 8 MMAs of M=128, N=128, K=32 per sub-stage took ~830
-// cycles with 1.5 commits per sub-stage and no handoff at all, 32 MMAs ~2,300), so the
-// merged batches — 16 MMAs per commit instead of 8 per 1.5 — keep it busier.
-template <bool kPassB, int kHb, bool kMerged>
+// What bounds it.  The tensor pipe needs 64 cycles for an MMA (M = 128, N = 128, K = 32), 512
+// per sub-stage of 128 x 128 entries (4 K-steps x genotype and missing accumulators); at 42
+// columns and 200,000 x 150,000 both passes run long enough for the chip's power limit to
+// lower the SM clock (1.62-1.77 GHz sampled inside the kernel).  Below that, the MMA warp's own
+// instructions (see there), and in pass B shared memory: 36 KB of copies, 32 KB of operand
+// reads and 4 KB of codes per sub-stage, against 20 + 32 + 4 KB in pass A.
+// 37 columns at 50,000 x 100,000, pass A / pass B in us:
+//   1222 / 1182  MMAs issued under a branch on the lane number;
+//    945 /  956  by an elected lane, two unpack groups, two sub-stages per handoff, a CTA
+//                per tile (five and two waves, the last one partly empty);
+//    860 /  845  four unpack groups, a persistent CTA per SM, the tiles left over shared;
+//    740 /  852  and the next sub-stage's barrier tested between the halves of this one's MMAs.
+// (Two MMA warps, one per accumulator: 785 / 962.  Whole tiles started at different K per CTA:
+// no change, so the operand tiles' L2 reads do not bound it.)
+template <bool kPassB, bool kTrace>
 __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -234,18 +303,24 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
   auto gptr = [&](uint32_t saddr) { return gen + (saddr - P.base); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gptr(P.MISC()));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gptr(P.MISC() + 8u));
+  volatile int* last_part = reinterpret_cast<volatile int*>(gptr(P.MISC() + 12u));
 
   // warp: uniform over the warp, and known to be
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int tile = blockIdx.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.sl; ++s) {
       mbar_init(P.FULL(s), 1);
       mbar_init(P.LDONE(s), 1);
     }
-    for (int s = 0; s < a.sa; ++s) mbar_init(P.ADONE(s), 1);
+    for (int g = 0; g < kGroups; ++g) {
+      mbar_init(P.AFULL(g), kUnpackWarps / kGroups);
+      mbar_init(P.ADONE(g), 1);
+    }
     mbar_init(P.ACCF(), 1);
+    mbar_init(P.AFREE(), kUnpackWarps);
+    mbar_init(P.PSUM(), kUnpackWarps);
+    mbar_init(P.PLAST(), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -261,247 +336,224 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
   const uint32_t tmem = *tmem_slot;
   const uint32_t tmem_g = tmem, tmem_m = tmem + (uint32_t)a.ng;
   const uint32_t tmem_a = tmem + tmem_a0(a.ng);
+  Segments seg(a);
 
   if (warp == 0) {
     // ---------------- producer: code tiles and limb tiles by bulk copy ----------------
     if (lane == 0) {
-      const int n_load = (a.nk + a.sub - 1) / a.sub;
-      const uint8_t* codes = a.tiles + (size_t)tile * a.tile_ld * kTileBytes;
-      int S = 0;
-      uint32_t ph = 0;  // (J / sl) & 1
-      int issued = 0;   // load stages whose copies were issued
-      for (int J = 0; J < n_load; ++J) {
-        // the slot is free once the MMAs of load stage J - sl completed
-        if (J >= a.sl && !mbar_wait_sleep(P.LDONE(S), ph ^ 1u, abort_flag, a.err, a.wait_cycles))
-          break;
-        if (J < kTraceStages) trace_mark(a, J, 0);  // load issued
-        const int k0 = J * a.sub;
-        const uint32_t cnt = (uint32_t)min(a.sub, a.nk - k0);
-        mbar_expect_tx(P.FULL(S), cnt * (kTileBytes + P.b_bytes * (kPassB ? 2u : 1u)));
-        bulk_load(P.CODES(S, 0), codes + (size_t)k0 * kTileBytes, cnt * kTileBytes, P.FULL(S));
-        for (uint32_t t = 0; t < cnt; ++t) {  // limb tiles: one copy per sub-stage (<= 24 KB)
-          bulk_load(P.B_g(S, t), a.img_g + (size_t)(k0 + t) * P.b_bytes, P.b_bytes, P.FULL(S));
-          if (kPassB)
-            bulk_load(P.B_m(S, t), a.img_m + (size_t)(k0 + t) * P.b_bytes, P.b_bytes, P.FULL(S));
+      int S = 0, J = 0;  // load slot, load stages so far
+      uint32_t ph = 0;   // (J / sl) & 1
+      bool live = true;
+      while (live && seg.next()) {
+        const uint8_t* codes = a.tiles + (size_t)seg.tile * a.tile_ld * kTileBytes;
+        for (int k0 = seg.k0; k0 < seg.k1; k0 += a.sub) {
+          // the slot is free once the MMAs of load stage J - sl completed
+          if (J >= a.sl && !mbar_wait_poll(P.LDONE(S), ph ^ 1u, abort_flag, a.err, a.wait_cycles)) {
+            live = false;
+            break;
+          }
+          if (J < kTraceStages) trace_mark<kTrace>(a, J, 0);  // load issued
+          const uint32_t cnt = (uint32_t)min(a.sub, seg.k1 - k0);
+          mbar_expect_tx(P.FULL(S), cnt * (kTileBytes + P.b_bytes * (kPassB ? 2u : 1u)));
+          bulk_load(P.CODES(S, 0), codes + (size_t)k0 * kTileBytes, cnt * kTileBytes, P.FULL(S));
+          for (uint32_t t = 0; t < cnt; ++t) {  // limb tiles: one copy per sub-stage (<= 24 KB)
+            bulk_load(P.B_g(S, t), a.img_g + (size_t)(k0 + t) * P.b_bytes, P.b_bytes, P.FULL(S));
+            if (kPassB)
+              bulk_load(P.B_m(S, t), a.img_m + (size_t)(k0 + t) * P.b_bytes, P.b_bytes, P.FULL(S));
+          }
+          ++J;
+          if (++S == a.sl) { S = 0; ph ^= 1u; }
         }
-        issued = J + 1;
-        if (++S == a.sl) { S = 0; ph ^= 1u; }
       }
-      // Before the CTA exits, every issued copy has landed: load stage J completes
-      // phase (J / sl) & 1 of FULL(J % sl), and only the last sl issued stages can
-      // still be in flight (stage J was issued after stage J - sl was consumed).  On
+      // Before the CTA exits, every issued copy has landed: load stage j completes
+      // phase (j / sl) & 1 of FULL(j % sl), and only the last sl issued stages can
+      // still be in flight (stage j was issued after stage j - sl was consumed).  On
       // the normal path these phases completed long ago and the waits return at once.
-      for (int J = issued > a.sl ? issued - a.sl : 0; J < issued; ++J)
-        mbar_wait_drain(P.FULL(J % a.sl), (uint32_t)((J / a.sl) & 1), a.err);
+      for (int j = J > a.sl ? J - a.sl : 0; j < J; ++j)
+        mbar_wait_drain(P.FULL(j % a.sl), (uint32_t)((j / a.sl) & 1), a.err);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    // The whole warp takes each filled operand slot from its unpack group through
-    // a named barrier and one elected lane issues the stage's MMAs.  The lane comes from
-    // elect.sync, in a branch that is otherwise uniform over the warp: the compiler then
-    // keeps descriptors and addresses in uniform registers, which tcgen05.mma reads.
-    // Under a branch on the lane number each MMA first moved its operands there, 47 cycles
-    // per MMA alone (measured with N = 32; 16 cycles elected) and 79 instead of 65 cycles
-    // with N = 128 beside the unpack's TMEM stores, where the tensor pipe needs 64.
-    // The issuing thread performs no memory access while its MMAs are in flight: on
-    // sm_100 such an access waits for all of them to complete, which would drain the tensor
-    // pipe at every stage.
+    // All lanes wait for each filled operand slot of the unpack groups and an elected one
+    // issues the sub-stage's MMAs.  This warp's instructions set the pace wherever they take
+    // longer than the 512 cycles of the tensor pipe (measured per sub-stage, 8 MMAs and
+    // their commits, with nothing else running, N = 48 / N = 128):
+    //   268 / 512 without a wait: elect.sync, in a branch that is otherwise uniform over the
+    //     warp, lets the compiler keep descriptors and addresses in uniform registers, which
+    //     tcgen05.mma reads (under a branch on the lane number: 47 cycles per MMA);
+    //   325 / 512 with one test of the barrier by all lanes, the polling loop out of line;
+    //   399 / 579 with the polling loop inline; 489 / 669 with a lane of its own polling and
+    //     a vote.
+    // Beside the unpack warps, which share its scheduler, they take longer, and the pipe
+    // queues only about two MMAs: so the next sub-stage's barrier is tested while half of
+    // this one's are still to be issued.
     // Ring positions advance incrementally: no division in the loop.
     const uint32_t idesc = i8_idesc(a.ng);
-    const int flag_lane = elected_lane() ^ 1;  // not the issuing lane
-    int t = 0, s = 0, ab = 0;  // sub-stage within the load stage, load slot, operand slot
-    // the last load stage and sub-stage whose LDONE / ADONE was committed
-    int j_done = -1, k_done = -1;
-    // One named-barrier handoff per batch of hb sub-stages (slots ab .. ab + hb - 1,
-    // barrier 1 + ab / hb): the warp waits once, then one lane issues the whole batch.
-    for (int k = 0; k < a.nk;) {
-      if (lane == 1) {
-        trace_mark(a, k, 6);  // MMA warp reaches the stage
-        if (a.trace && blockIdx.x == 0 && k < kTraceStages)
-          a.trace[k * kTraceSlots + 7] = (unsigned long long)clock64();  // SM clock at the same point
-      }
-      named_bar_sync(1 + (ab >> (kHb - 1)), kHandoffThreads);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // After an abort no further MMA is issued (the handoffs still run, in step with
-      // the unpack groups).  The flag is read by a lane that has no MMAs in flight.
-      const bool aborted = __any_sync(0xffffffffu, lane == flag_lane && *abort_flag);
-      const int k_batch = k;
-      if (lane == flag_lane) trace_mark(a, k, 4);  // MMA may issue
-#pragma unroll
-      for (int j = 0; j < kHb; ++j, ++k) {
-        if (kHb > 1 && k >= a.nk) break;
-        if (!aborted) {
-          // genotype and missing-flag MMAs alternate (two independent accumulators)
-          const uint64_t bg = sw128_desc(P.B_g(s, t));
-          const uint64_t bm = kPassB ? sw128_desc(P.B_m(s, t)) : bg;
-          const uint32_t ag = tmem_a + (uint32_t)ab * kSlotCols, am = ag + 32u;
-          const bool stage_end = t == a.sub - 1 || k == a.nk - 1;
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < kKt / 32; ++kk) {
-              // K advance of 32 int8: 8 TMEM columns of A, 32 bytes (2 x 16 B) along a B row
-              const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-              mma_i8_ts(tmem_g, ag + 8u * kk, bg + 2u * kk, idesc, acc);
-              mma_i8_ts(tmem_m, am + 8u * kk, bm + 2u * kk, idesc, acc);
-            }
-            if (!kMerged) mma_commit(P.ADONE(ab));
-            if (stage_end) mma_commit(P.LDONE(s));
-          }
-          if (!kMerged) k_done = k;
-          if (stage_end) j_done = k / a.sub;
+    int t = 0, s = 0, ab = 0, grp = 0;  // sub-stage within the load stage, load slot, operand
+                                        // slot, unpack group
+    uint32_t ph_a = 0;                  // (K / kGroups) & 1
+    int K = 0, J = 0, n_seg = 0;        // sub-stages, load stages and segments committed so far
+    bool live = true, ready = false;    // ready: the sub-stage's operands are known to be in place
+    // all lanes: a bounded wait
+    auto wait_for = [&](uint32_t bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, abort_flag, a.err,
+                                                    a.wait_cycles)) != 0;
+    };
+    while (live && seg.next()) {
+      // the accumulators of the segment before have been read
+      if (n_seg > 0) live = wait_for(P.AFREE(), (uint32_t)(n_seg - 1) & 1u);
+      const int n = __shfl_sync(0xffffffffu, seg.k1 - seg.k0, 0);
+      for (int k = 0; live && k < n; ++k) {
+        if (kTrace && lane == 0) {
+          trace_mark<kTrace>(a, K, 6);  // MMA warp reaches the sub-stage
+          if (blockIdx.x == 0 && K < kTraceStages)
+            a.trace[K * kTraceSlots + 7] = (unsigned long long)clock64();  // SM clock at the same point
         }
-        if (++t == a.sub) {
+        if (!ready) live = wait_for(P.AFULL(grp), ph_a);
+        if (!live) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (kTrace && lane == 0) trace_mark<kTrace>(a, K, 4);  // MMA may issue
+        const bool stage_end = t == a.sub - 1 || k == n - 1;
+        // genotype and missing-flag MMAs alternate (two independent accumulators)
+        const uint64_t bg = sw128_desc(P.B_g(s, t));
+        const uint64_t bm = kPassB ? sw128_desc(P.B_m(s, t)) : bg;
+        const uint32_t ag = tmem_a + (uint32_t)ab * kSlotCols, am = ag + 32u;
+        const uint32_t later = k > 0 ? 1u : 0u;
+        // K advance of 32 int8: 8 TMEM columns of A, 32 bytes (2 x 16 B) along a B row
+        auto issue = [&](int kk, uint32_t acc) {
+          mma_i8_ts(tmem_g, ag + 8u * kk, bg + 2u * kk, idesc, acc);
+          mma_i8_ts(tmem_m, am + 8u * kk, bm + 2u * kk, idesc, acc);
+        };
+        if (elect_one()) {
+          issue(0, later);
+          issue(1, 1u);
+        }
+        // between the halves, while MMAs are queued: is the next sub-stage in place?
+        ready = __all_sync(0xffffffffu, mbar_test_wait(P.AFULL((grp + 1) % kGroups),
+                                                       grp == kGroups - 1 ? ph_a ^ 1u : ph_a));
+        if (elect_one()) {
+          issue(2, 1u);
+          issue(3, 1u);
+          mma_commit(P.ADONE(grp));
+          if (stage_end) mma_commit(P.LDONE(s));
+        }
+        ++K;
+        ++t;
+        if (stage_end) {
           t = 0;
+          ++J;
           if (++s == a.sl) s = 0;
         }
         if (++ab == a.sa) ab = 0;
+        if (++grp == kGroups) { grp = 0; ph_a ^= 1u; }
+        if (kTrace && lane == 0) trace_mark<kTrace>(a, K - 1, 5);  // MMAs issued
       }
-      __syncwarp();
-      if (lane == flag_lane) trace_mark(a, k_batch, 5);  // MMAs issued
+      if (live) {
+        if (elect_one()) mma_commit(P.ACCF());
+        ++n_seg;
+      }
     }
-    if (elect_one()) {
-      mma_commit(P.ACCF());
-      // A commit's mbarrier arrival is performed when its MMAs complete, in no set order
-      // with the other commits: the epilogue's wait on ACCF does not cover the last
-      // LDONE / ADONE arrivals, and one still in flight when the CTA exits would land in
-      // the shared memory of the next CTA on this SM.  So wait for the last committed
-      // phase of every such barrier (bounded) before the CTA can finish.
-      for (int ls = 0; ls < a.sl; ++ls) {
-        if (j_done < ls) continue;  // slot never committed
-        const int j = j_done - (j_done - ls) % a.sl;
+    if (lane == 0) {
+      // Before the CTA can finish, wait (bounded) for the last committed phase of every
+      // barrier: all MMAs are complete then, and no commit's arrival — performed in no set
+      // order with the others — can land in the shared memory of the SM's next CTA.
+      for (int ls = 0; ls < a.sl && ls < J; ++ls) {
+        const int j = J - 1 - (J - 1 - ls) % a.sl;
         mbar_wait_drain(P.LDONE(ls), (uint32_t)((j / a.sl) & 1), a.err);
       }
-      if (!kMerged)
-        for (int as = 0; as < a.sa; ++as) {
-          if (k_done < as) continue;
-          const int kk2 = k_done - (k_done - as) % a.sa;
-          mbar_wait_drain(P.ADONE(as), (uint32_t)((kk2 / a.sa) & 1), a.err);
-        }
+      for (int g = 0; g < kGroups && g < K; ++g) {
+        const int k = K - 1 - (K - 1 - g) % kGroups;
+        mbar_wait_drain(P.ADONE(g), (uint32_t)((k / kGroups) & 1), a.err);
+      }
+      if (n_seg > 0) mbar_wait_drain(P.ACCF(), (uint32_t)(n_seg - 1) & 1u, a.err);
     }
+    __syncwarp();
   } else {
-    // ---------------- unpack (warps 2-9) ----------------
-    // group 0 (warps 2-5) takes even stages, group 1 (warps 6-9) odd stages;
+    // ---------------- unpack (warps 2-17) ----------------
+    // Group g takes the sub-stages K = g, g + 4, ... of the CTA's run;
     // a warp may only address its own TMEM lane group (warp % 4), so thread
     // `lane` of warp w expands row 32 (w % 4) + lane.
     const int grp = (warp - 2) >> 2;
     const int lg = warp & 3;
     const int row = lg * 32 + lane;
     const uint32_t lane_off = (uint32_t)(lg * 32) << 16;
-    bool live = true;  // false once a wait gave up: the remaining stages only hand over
-    // Group g takes the batches b = g, g + 2, ... of hb sub-stages (sub-stages b hb ..
-    // b hb + hb - 1).  Ring positions of the current sub-stage advance one sub-stage at
-    // a time (no division in the loop).
-    constexpr int hb = kHb;
-    int t = 0, s = 0, ab = 0;
-    uint32_t ph_l = 0;  // phase parity of FULL(s) for the current sub-stage
-    uint32_t ph_a = 0;  // (k / sa) & 1
-    auto step = [&]() {
-      if (++t == a.sub) {
-        t = 0;
-        if (++s == a.sl) { s = 0; ph_l ^= 1u; }
-      }
-      if (++ab == a.sa) { ab = 0; ph_a ^= 1u; }
-    };
-    for (int j = 0; j < grp * hb; ++j) step();
-    for (int kb = grp * hb; kb < a.nk; kb += 2 * hb) {
-      const int bar = 1 + (ab >> (hb - 1));  // the batch's named barrier
+    bool live = true;  // false once a wait gave up (the same for the whole warp)
+    const int lsub = a.sub >> 1;  // log2 (sub is 1, 2 or 4)
+    int K0 = 0, s0 = 0;           // sub-stages before the segment, load slot at its start
+    uint32_t ph0 = 0;             // phase parity of FULL(s0)
+    uint32_t ph_acc = 0, ph_part = 0;
+    while (live && seg.next()) {
+      const int n = seg.k1 - seg.k0;
+      // this group's sub-stages i = i0, i0 + 4, ... of the segment (4 is a multiple of sub: the
+      // place in the load stage stays)
+      int i = (grp - K0) & (kGroups - 1), s = s0 + (i >> lsub), ab = (K0 + i) % a.sa;
+      const int t = i & (a.sub - 1);
+      uint32_t ph_l = ph0;
+      while (s >= a.sl) { s -= a.sl; ph_l ^= 1u; }
+      for (; i < n; i += kGroups) {
+        const int K = K0 + i;
+        // The operand slot is free once the MMAs of its previous use (sub-stage K - sa)
+        // completed.  Sub-stage k's completion is phase k / 4 of ADONE(k % 4): a barrier
+        // per group, not per slot, so that the phase before (sub-stage K - 4 - sa) is the
+        // one this group waited for last and the next one (K + 4 - sa) cannot complete before
+        // this sub-stage is unpacked — with fewer slots than groups a slot's barrier could
+        // pass two phases between two waits of a group, which a parity cannot tell.
+        // This wait comes before the one on the codes: a group sees only every
+        // fourth sub-stage, so FULL(s) may still be a phase behind — its previous load in
+        // flight — and its parity would then already read as this load's.  Once the MMA
+        // warp has taken sub-stage K - sa, every load stage up to it was seen complete, and
+        // at a segment's start all loads before it (the epilogue waited for their MMAs), which
+        // covers load stage J - sl for every accepted ring shape ((sl - 1) sub + 1 >= sa),
+        // so the parity below is unambiguous.
+        if (K >= a.sa)
+          live = mbar_wait_poll(P.ADONE((K - a.sa) % kGroups),
+                                (uint32_t)((K - a.sa) / kGroups) & 1u, abort_flag, a.err,
+                                a.wait_cycles);
+        if (live) live = mbar_wait_poll(P.FULL(s), ph_l, abort_flag, a.err, a.wait_cycles);
+        if (live && row == 0) trace_mark<kTrace>(a, K, 1);  // codes landed
+        live = __all_sync(0xffffffffu, live);  // warp-uniform: the barrier calls below must agree
+        if (!live) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (row == 0) trace_mark<kTrace>(a, K, 2);  // operand slot free
+        const uint32_t crow = P.CODES(s, t) + (uint32_t)row * 32u;
+        const uint4 c0 = lds128(crow), c1 = lds128(crow + 16u);
+        const uint32_t words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const uint32_t slot = tmem_a + lane_off + (uint32_t)ab * kSlotCols;
 #pragma unroll
-      for (int j = 0; j < hb; ++j) {
-        const int k = kb + j;
-        if (hb == 1 || k < a.nk) {
-          // Operand slot ab is free once the MMAs of its previous use (sub-stage k - sa)
-          // completed; merged: both slots of the batch once the MMAs of the batch two
-          // before (this group's previous batch, load stage kb/2 - 2, in the slot two
-          // back) completed.  This wait comes before the one on the codes: a group sees
-          // only every other phase of a load slot that the two groups share (an odd ring
-          // depth), so FULL(s) may still be a phase behind — its previous load in flight
-          // — and its parity would then already read as this load's.  Once the MMA warp
-          // has taken sub-stage k - sa (merged: batch kb/2 - 2), every load stage up to
-          // it was seen complete, which covers load stage k/sub - sl for every accepted
-          // ring shape ((sl - 1) sub + 1 >= sa; merged: sl >= 3), so the parity below is
-          // unambiguous.  The LDONE phase is the latest of its slot, since the next use
-          // of the slot, load stage kb/2 - 2 + sl, follows this batch.
-          if (!kMerged) {
-            if (live && k >= a.sa)
-              live = mbar_wait_sleep(P.ADONE(ab), ph_a ^ 1u, abort_flag, a.err, a.wait_cycles);
-          } else if (j == 0 && live && kb >= 2 * hb) {
-            const int s2 = s >= 2 ? s - 2 : s - 2 + a.sl;
-            const uint32_t ph2 = s >= 2 ? ph_l : (ph_l ^ 1u);
-            live = mbar_wait_sleep(P.LDONE(s2), ph2, abort_flag, a.err, a.wait_cycles);
-          }
-          if (live) live = mbar_wait_sleep(P.FULL(s), ph_l, abort_flag, a.err, a.wait_cycles);
-          if (live && row == 0) trace_mark(a, k, 1);  // codes landed
-          live = __all_sync(0xffffffffu, live);  // warp-uniform: the barrier calls below must agree
-          if (live) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (row == 0) trace_mark(a, k, 2);  // operand slot free
-            const uint32_t crow = P.CODES(s, t) + (uint32_t)row * 32u;
-            const uint4 c0 = lds128(crow), c1 = lds128(crow + 16u);
-            const uint32_t words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            uint32_t g[32], m[32];
+        for (int h = 0; h < 2; ++h) {  // in halves: fewer registers live
+          uint32_t g[16], m[16];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) expand_word(words[c], g + 4 * c, m + 4 * c);
-            const uint32_t slot = tmem_a + lane_off + (uint32_t)ab * kSlotCols;
-            tmem_st32(slot, g);
-            tmem_st32(slot + 32u, m);
-            tmem_wait_st();
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            if (row == 0) trace_mark(a, k, 3);  // unpack done
-          }
+          for (int c = 0; c < 4; ++c) expand_word(words[4 * h + c], g + 4 * c, m + 4 * c);
+          tmem_st16(slot + 16u * h, g);
+          tmem_st16(slot + 32u + 16u * h, m);
         }
-        step();
+        tmem_wait_st();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (row == 0) trace_mark<kTrace>(a, K, 3);  // unpack done
+        __syncwarp();
+        if (lane == 0) mbar_arrive_local(P.AFULL(grp));
+        s += kGroups >> lsub;
+        while (s >= a.sl) { s -= a.sl; ph_l ^= 1u; }
+        if (a.sa == 3 && ++ab == 3) ab = 0;  // 4 mod sa: 0 for two and four slots
       }
-      // Every batch is handed over, also after an abort, so that the MMA warp never
-      // waits for an arrival that does not come.  While live, the wait on the slots'
-      // previous use keeps this group at most one use ahead of the MMA warp on its
-      // named barrier; after an abort bar.sync does that instead.
-      if (live)
-        named_bar_arrive(bar, kHandoffThreads);
-      else
-        named_bar_sync(bar, kHandoffThreads);
-#pragma unroll
-      for (int j = 0; j < hb; ++j) step();  // the other group's batch
-    }
-    // ---------------- epilogue: two warps per TMEM lane group ----------------
-    __syncwarp();
-    const int sub = grp;  // 0 or 1: which half of the column chunks
-    const int trow = row;
-    // The MMA warp always commits ACCF after its last MMA (none after an abort), so
-    // this wait also ensures that no MMA is in flight when the TMEM is freed.
-    const bool ok = mbar_wait_drain(P.ACCF(), 0u, a.err) && !*abort_flag;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int64_t grow = (int64_t)tile * kRows + trow;  // marker (A) or sample (B)
-    double rowa = 0.0, rowb = 0.0;
-    if (!kPassB) {
-      rowa = a.inv_s[grow];
-      rowb = a.two_p[grow];
-    }
-    for (int r0 = 16 * sub; r0 < a.r; r0 += 32) {
-      uint32_t g[48], m[48];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int col = 3 * r0 + 16 * j;
-        if (col < a.ng) {
-          uint32_t tv[16];
-          tmem_ld16(tmem_g + lane_off + (uint32_t)col, tv);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) g[16 * j + e] = tv[e];
-          tmem_ld16(tmem_m + lane_off + (uint32_t)col, tv);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) m[16 * j + e] = tv[e];
-        }
-      }
-      tmem_wait_ld();
-      if (!ok) continue;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const int r = r0 + e;
-        if (r >= a.r) break;
-        const double G = 65536.0 * (double)(int)g[3 * e] + 256.0 * (double)(int)g[3 * e + 1] +
-                         (double)(int)g[3 * e + 2];
-        const double Mi = 65536.0 * (double)(int)m[3 * e] + 256.0 * (double)(int)m[3 * e + 1] +
-                          (double)(int)m[3 * e + 2];
-        const double S = (double)a.sum_q[r];
+      K0 += n;
+      const int s1 = s0 + ((n + a.sub - 1) >> lsub);
+      s0 = s1 % a.sl;
+      ph0 ^= (uint32_t)(s1 / a.sl) & 1u;
+      // ---------------- epilogue of the segment: four warps per TMEM lane group ----------------
+      if (live) live = mbar_wait_poll(P.ACCF(), ph_acc, abort_flag, a.err, a.wait_cycles);
+      live = __all_sync(0xffffffffu, live);
+      if (!live) break;
+      ph_acc ^= 1u;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const bool whole = seg.k0 == 0 && seg.k1 == a.nk;
+      const int64_t grow = (int64_t)seg.tile * kRows + row;  // marker (A) or sample (B)
+      const double rowa = kPassB ? 0.0 : a.inv_s[grow], rowb = kPassB ? 0.0 : a.two_p[grow];
+      const int slot = whole ? 0 : part_slot(a, seg.tile);
+      unsigned long long* part = a.part + (size_t)slot * 2 * a.r * kRows + row;
+      // the output of column r from the exact integer sums
+      auto finish = [&](int r, long long gi, long long mi) {
+        const double G = (double)gi, Mi = (double)mi, S = (double)a.sum_q[r];
         if (!kPassB) {
           // u = (1/s) scale (G - 2p (S - Mi)); explicit roundings (no contraction)
           const double tt = __dsub_rn(G, __dmul_rn(rowb, S - Mi));
@@ -511,6 +563,76 @@ __global__ void __launch_bounds__(kThreads, 1) tc_grm_kernel(TcArgs a) {
           const double y = __dmul_rn(a.out_scale, __dsub_rn(__dmul_rn(a.scale_g[r], G),
                                                             __dmul_rn(a.scale_m[r], S - Mi)));
           a.out[(int64_t)a.col_map[r] * a.out_ld + grow] = y;
+        }
+      };
+      auto free_acc = [&]() {  // this warp has read the accumulators
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive_local(P.AFREE());
+      };
+      if (kEpi * grp >= a.r) free_acc();
+      for (int r0 = kEpi * grp; r0 < a.r; r0 += kEpi * kGroups) {
+        uint32_t g[3 * kEpi], m[3 * kEpi];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int col = 3 * r0 + 4 * j;
+          if (col < a.ng) {
+            tmem_ld4(tmem_g + lane_off + (uint32_t)col, g + 4 * j);
+            tmem_ld4(tmem_m + lane_off + (uint32_t)col, m + 4 * j);
+          }
+        }
+        tmem_wait_ld();
+        if (r0 + kEpi * kGroups >= a.r) free_acc();  // the last read
+#pragma unroll
+        for (int e = 0; e < kEpi; ++e) {
+          const int r = r0 + e;
+          if (r >= a.r) break;
+          // limbs to the exact integers: below 2^53, so exact in FP64 too
+          const long long gi = 65536LL * (int)g[3 * e] + 256LL * (int)g[3 * e + 1] + (int)g[3 * e + 2];
+          const long long mi = 65536LL * (int)m[3 * e] + 256LL * (int)m[3 * e + 1] + (int)m[3 * e + 2];
+          if (whole) {
+            finish(r, gi, mi);
+          } else {
+            atomicAdd(part + (size_t)r * kRows, (unsigned long long)gi);
+            atomicAdd(part + (size_t)(a.r + r) * kRows, (unsigned long long)mi);
+          }
+        }
+      }
+      if (!whole) {
+        // the part that brings a tile's sub-stages to nk finishes it and leaves zeros
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_local(P.PSUM());
+        if (threadIdx.x == 64) {  // every warp's sums are added: take the count
+          live = mbar_wait_poll(P.PSUM(), ph_part, abort_flag, a.err, a.wait_cycles);
+          if (live) {
+            __threadfence();
+            const unsigned int len = (unsigned int)(seg.k1 - seg.k0);
+            const bool last = atomicAdd(a.part_done + slot, len) + len == (unsigned int)a.nk;
+            if (last) a.part_done[slot] = 0u;
+            *last_part = last ? 1 : 0;
+            __threadfence();
+            mbar_arrive_local(P.PLAST());
+          }
+        }
+        if (live) live = mbar_wait_poll(P.PLAST(), ph_part, abort_flag, a.err, a.wait_cycles);
+        live = __all_sync(0xffffffffu, live);
+        if (!live) break;
+        ph_part ^= 1u;
+        if (*last_part) {
+          __threadfence();
+          for (int r0 = kEpi * grp; r0 < a.r; r0 += kEpi * kGroups)
+#pragma unroll
+            for (int e = 0; e < kEpi; ++e) {
+              const int r = r0 + e;
+              if (r >= a.r) break;
+              unsigned long long* pg = part + (size_t)r * kRows;
+              unsigned long long* pm = part + (size_t)(a.r + r) * kRows;
+              const long long gi = (long long)__ldcg(pg), mi = (long long)__ldcg(pm);
+              *pg = 0ull;
+              *pm = 0ull;
+              finish(r, gi, mi);
+            }
         }
       }
     }
@@ -1256,57 +1378,73 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-size_t tc_fixed_bytes() { return 1024 + 8 * (2 * kMaxSL + kMaxSA + 1) + 16; }
+size_t tc_fixed_bytes() { return 1024 + 8 * (2 * kMaxSL + 2 * kGroups + 4) + 16; }
 
 struct Rings {
-  int sub, sl, sa, hb;
-  bool merged = false;  // one commit per batch of two sub-stages (kMerged)
+  int sub, sl, sa;
 };
 
-// Ring shapes for a launch: load stages of up to four sub-stages (16 KB of
-// codes) while at least two such stages fit in shared memory; as many load
-// stages as fit (at most kMaxSL); as many TMEM operand slots as the
-// accumulators leave room for (at most kMaxSA, even, so that each unpack group
-// owns its slots and named barriers).
-// Operand slots (even) that a ring of sl load stages of sub sub-stages accepts: at
-// most (sl - 1) sub + 1, so that the slot-reuse wait of an unpack group implies its
-// load slot's previous load landed.
-int slots_for_ring(int slots, int sl, int sub) {
-  return std::min(slots, (sl - 1) * sub + 1) & ~1;
+// Operand slots that a ring of sl load stages of sub sub-stages accepts: at most
+// (sl - 1) sub + 1, so that the slot-reuse wait of an unpack group implies its load slot's
+// previous load landed; at most what the accumulators leave of the TMEM.
+int slots_for_ring(int ng, int sl, int sub) {
+  const int room = std::min<int>(kMaxSA, (int)((kTmemCols - tmem_a0(ng)) / kSlotCols));
+  return std::min(room, (sl - 1) * sub + 1);
 }
 
-Rings tc_rings(int ng, bool pass_b) {
-  Rings g;
+Rings ring_of(int ng, bool pass_b, int sub) {
   const size_t room = kSmemBudget - tc_fixed_bytes();
-  // batches of two sub-stages with one commit each (the load stage = the batch), where
-  // four operand slots and a ring of three such stages fit
-  const int slots = std::min<int>(kMaxSA, (int)((kTmemCols - tmem_a0(ng)) / kSlotCols));
-  if (slots >= 4 && room / plan_l_stage(ng, pass_b, 2) >= 3) {
-    g.sub = 2;
-    g.sl = (int)std::min<size_t>(kMaxSL, room / plan_l_stage(ng, pass_b, 2));
-    g.sa = 4;
-    g.hb = 2;
-    g.merged = true;
-    return g;
-  }
-  // the most sub-stages per load stage that still leave a ring of four load stages:
-  // at the bench size the autotuner's trials put the shapes with a 2-3 stage ring
-  // 2-25 % behind (pass B at 43-64 columns most), and no deeper ring of fewer
-  // sub-stages lost more than 1 %
-  g.sub = 4;
-  while (g.sub > 1 && room / plan_l_stage(ng, pass_b, g.sub) < 4) g.sub >>= 1;
-  g.sl = (int)std::min<size_t>(kMaxSL, room / plan_l_stage(ng, pass_b, g.sub));
-  g.sa = slots_for_ring(std::min<int>(kMaxSA, (int)((kTmemCols - tmem_a0(ng)) / kSlotCols)),
-                        g.sl, g.sub);
-  // one sub-stage per handoff (two, a tuner candidate, measured 1-5 % slower)
-  g.hb = 1;
+  Rings g;
+  g.sub = sub;
+  g.sl = (int)std::min<size_t>(kMaxSL, room / plan_l_stage(ng, pass_b, sub));
+  g.sa = slots_for_ring(ng, g.sl, sub);
   return g;
+}
+
+// Ring shape of a launch: the most sub-stages per load stage (a copy's fixed cost is shared)
+// that leave a ring of at least three load stages; as many load stages as fit; as many
+// operand slots as the accumulators leave.
+Rings tc_rings(int ng, bool pass_b) {
+  for (int sub : {4, 2}) {
+    const Rings g = ring_of(ng, pass_b, sub);
+    if (g.sl >= 3) return g;
+  }
+  return ring_of(ng, pass_b, 1);
+}
+
+// Division of a launch's tiles over CTAs (one per SM).  Full waves of whole tiles first; the
+// tiles left over, fewer than CTAs, are shared out by sub-stages when that saves at least
+// kMinSaved of them per CTA, else one CTA takes each.  A part of a tile costs its atomics and the
+// last part's second pass (a few us together).
+struct TcWork {
+  int grid, whole, extra, tail_tile;
+  int64_t tail_units;
+};
+constexpr int64_t kMinSaved = 24;
+
+TcWork tc_work(int64_t tiles, int64_t nk, int sms) {
+  TcWork w;
+  w.grid = sms;
+  w.whole = (int)(tiles / sms);
+  w.tail_tile = w.whole * sms;
+  const int64_t rest = tiles - w.tail_tile, share = ceil_div(rest * nk, (int64_t)sms);
+  w.extra = 0;
+  w.tail_units = 0;
+  if (rest > 0 && nk - share >= kMinSaved) {
+    w.tail_units = rest * nk;
+  } else {
+    w.extra = (int)rest;
+    if (w.whole == 0) w.grid = (int)rest;
+  }
+  return w;
 }
 
 }  // namespace
 
 struct TcPlan {
   DevBuf tiles_m, tiles_s, img_a, img_w, img_c, u, scal, cmap, trace;
+  DevBuf part;  // sums of the tiles that CTAs share, and their counts: zero between launches
+  int sms = 0;
   int64_t s_ld = 0;  // tiles_s: marker tiles per sample tile (>= m_pad / 128)
   bool tracing = false;
   // one-column products: the missing-call lists and qc as int32 (m_pad) for pass B's
@@ -1387,9 +1525,14 @@ static Status tc_plan_new(TcPlan** out) {
     delete p;
     return s;
   };
-  for (auto kern : {tc_grm_kernel<false, 1, false>, tc_grm_kernel<true, 1, false>,
-                    tc_grm_kernel<false, 2, false>, tc_grm_kernel<true, 2, false>,
-                    tc_grm_kernel<false, 2, true>, tc_grm_kernel<true, 2, true>}) {
+  {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return bail(fail(SAIGE_ECUDA, "device: %s", cudaGetErrorString(e)));
+  }
+  for (auto kern : {tc_grm_kernel<false, false>, tc_grm_kernel<true, false>,
+                    tc_grm_kernel<false, true>, tc_grm_kernel<true, true>}) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kSmemBudget);
     if (e != cudaSuccess)
@@ -1492,23 +1635,17 @@ template <bool kPassB>
 static cudaError_t launch_tc(unsigned grid, const TcArgs& args, cudaStream_t st) {
   TcArgs a = args;
   a.wait_cycles = g_tc_wait_cycles.load(std::memory_order_relaxed);
-  if (a.hb < 1 || a.hb > 2 || a.sa < 2 * a.hb || a.sa % (2 * a.hb) || a.sa > kMaxSA ||
-      a.sl < 2 || a.sl > kMaxSL || a.sub < 1 ||
-      a.sub > 4)
-    return cudaErrorInvalidValue;
-  if (a.merged && !(a.hb == 2 && a.sub == 2 && a.sa == 4 && a.sl >= 3))
+  if (a.sa < 2 || a.sa > kMaxSA || a.sl < 2 || a.sl > kMaxSL || a.sub < 1 || a.sub > 4)
     return cudaErrorInvalidValue;
   // an unpack group may wait on a load slot's codes only once the slot's previous load
   // is known to have landed (see the unpack loop): (sl - 1) sub + 1 >= sa
-  if (!a.merged && (a.sl - 1) * a.sub + 1 < a.sa) return cudaErrorInvalidValue;
+  if ((a.sl - 1) * a.sub + 1 < a.sa) return cudaErrorInvalidValue;
   const size_t smem = tc_fixed_bytes() + (size_t)a.sl * plan_l_stage(a.ng, kPassB, a.sub);
   if (smem > kSmemBudget) return cudaErrorInvalidValue;
-  if (a.merged)
-    tc_grm_kernel<kPassB, 2, true><<<grid, kThreads, smem, st>>>(a);
-  else if (a.hb == 2)
-    tc_grm_kernel<kPassB, 2, false><<<grid, kThreads, smem, st>>>(a);
+  if (a.trace)
+    tc_grm_kernel<kPassB, true><<<grid, kThreads, smem, st>>>(a);
   else
-    tc_grm_kernel<kPassB, 1, false><<<grid, kThreads, smem, st>>>(a);
+    tc_grm_kernel<kPassB, false><<<grid, kThreads, smem, st>>>(a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1519,8 +1656,8 @@ static cudaError_t launch_tc(unsigned grid, const TcArgs& args, cudaStream_t st)
 // is per element — only its speed.  So the tuning needs no launches of its own: the
 // first launches of each key — pass, ng and the launch's size class (log2 of its 4 KB
 // stages) — in the process each run the real product with the next candidate shape
-// (sub 4, 2, 1 with the deepest ring the shared memory holds; one or two sub-stages per
-// handoff where four operand slots fit; tc_rings' choice first), timed with CUDA events
+// (sub 4, 2, 1 with the deepest ring the shared memory holds; tc_rings' choice first),
+// timed with CUDA events
 // that are read at the key's next launch; once every candidate has run, the fastest is
 // kept for the later launches.  Launches of fewer than kTuneMinStages stages keep the
 // fixed choice of tc_rings, as does SAIGE_TC_AUTOTUNE=0 (=2 tunes every size).
@@ -1571,39 +1708,10 @@ int autotune_level() {
 }
 
 std::vector<Rings> tc_candidates(int ng, bool pass_b) {
-  std::vector<Rings> out;
-  const size_t room = kSmemBudget - tc_fixed_bytes();
-  const Rings base = tc_rings(ng, pass_b);
-  out.push_back(base);  // the fixed choice first
-  const int slots = std::min<int>(kMaxSA, (int)((kTmemCols - tmem_a0(ng)) / kSlotCols)) & ~1;
+  std::vector<Rings> out = {tc_rings(ng, pass_b)};  // the fixed choice first
   for (int sub : {4, 2, 1}) {
-    const size_t ls = plan_l_stage(ng, pass_b, sub);
-    if (2 * ls > room) continue;
-    Rings g;
-    g.sub = sub;
-    g.sl = (int)std::min<size_t>(kMaxSL, room / ls);
-    g.sa = slots_for_ring(slots, g.sl, sub);
-    g.hb = 1;
-    if (g.sa < 2) continue;
-    out.push_back(g);
-    if (g.sa >= 4) {  // the same ring with two sub-stages per handoff (four slots)
-      g.hb = 2;
-      g.sa = 4;
-      out.push_back(g);
-      if (sub == 2 && g.sl >= 3) {  // and one commit per batch
-        g.merged = true;
-        out.push_back(g);
-      }
-    }
-  }
-  // the fixed choice appears once
-  for (size_t i = 1; i < out.size();) {
-    const Rings& g = out[i];
-    if (g.sub == base.sub && g.sl == base.sl && g.sa == base.sa && g.hb == base.hb &&
-        g.merged == base.merged)
-      out.erase(out.begin() + (std::ptrdiff_t)i);
-    else
-      ++i;
+    const Rings g = ring_of(ng, pass_b, sub);
+    if (sub != out[0].sub && g.sl >= 2 && g.sa >= 2) out.push_back(g);
   }
   return out;
 }
@@ -1615,14 +1723,12 @@ std::vector<Rings> tc_candidates(int ng, bool pass_b) {
 template <bool kPassB>
 static Status launch_tc_tuned(int dev, unsigned grid, TcArgs a, cudaStream_t st) {
   const Rings fixed = tc_rings(a.ng, kPassB);
-  const double stages = (double)grid * (double)a.nk;
+  const double stages = ((double)a.whole * grid + a.extra) * a.nk + (double)a.tail_units;
   const int level = autotune_level();
   if (level == 0 || (level == 1 && stages < kTuneMinStages)) {
     a.sub = fixed.sub;
     a.sl = fixed.sl;
     a.sa = fixed.sa;
-    a.hb = fixed.hb;
-    a.merged = fixed.merged ? 1 : 0;
     SG_CUDA(launch_tc<kPassB>(grid, a, st));
     return Status();
   }
@@ -1631,8 +1737,6 @@ static Status launch_tc_tuned(int dev, unsigned grid, TcArgs a, cudaStream_t st)
     a.sub = g.sub;
     a.sl = g.sl;
     a.sa = g.sa;
-    a.hb = g.hb;
-    a.merged = g.merged ? 1 : 0;
   };
   // the state is held under the lock through the (asynchronous) launch, so that one
   // key's candidates and events are used by one launch at a time
@@ -1658,8 +1762,8 @@ static Status launch_tc_tuned(int dev, unsigned grid, TcArgs a, cudaStream_t st)
     ts.ms[(size_t)ts.pending] = ms;
     const Rings& g = ts.cand[(size_t)ts.pending];
     if (log)
-      fprintf(stderr, "[saige tune] pass %c ng %d grid %u nk %d: sub %d sl %d hb %d merged %d -> %.3f ms\n",
-              kPassB ? 'B' : 'A', a.ng, grid, a.nk, g.sub, g.sl, g.hb, g.merged ? 1 : 0, ms);
+      fprintf(stderr, "[saige tune] pass %c ng %d grid %u nk %d: sub %d sl %d sa %d -> %.3f ms\n",
+              kPassB ? 'B' : 'A', a.ng, grid, a.nk, g.sub, g.sl, g.sa, ms);
     ts.pending = -1;
   }
   while (ts.next < ts.cand.size()) {
@@ -1695,6 +1799,16 @@ int64_t tc_missing_listed(const saige_grm* h) {
 
 void tc_set_wait_budget(long long cycles) {
   g_tc_wait_cycles.store(cycles < 0 ? kWaitCycles : cycles, std::memory_order_relaxed);
+}
+
+// Sets the work division of a launch over `tiles` tiles; returns its grid.
+static unsigned set_work(TcArgs* a, int64_t tiles, int sms) {
+  const TcWork w = tc_work(tiles, a->nk, sms);
+  a->whole = w.whole;
+  a->extra = w.extra;
+  a->tail_tile = w.tail_tile;
+  a->tail_units = w.tail_units;
+  return (unsigned)w.grid;
 }
 
 Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
@@ -1813,6 +1927,13 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->stats.sc_list_launches += lists ? 1 : 0;
     h->n_kv += 1;
   }
+  // a slot for every tile that CTAs share (at most one per CTA boundary)
+  const size_t part_slots = (size_t)p->sms;
+  const size_t part_bytes = part_slots * (2 * kMaxR * kRows * 8 + 4);
+  if (!single && !p->part.ptr) {
+    SG_TRY(p->part.reserve(part_bytes));
+    SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes, st));
+  }
   for (size_t c0 = 0; c0 < (single ? 0 : cols.size()); c0 += kMaxR) {
     const int r = (int)std::min<size_t>(kMaxR, cols.size() - c0);
     const int ng = (int)round_up(3 * r, 16);
@@ -1846,7 +1967,9 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_ld = h->m_pad;
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = (unsigned)(h->m_pad / kRows);
+      const unsigned grid = set_work(&a, h->m_pad / kRows, p->sms);
+      a.part = p->part.as<unsigned long long>();
+      a.part_done = reinterpret_cast<unsigned int*>(a.part + part_slots * 2 * kMaxR * kRows);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<false>(h->device, grid, a, st));
@@ -1892,7 +2015,9 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = (unsigned)(h->n_pad / kRows);
+      const unsigned grid = set_work(&a, h->n_pad / kRows, p->sms);
+      a.part = p->part.as<unsigned long long>();
+      a.part_done = reinterpret_cast<unsigned int*>(a.part + part_slots * 2 * kMaxR * kRows);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<true>(h->device, grid, a, st));
@@ -1925,7 +2050,12 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
   for (cudaEvent_t e : ev) cudaEventDestroy(e);
   if (err & kSrListErr)
     return fail(SAIGE_ECUDA, "one-column GRM product: a missing-call list entry out of range");
-  if (err) return fail(SAIGE_TIMEOUT, "tensor-core GRM product: a pipeline wait timed out");
+  if (err) {
+    // shared tiles may be left half summed
+    if (p->part.ptr) SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    return fail(SAIGE_TIMEOUT, "tensor-core GRM product: a pipeline wait timed out");
+  }
   return Status();
 }
 

@@ -87,11 +87,6 @@ __device__ __forceinline__ void mma_bf16_ss(uint32_t tmem_d, uint64_t adesc, uin
           tmem_d),
       "l"(adesc), "l"(bdesc), "r"(kIdescBf16), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z));
 }
-
-__device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 // Example e of slot s of a pass: the slots of a training step walk the examples with a
 // stride coprime with n_ex from the device step counter; otherwise slot s is example
 // s0 + s.  Held-out examples (sample index (e % n) % holdout == 0) carry no weight.

@@ -24,6 +24,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
                : "memory");
 }
 
+// Arrival of one thread on an mbarrier of its own CTA.
+__device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -89,6 +94,20 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint32_t bar, uint32_t parity,
                                                 volatile int* abort_flag, unsigned int* err,
                                                 long long budget) {
   return mbar_wait_impl<true>(bar, parity, abort_flag, err, budget);
+}
+
+// Wait without back-off (mbarrier.try_wait itself suspends the thread for a while).
+__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, unsigned int* err,
+                                               long long budget) {
+  return mbar_wait_impl<false>(bar, parity, abort_flag, err, budget);
+}
+
+// The same out of line, for callers that test the barrier themselves first.
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity,
+                                                   volatile int* abort_flag, unsigned int* err,
+                                                   long long budget) {
+  return mbar_wait_impl<false>(bar, parity, abort_flag, err, budget);
 }
 
 // Wait for asynchronous work this CTA already issued (its bulk copies, its MMAs),
@@ -159,13 +178,6 @@ __device__ __forceinline__ bool elect_one() {
   return one != 0;
 }
 
-// The lane that elect_one picks.
-__device__ __forceinline__ int elected_lane() {
-  uint32_t lane;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync %0|p, 0xffffffff;\n\t}" : "=r"(lane));
-  return (int)lane;
-}
-
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    bar)
@@ -180,6 +192,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
         "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(taddr));
 }
 
 __device__ __forceinline__ void tmem_wait_ld() {
