@@ -894,15 +894,21 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---------------------------------------------------------------------------
-// Single-column products on the CUDA cores.  With one column the tensor-core
-// passes are bound by their fixed per-stage cost (eight MMAs and the unpack of a
-// 4 KB code tile for three limb columns), so one column costs nearly what 42 do.
-// These kernels form the same exact integer sums with dp4a — the limbs of q as
-// int8 planes, genotypes and missing flags expanded four at a time by byte
-// permutes — and apply the same FP64 epilogue, so their results are bit-identical
-// to the tensor-core path's.  With the missing-call lists of the handle
-// (miss_lists.cuh) the flag sums give way to int64 sums over the ~1 % missing calls,
-// a third fewer instructions per entry for the same integers.
+// Single-column products.  With one column the tcgen05 passes are bound by their fixed
+// per-stage cost (eight MMAs and the unpack of a 4 KB code tile for three limb columns), so
+// one column costs nearly what 42 do.  These kernels form the same exact integer sums and
+// apply the same FP64 epilogue, so their results are bit-identical to the block path's.
+// With the missing-call lists of the handle (miss_lists.cuh) the flag sums give way to int64
+// sums over the ~1 % missing calls, a third fewer instructions per entry for the same
+// integers.
+//
+// What bounds it: the unpack (four masks and four byte permutes per 16 entries, and four
+// more for the flags), then HBM (7.5 GB of codes at 200,000 x 150,000: 1.15 ms per pass).
+// The unpacked bytes stay in registers: they are the A fragments of mma.m16n8k32 over the
+// three limb columns of q (one instruction for 16 x 32 entries), which a tcgen05.mma would
+// want stored to TMEM or shared memory first.  Formed with dp4a (three per four entries and
+// accumulator) the sums took 2.7 and 3.1 ms per pass at 200,000 x 148,979; now 1.82 and 1.79
+// (1.31 without the flags).
 // ---------------------------------------------------------------------------
 // prmt tables of the NEGATED genotype (codes 00, 01, 10, 11 -> -2, 0, -1, 0) and of
 // the missing flag (01 -> 1).  A selector nibble holds the code either in its bits
@@ -912,23 +918,20 @@ __global__ void __launch_bounds__(128)
 // selectors need masks but no shifts.
 constexpr uint32_t kNegGenoX = 0x00FF00FEu, kNegGenoY = 0u;
 constexpr uint32_t kMissX = 0x00000100u, kMissY = 0x00000001u;
-constexpr int kSrWarpMarkers = 8;                        // pass A: markers per warp
-constexpr int kSrBlockMarkers = 8 * kSrWarpMarkers;      // pass A: markers per block
-constexpr int kSrWords = 1024;                           // pass A: sample words staged per round
-constexpr int kSrChunk = 2048;  // markers of limb planes staged per pass-B round
+constexpr int kSrRowsA = 64;     // pass A: markers per block
+constexpr int kSrRowsB = 256;    // pass B: samples per block
+constexpr int kSrChunkA = 4096;  // pass A: samples per chunk of the missing-call lists
+constexpr int kSrChunkB = 1024;  // pass B: markers per chunk
 // error word bit of a one-column product: a missing-call list entry out of range (the
 // entry is skipped; timeouts of the tensor-core pipeline set other bits)
 constexpr unsigned int kSrListErr = 1u << 30;
-// Missing-call entries of a pass-A segment staged at once in shared memory (a block's 64
-// markers x 16,384 samples: ~10,500 calls at 1 % missing); larger segments take several
-// pieces.  (Pass B reads its segments, ~5,200 calls per chunk, from global memory: staging
-// them cost it more resident blocks than the uncoalesced reads cost; 3.89 against 3.09 ms
-// per pass at 200,000 x 150,000.)
-constexpr int kPieceA = 12288;
-// dynamic shared memory of sr_pass_a_kernel: three planes of kSrWords 16-byte words, and
-// with the missing-call lists a piece of entries and one int64 counter per marker
-constexpr size_t sr_pass_a_smem(bool lists) {
-  return 3 * kSrWords * 16 + (lists ? kPieceA * 4 + kSrBlockMarkers * 8 : 0);
+// Missing-call entries of a segment staged in shared memory (2,621 on average at 1 % missing,
+// in both passes); what a segment has beyond them is read from global memory.
+constexpr int kSrPiece = 4096;
+// dynamic shared memory with the lists: two chunks' values and entries, and two counters
+// per row
+constexpr size_t sr_list_smem(int chunk, int rows) {
+  return 2 * 4 * (size_t)(chunk + kSrPiece + rows);
 }
 static_assert(kSamplePad % 256 == 0, "pass B of one column takes sample tiles in pairs");
 
@@ -951,61 +954,120 @@ __device__ __forceinline__ void sr_expand(uint32_t w, int neg_g[4], int miss[4])
   }
 }
 
-// Asynchronous 4-byte copies global -> shared (cp.async), their commit, and the wait
-// for all of this thread's committed copies.
+// Asynchronous copies global -> shared (cp.async) and the wait for all of this thread's
+// committed groups but the latest kLeft.
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
+template <int kLeft>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
 }
 
-// Entries [p0, p0 + n) of a list copied into buf (shared memory) by the block's nt
-// threads, asynchronously: complete after cp_async_wait_all and a barrier.
-__device__ __forceinline__ void stage_piece(uint32_t* buf, const uint32_t* __restrict__ ent,
-                                            int64_t p0, int n, int t, int nt) {
-  for (int i = t; i < n; i += nt) cp_async4(buf + i, ent + p0 + i);
-  cp_async_commit();
-}
+// The missing sums of a block's kRows rows over its segments of the lists: chunk c has the
+// entries ent[seg[c] .. seg[c + 1]), ascending, each (row in block) << bits | (position in
+// chunk), and adds q[c kChunk + position] to the row's sum.  Chunks are staged one ahead of
+// the dense steps; 256 threads.
+template <int kChunk, int kRows_>
+struct SrList {
+  const uint32_t* __restrict__ ent;
+  const int64_t* __restrict__ seg;
+  const int32_t* __restrict__ q;
+  int64_t len;  // values (a multiple of 128)
+  int bits;
+  unsigned int* err;
+  uint32_t* smem;
+  long long sum = 0;  // thread t < kRows_: the sum of row t
 
-// One thread's share of a segment of missing-call entries (tag << bits | position),
-// ascending: the contiguous slice [e0 + t L, e0 + (t + 1) L) of [e0, e1) with L =
-// ceil((e1 - e0) / nt).  Consecutive entries mostly share a tag (a row or a sample), so
-// the thread sums value(position) per run of equal tags in int64 and adds each run to
-// counters[tag] with one shared-memory atomic.  An entry whose tag or position is out of
-// range (tag >= n_tags, position >= n_pos) sets kSrListErr in err and is skipped.
-template <class Value>
-__device__ __forceinline__ void add_slice(const uint32_t* ent, int64_t e0, int64_t e1,
-                                          int t, int nt, int bits, uint32_t n_tags, uint32_t n_pos,
-                                          unsigned long long* counters, unsigned int* err,
-                                          Value value) {
-  const int64_t len = (e1 - e0 + nt - 1) / nt;
-  const int64_t lo = e0 + (int64_t)t * len;
-  const int64_t hi = lo + len < e1 ? lo + len : e1;
-  const uint32_t pmask = (1u << bits) - 1u;
-  uint32_t tag = 0xFFFFFFFFu;
-  long long acc = 0;
-#pragma unroll 4
-  for (int64_t e = lo; e < hi; ++e) {
-    const uint32_t x = ent[e];
-    const uint32_t g = x >> bits, pos = x & pmask;
-    if (g >= n_tags || pos >= n_pos) {
-      atomicOr(err, kSrListErr);
-      continue;
-    }
-    if (g != tag) {
-      if (tag != 0xFFFFFFFFu) atomicAdd(&counters[tag], (unsigned long long)acc);
-      tag = g;
-      acc = 0;
-    }
-    acc += value(pos);
+  __device__ uint32_t* piece(int64_t c) const { return smem + (c & 1) * kSrPiece; }
+  __device__ int32_t* values(int64_t c) const {
+    return reinterpret_cast<int32_t*>(smem + 2 * kSrPiece) + (c & 1) * kChunk;
   }
-  if (tag != 0xFFFFFFFFu) atomicAdd(&counters[tag], (unsigned long long)acc);
-}
+  __device__ int* counters() const {
+    return reinterpret_cast<int*>(smem + 2 * (kSrPiece + kChunk));
+  }
+  __device__ int positions(int64_t c) const {
+    return (int)(len - c * kChunk < kChunk ? len - c * kChunk : kChunk);
+  }
+  // before the first add (a barrier in between)
+  __device__ void init() const {
+    for (int i = threadIdx.x; i < 2 * kRows_; i += 256) counters()[i] = 0;
+  }
+  __device__ void stage(int64_t c) const {
+    const int n = positions(c);
+    int32_t* v = values(c);
+    for (int i = threadIdx.x; 4 * i < n; i += 256) cp_async16(v + 4 * i, q + c * kChunk + 4 * i);
+    const int64_t e0 = __ldg(seg + c), left = __ldg(seg + c + 1) - e0;
+    const int k = (int)(left < kSrPiece ? left : kSrPiece);
+    uint32_t* e = piece(c);
+    for (int i = threadIdx.x; i < k; i += 256) cp_async4(e + i, ent + e0 + i);
+  }
+  // k <= kSrPiece consecutive entries.  A thread takes a contiguous slice (of odd length:
+  // no bank conflicts), whose entries mostly share a row, and adds each run of one row with
+  // two 32-bit atomics: at most 17 values of 24 bits, split at bit 12, so that the counters
+  // of one chunk stay in range.  An entry out of range sets kSrListErr and is skipped.
+  __device__ void add_piece(const uint32_t* e, int k, const int32_t* v, int n) const {
+    const int slice = ((k + 255) >> 8) | 1;
+    const int lo = threadIdx.x * slice, hi = lo + slice < k ? lo + slice : k;
+    const uint32_t pmask = (1u << bits) - 1u;
+    int* cnt = counters();
+    int row = -1, acc = 0;
+    for (int i = lo; i < hi; i += 4) {
+      uint32_t x[4];
+      int val[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = i + j < hi ? e[i + j] : 0xFFFFFFFFu;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) val[j] = (int)(x[j] & pmask) < n ? v[x[j] & pmask] : 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (i + j >= hi) break;
+        const uint32_t g = x[j] >> bits;
+        if (g >= (uint32_t)kRows_ || (int)(x[j] & pmask) >= n) {
+          atomicOr(err, kSrListErr);
+          continue;
+        }
+        if ((int)g != row) {
+          if (row >= 0) {
+            atomicAdd(&cnt[row], acc >> 12);
+            atomicAdd(&cnt[kRows_ + row], acc & 4095);
+          }
+          row = (int)g;
+          acc = 0;
+        }
+        acc += val[j];
+      }
+    }
+    if (row >= 0) {
+      atomicAdd(&cnt[row], acc >> 12);
+      atomicAdd(&cnt[kRows_ + row], acc & 4095);
+    }
+  }
+  // chunk c, staged and waited for; a barrier before and after it
+  __device__ void add(int64_t c) {
+    const int64_t e0 = __ldg(seg + c), left = __ldg(seg + c + 1) - e0;
+    const int n = positions(c);
+    add_piece(piece(c), (int)(left < kSrPiece ? left : kSrPiece), values(c), n);
+    for (int64_t done = kSrPiece; done < left; done += kSrPiece)
+      add_piece(ent + e0 + done, (int)(left - done < kSrPiece ? left - done : kSrPiece), values(c),
+                n);
+    __syncthreads();
+    int* cnt = counters();
+    if (threadIdx.x < kRows_) {
+      sum += 4096LL * cnt[threadIdx.x] + cnt[kRows_ + threadIdx.x];
+      cnt[threadIdx.x] = 0;
+      cnt[kRows_ + threadIdx.x] = 0;
+    }
+  }
+};
 
 // The same groups as bytes of -g only (the missing sums come from the lists).
 __device__ __forceinline__ void sr_expand_g(uint32_t w, int neg_g[4]) {
@@ -1015,12 +1077,87 @@ __device__ __forceinline__ void sr_expand_g(uint32_t w, int neg_g[4]) {
   for (int g = 0; g < 4; ++g) neg_g[g] = (int)prmt(kNegGenoX, kNegGenoY, sel[g]);
 }
 
+// d += a b: a 16 x 32 int8 (row-major fragment), b 32 x 8 int8 (column-major), d int32.
+__device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int a3, uint32_t b0,
+                                       uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A warp's share of one step: kSrTiles row tiles of 16 rows of one 4 KB code tile (128 rows
+// of 32 bytes) against the limb planes.  Lane (g = lane / 4, t = lane % 4) holds words 2t
+// and 2t + 1 of rows g and g + 8 of each row tile, and of plane g (the last plane from there
+// on: columns nobody reads) the 32 limbs of these words' entries.  The fragments' K order is
+// then a permutation of the tile's entries, the same for both operands.
+constexpr int kSrTiles = 4;
+constexpr int kSrWarpRows = 16 * kSrTiles;
+struct SrStep {
+  uint2 a[kSrTiles][2];
+  uint4 b[2];
+};
+
+__device__ __forceinline__ void sr_load(SrStep& s, const uint8_t* __restrict__ rows,
+                                        const int8_t* __restrict__ plane) {
+#pragma unroll
+  for (int k = 0; k < kSrTiles; ++k)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      s.a[k][h] = __ldg(reinterpret_cast<const uint2*>(rows + (16 * k + 8 * h) * 32));
+  s.b[0] = __ldg(reinterpret_cast<const uint4*>(plane));
+  s.b[1] = __ldg(reinterpret_cast<const uint4*>(plane) + 1);
+}
+
+// The step's sums: dg with the bytes of -g, dm (kMiss) with the missing flags.
+template <bool kMiss>
+__device__ __forceinline__ void sr_step(const SrStep& s, int (&dg)[kSrTiles][4],
+                                        int (&dm)[kSrTiles][4]) {
+  const uint32_t b[2][4] = {{s.b[0].x, s.b[0].y, s.b[0].z, s.b[0].w},
+                            {s.b[1].x, s.b[1].y, s.b[1].z, s.b[1].w}};
+#pragma unroll
+  for (int k = 0; k < kSrTiles; ++k)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t w0 = i ? s.a[k][0].y : s.a[k][0].x, w1 = i ? s.a[k][1].y : s.a[k][1].x;
+      int g0[4], g1[4];
+      if constexpr (kMiss) {
+        int m0[4], m1[4];
+        sr_expand(w0, g0, m0);
+        sr_expand(w1, g1, m1);
+        mma_s8(dm[k], m0[0], m1[0], m0[1], m1[1], b[i][0], b[i][1]);
+        mma_s8(dm[k], m0[2], m1[2], m0[3], m1[3], b[i][2], b[i][3]);
+      } else {
+        sr_expand_g(w0, g0);
+        sr_expand_g(w1, g1);
+      }
+      mma_s8(dg[k], g0[0], g1[0], g0[1], g1[1], b[i][0], b[i][1]);
+      mma_s8(dg[k], g0[2], g1[2], g0[3], g1[3], b[i][2], b[i][3]);
+    }
+}
+
+// Adds a warp's sums to red[row][column]: columns c0 .. c0 + 2 of d to columns at .. at + 2.
+__device__ __forceinline__ void sr_add(int (*red)[6], int row0, const int (&d)[kSrTiles][4],
+                                       int c0, int at) {
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+  for (int k = 0; k < kSrTiles; ++k)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int row = row0 + 16 * k + 8 * (e >> 1) + g, c = 2 * t + (e & 1) - c0;
+      if (c >= 0 && c < 3) atomicAdd(&red[row][at + c], d[k][e]);
+    }
+}
+
 // q = rint(x / scale) as in quant_v_kernel, into three int8 planes (l2, l1, l0) of
-// length n_pad (zero past len), and sum q.
+// length n_pad (zero past len) and, when q32 is given, as int32 (|q| <= 127 * 2^16); and
+// sum q.
 __global__ void __launch_bounds__(256)
     sr_quant_v_kernel(const double* __restrict__ v, int64_t len, int64_t n_pad,
                       const unsigned long long* __restrict__ amax, double* __restrict__ scale_out,
-                      int8_t* __restrict__ planes, unsigned long long* __restrict__ sum_q) {
+                      int8_t* __restrict__ planes, int32_t* __restrict__ q32,
+                      unsigned long long* __restrict__ sum_q) {
   __shared__ long long sh[8];
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   const double sc = scale_of(amax[0]);
@@ -1033,6 +1170,7 @@ __global__ void __launch_bounds__(256)
     planes[i] = (int8_t)l2;
     planes[n_pad + i] = (int8_t)l1;
     planes[2 * n_pad + i] = (int8_t)l0;
+    if (q32) q32[i] = (int32_t)q;
   }
   long long t = q;
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -1091,356 +1229,171 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Pass A of one column: block = 64 markers x all samples, warp = 8 markers.  The
-// limb planes of q are staged in shared memory kSrWords words (16 samples each) at a
-// time and shared by the block's warps; each lane keeps the six sums of its warp's 8
-// markers over its words, and the warp's sums are finished as in the tensor-core
-// epilogue.  With kLists the lanes keep the three genotype sums only: after each chunk
-// the block adds q (rebuilt from its staged limbs) over the missing calls of its markers
-// in the chunk — one segment of miss_ent, each entry (marker in block) << bits | (sample
-// in chunk) — into per-marker int64 counters: the same integer Mi the flag sums give.
-template <bool kLists>
-__global__ void __launch_bounds__(256, 2)
-    sr_pass_a_kernel(const uint32_t* __restrict__ geno, int64_t wpr,
-                     const int8_t* __restrict__ planes, int64_t n_pad,
-                     const unsigned long long* __restrict__ sum_q,
-                     const double* __restrict__ scale_v, const double* __restrict__ two_p,
-                     const double* __restrict__ inv_s, const uint32_t* __restrict__ miss_ent,
-                     const int64_t* __restrict__ miss_seg, int64_t nch, int bits,
-                     unsigned int* __restrict__ err, double* __restrict__ u) {
-  constexpr int kSums = kLists ? 3 : 6;
-  // dynamic shared memory (sr_pass_a_smem bytes): the three staged limb planes, then
-  // with kLists the per-marker missing sums and a piece of the chunk's entries
-  extern __shared__ uint4 sr_dyn[];
-  uint4(*sp)[kSrWords] = reinterpret_cast<uint4(*)[kSrWords]>(sr_dyn);
-  unsigned long long* mi_s = reinterpret_cast<unsigned long long*>(sr_dyn + 3 * kSrWords);
-  uint32_t* piece = reinterpret_cast<uint32_t*>(mi_s + kSrBlockMarkers);
-  if constexpr (kLists) {
-    if (threadIdx.x < kSrBlockMarkers) mi_s[threadIdx.x] = 0ull;
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t m0 = (int64_t)blockIdx.x * kSrBlockMarkers + warp * kSrWarpMarkers;
-  const uint32_t* rows = geno + m0 * wpr;
-  int acc[kSrWarpMarkers][kSums];
-#pragma unroll
-  for (int k = 0; k < kSrWarpMarkers; ++k)
-#pragma unroll
-    for (int j = 0; j < kSums; ++j) acc[k][j] = 0;
-  const int64_t n_words = n_pad / 16;
-  for (int64_t c0 = 0; c0 < n_words; c0 += kSrWords) {
-    const int cn = n_words - c0 < kSrWords ? (int)(n_words - c0) : kSrWords;
-    int64_t e0 = 0, e1 = 0;  // kLists: this chunk's segment
-    if constexpr (kLists) {
-      const int64_t* sg = miss_seg + (int64_t)blockIdx.x * nch + c0 / kSrWords;
-      e0 = sg[0];
-      e1 = sg[1];
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 3 * kSrWords; t += 256) {
-      const int pl = t / kSrWords, k = t % kSrWords;
-      sp[pl][k] = k < cn ? __ldg(reinterpret_cast<const uint4*>(planes + pl * n_pad) + c0 + k)
-                         : make_uint4(0u, 0u, 0u, 0u);
-    }
-    // kLists: the segment's first piece lands while the dense loop runs
-    if constexpr (kLists)
-      stage_piece(piece, miss_ent, e0, (int)(e1 - e0 < kPieceA ? e1 - e0 : kPieceA), threadIdx.x,
-                  256);
-    __syncthreads();
-#pragma unroll 4
-    for (int t = lane; t < cn; t += 32) {
-      uint32_t w[kSrWarpMarkers];
-#pragma unroll
-      for (int k = 0; k < kSrWarpMarkers; ++k) w[k] = __ldg(rows + k * wpr + c0 + t);
-      const uint4 a2 = sp[0][t], a1 = sp[1][t], a0 = sp[2][t];
-      const int l2[4] = {(int)a2.x, (int)a2.y, (int)a2.z, (int)a2.w};
-      const int l1[4] = {(int)a1.x, (int)a1.y, (int)a1.z, (int)a1.w};
-      const int l0[4] = {(int)a0.x, (int)a0.y, (int)a0.z, (int)a0.w};
-#pragma unroll
-      for (int k = 0; k < kSrWarpMarkers; ++k) {
-        if constexpr (kLists) {
-          int gbs[4];
-          sr_expand_g(w[k], gbs);
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            acc[k][0] = __dp4a(gbs[g], l2[g], acc[k][0]);
-            acc[k][1] = __dp4a(gbs[g], l1[g], acc[k][1]);
-            acc[k][2] = __dp4a(gbs[g], l0[g], acc[k][2]);
-          }
-        } else {
-          int gbs[4], mbs[4];
-          sr_expand(w[k], gbs, mbs);
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const int gb = gbs[g], mb = mbs[g];
-            acc[k][0] = __dp4a(gb, l2[g], acc[k][0]);
-            acc[k][1] = __dp4a(gb, l1[g], acc[k][1]);
-            acc[k][2] = __dp4a(gb, l0[g], acc[k][2]);
-            acc[k][3] = __dp4a(mb, l2[g], acc[k][3]);
-            acc[k][4] = __dp4a(mb, l1[g], acc[k][4]);
-            acc[k][5] = __dp4a(mb, l0[g], acc[k][5]);
-          }
-        }
-      }
-    }
-    if constexpr (kLists) {
-      const int8_t* p2 = reinterpret_cast<const int8_t*>(sp[0]);
-      const int8_t* p1 = reinterpret_cast<const int8_t*>(sp[1]);
-      const int8_t* p0 = reinterpret_cast<const int8_t*>(sp[2]);
-      for (int64_t q0 = e0; q0 < e1; q0 += kPieceA) {  // uniform over the block
-        const int n = (int)(e1 - q0 < kPieceA ? e1 - q0 : kPieceA);
-        if (q0 != e0) {  // a later piece: after the last one's slices are done
-          __syncthreads();
-          stage_piece(piece, miss_ent, q0, n, threadIdx.x, 256);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        add_slice(piece, 0, n, threadIdx.x, 256, bits, kSrBlockMarkers, 16u * (uint32_t)cn, mi_s,
-                  err, [&](uint32_t s) {
-                    return 65536LL * p2[s] + 256LL * p1[s] + (long long)p0[s];
-                  });
-      }
-    }
-  }
-  if constexpr (kLists) __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kSrWarpMarkers; ++k)
-#pragma unroll
-    for (int j = 0; j < kSums; ++j)
-      for (int o = 16; o > 0; o >>= 1) acc[k][j] += __shfl_xor_sync(0xffffffffu, acc[k][j], o);
-  const double S = (double)(long long)sum_q[0];
-#pragma unroll
-  for (int k = 0; k < kSrWarpMarkers; ++k) {
-    if (lane != k) continue;
-    const int64_t m = m0 + k;
-    // the genotype sums were formed with -g; Mi is the same integer either way
-    const double G = -(65536.0 * (double)acc[k][0] + 256.0 * (double)acc[k][1] + (double)acc[k][2]);
-    double Mi;
-    if constexpr (kLists)
-      Mi = (double)(long long)mi_s[warp * kSrWarpMarkers + k];
-    else
-      Mi = 65536.0 * (double)acc[k][kSums - 3] + 256.0 * (double)acc[k][kSums - 2] +
-           (double)acc[k][kSums - 1];
-    const double tt = __dsub_rn(G, __dmul_rn(two_p[m], S - Mi));
-    u[m] = __dmul_rn(inv_s[m], __dmul_rn(scale_v[0], tt));
-  }
-}
-
-// How one-column pass B divides the markers: units of kSrChunk / sub markers, `units`
-// of them per block, n_units in all, over `blocks` blocks per pair of sample tiles.
-struct SrSplitB {
-  int sub;
-  int64_t units, n_units;
+// How a one-column pass divides the columns of its code tiles: `tiles` per block, `blocks`
+// blocks per row block, chosen for the shortest sum of waves x (tiles + ends), ends being what
+// a block's first loads and last sums cost in tiles (more where partial sums meet), fitted to
+// the times below.  A cohort's row blocks alone neither fill the SMs (n = 9,001: 36 in pass B)
+// nor come in whole waves.  us undivided / with pass B divided into 12 blocks per SM / now:
+//                         pass A        pass B
+//   200,000 x 148,979     1808 / -  / 1823   -  / 1847 / 1788
+//   100,000 x  49,000      348 / -  /  324   -  /  320 /  305
+//     9,001 x  21,011     20.0 / -  / 20.4   -  / 27.6 / 18.3
+//    30,000 x   9,033     23.3 / -  / 24.8   -  / 35.9 / 25.0
+//     2,000 x   4,077      4.0 / -  /  4.1   -  /  5.8 /  6.0
+struct SrSplit {
+  int64_t tiles;
   unsigned blocks;
 };
 
-// The line: kSrBlocksB blocks per SM in all.  Fewer than that many (pair of tiles, chunk)
-// units: the chunks are divided (up to one 128-marker tile per unit) until there are;
-// more: a block takes several chunks, so that its planes' staging and its sums at the
-// end stay small beside the dense loop.
-constexpr int64_t kSrBlocksB = 24;
-
-SrSplitB sr_split_b(int64_t n_pad, int64_t m_pad) {
-  const int64_t pairs = n_pad / (2 * kRows), chunks = ceil_div(m_pad, (int64_t)kSrChunk);
-  const int64_t want = 148 * kSrBlocksB;
-  SrSplitB s;
-  s.sub = 1;
-  while (s.sub < kSrChunk / 128 && pairs * chunks * s.sub * 4 < want) s.sub *= 2;
-  s.n_units = ceil_div(m_pad, (int64_t)(kSrChunk / s.sub));
-  const int64_t blocks = std::max<int64_t>(1, std::min(s.n_units, want / pairs));
-  s.units = ceil_div(s.n_units, blocks);
-  s.blocks = (unsigned)ceil_div(s.n_units, s.units);
-  return s;
+SrSplit sr_split(int64_t row_blocks, int64_t n_kt, int sms, int64_t ends, int64_t ends_split) {
+  const int64_t slots = 2 * (int64_t)sms;  // two blocks per SM are resident
+  SrSplit best{n_kt, 1};
+  int64_t least = ceil_div(row_blocks, slots) * (n_kt + ends);
+  for (int64_t b = 2; b <= std::min<int64_t>(n_kt, 64); ++b) {
+    const int64_t tiles = ceil_div(n_kt, b), blocks = ceil_div(n_kt, tiles);
+    const int64_t cost = ceil_div(row_blocks * blocks, slots) * (tiles + ends_split);
+    if (cost < least) {
+      least = cost;
+      best = SrSplit{tiles, (unsigned)blocks};
+    }
+  }
+  return best;
 }
 
-// Pass B of one column: block = two 128-sample tiles of tiles_s (thread = one sample of
-// each; the limb words it loads serve both) x a range of marker units.  A unit is a
-// chunk of kSrChunk markers or one of its `sub` equal parts; the unit's limb planes are
-// staged in shared memory.  With kLists the c planes give way to qc itself (qc32), and
-// the block adds qc over its part of the chunk's segment of missing calls — entries
-// (sample in block) << bits | (marker in chunk) — into per-sample int64 counters: the
-// integer Mi the flag sums give.
+struct SrArgs {
+  const uint8_t* tiles;   // A: tiles_m; B: tiles_s
+  int64_t ld;             // tiles from one row of tiles to the next
+  int64_t n_kt;           // column tiles
+  const int8_t* planes;   // A: three limb planes of v; B: of w, then of c
+  SrSplit split;
+  // with the missing-call lists
+  const int32_t* q32;     // A: the quantised v; B: c
+  const uint32_t* ent;
+  const int64_t* seg;
+  int64_t nch;
+  int bits;
+  unsigned int* err;
+  // per row, and tickets per row block (when a pass is divided): zero between launches
+  unsigned long long *sums_g, *sums_m;
+  unsigned int* tickets;
+  const unsigned long long* sum_q;  // A: sum q_v; B: sum q_c
+  const double *scale_g, *scale_m;  // A: scale of v (scale_m unused); B: of w and of c
+  const double *two_p, *inv_s;      // A
+  double out_scale;                 // B: 1 / M
+  double* out;                      // A: u; B: the product's column
+};
+
+// One pass of a one-column product: block = kSrRowsA markers (pass A) or kSrRowsB samples
+// (pass B; two tiles) x a range of column tiles.  A warp has 64 rows; the warps of the same
+// rows take the column tiles in turn, the next step's loads in flight, and their sums meet in
+// shared memory.  Without kLists the flag sums are a second set of accumulators over the same
+// limbs; in pass B, whose flags go with c, the planes of w and of c are the six columns of one
+// B fragment: the genotype sums are its first three, the flag sums its last three.  With
+// kLists the missing sums come from the handle's lists, a chunk falling to the block that has
+// its first tile: the same integers the flags give.
 //
-// Bound: integer issue (dp4a) once every SM has warps enough to hide the loads of the
-// codes.  The markers are split over blockIdx.y because a cohort's sample tiles alone do
-// not fill 148 SMs: at n = 9,001 they are 36 blocks of four warps, each walking all
-// m = 20,900 markers (331 us; 47 us split), and at n = 200,000, m = 150,000 they are 782
-// blocks, 5.3 per SM, where the SMs with six take 13 % longer (3.65 ms; 3.06 ms split).  The sums
-// are integers, so partial sums meet in sums_g / sums_m (int64 per sample, atomics) in any
-// order with the same result; the block that takes the last ticket of its sample tiles
-// runs the epilogue and leaves the sums and the ticket at zero for the next product.
-template <bool kLists>
-__global__ void __launch_bounds__(128)
-    sr_pass_b_kernel(const uint8_t* __restrict__ tiles_s, int64_t n_mt, int64_t s_ld,
-                     const int8_t* __restrict__ planes, int64_t m_pad,
-                     const unsigned long long* __restrict__ sum_c,
-                     const double* __restrict__ scale_w, const double* __restrict__ scale_c,
-                     const int32_t* __restrict__ qc32, const uint32_t* __restrict__ miss_ent,
-                     const int64_t* __restrict__ miss_seg, int64_t nch, int bits,
-                     unsigned int* __restrict__ err, SrSplitB split,
-                     unsigned long long* __restrict__ sums_g,
-                     unsigned long long* __restrict__ sums_m, unsigned int* __restrict__ tickets,
-                     double out_scale, double* __restrict__ out) {
-  constexpr int kPlanes = kLists ? 3 : 6;
-  __shared__ __align__(16) int8_t sp[kPlanes][kSrChunk];
-  __shared__ __align__(16) int32_t sq[kLists ? kSrChunk : 4];
-  const int64_t st0 = 2 * (int64_t)blockIdx.x;
-  const int r = threadIdx.x;
-  int acc[2][kPlanes];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int e = 0; e < kPlanes; ++e) acc[h][e] = 0;
-  __shared__ unsigned long long mi_s[kLists ? 2 * kRows : 1];
+// The sums are integers, so the partial sums of the blocks of one row block meet in sums_g /
+// sums_m (int64 per row, atomics) in any order with the same result; the block that takes the
+// last ticket runs the epilogue and leaves the sums and the ticket at zero for the next pass.
+template <bool kPassB, bool kLists>
+__global__ void __launch_bounds__(256, 2) sr_pass_kernel(SrArgs a) {
+  constexpr int kRowsBlk = kPassB ? kSrRowsB : kSrRowsA;
+  constexpr int kRowGroups = kRowsBlk / kSrWarpRows, kColGroups = 8 / kRowGroups;
+  constexpr int kChunk = kPassB ? kSrChunkB : kSrChunkA;
+  constexpr int64_t kChunkTiles = kChunk / kKt;
+  extern __shared__ uint4 sr_dyn[];
+  __shared__ int red[kRowsBlk][6];
+  const int r = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = r; i < kRowsBlk * 6; i += 256) (&red[0][0])[i] = 0;
+  const int64_t t0 = (int64_t)blockIdx.y * a.split.tiles;
+  const int64_t t1 = min(t0 + a.split.tiles, a.n_kt), k_len = a.n_kt * kKt;
+  const int64_t c0 = (t0 + kChunkTiles - 1) / kChunkTiles, c1 = (t1 + kChunkTiles - 1) / kChunkTiles;
+  SrList<kChunk, kRowsBlk> list{a.ent, a.seg + (int64_t)blockIdx.x * a.nch, a.q32, k_len, a.bits,
+                                a.err, reinterpret_cast<uint32_t*>(sr_dyn)};
   if constexpr (kLists) {
-    mi_s[r] = 0ull;
-    mi_s[kRows + r] = 0ull;
+    list.init();
+    if (c0 < c1) list.stage(c0);
+    cp_async_commit();
   }
-  const int64_t tiles_per_unit = (kSrChunk / 128) / split.sub;
-  const int64_t u_end = min((int64_t)(blockIdx.y + 1) * split.units, split.n_units);
-  for (int64_t unit = (int64_t)blockIdx.y * split.units; unit < u_end; ++unit) {
-    const int64_t chunk = unit / split.sub;
-    const int part = (int)(unit - chunk * split.sub);
-    const int64_t mt0 = unit * tiles_per_unit;
-    const int64_t base = mt0 * 128;
-    const int64_t cbase = chunk * kSrChunk;  // kLists: the segment's positions count from here
-    const int len = (int)max((int64_t)0, min(m_pad - base, tiles_per_unit * 128));
-    const int clen = (int)min(m_pad - cbase, (int64_t)kSrChunk);
-    int64_t e0 = 0, e1 = 0;  // kLists: this unit's part of the chunk's segment
-    if constexpr (kLists) {
-      const int64_t* sg = miss_seg + (int64_t)blockIdx.x * nch + chunk;
-      // the last chunk may have fewer parts than sub
-      const int64_t left = split.n_units - chunk * split.sub;
-      const int64_t parts = left < split.sub ? left : split.sub;
-      const int64_t s0 = sg[0], cnt = sg[1] - sg[0];
-      e0 = s0 + cnt * part / parts;
-      e1 = s0 + cnt * (part + 1) / parts;
+  const int row0 = (warp % kRowGroups) * kSrWarpRows;
+  const int64_t grow = (int64_t)blockIdx.x * kRowsBlk + row0;
+  const uint8_t* rows = a.tiles + grow / kRows * a.ld * kTileBytes +
+                        (grow % kRows + (lane >> 2)) * 32 + (lane & 3) * 8;
+  const int8_t* plane = a.planes + min(lane >> 2, kPassB && !kLists ? 5 : 2) * k_len +
+                        (lane & 3) * 32;
+  int dg[kSrTiles][4] = {}, dm[kSrTiles][4] = {};
+  SrStep cur, next;
+  int64_t kt = t0 + warp / kRowGroups;
+  if (kt < t1) sr_load(cur, rows + kt * kTileBytes, plane + kt * kKt);
+  auto dense = [&](int64_t end) {
+    for (; kt < end; kt += kColGroups) {
+      const int64_t to = kt + kColGroups;
+      if (to < t1) sr_load(next, rows + to * kTileBytes, plane + to * kKt);
+      sr_step<!kLists>(cur, dg, dm);
+      cur = next;
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < kPlanes * (kSrChunk / 16); t += 128) {
-      const int pl = t / (kSrChunk / 16), k = t % (kSrChunk / 16);
-      if (16 * k < len)
-        reinterpret_cast<uint4*>(sp[pl])[k] =
-            __ldg(reinterpret_cast<const uint4*>(planes + (int64_t)pl * m_pad + base) + k);
-    }
-    if constexpr (kLists) {
-      for (int t = threadIdx.x; t < kSrChunk / 4; t += 128) {
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (4 * t < clen) v = __ldg(reinterpret_cast<const uint4*>(qc32 + cbase) + t);
-        reinterpret_cast<uint4*>(sq)[t] = v;
-      }
-    }
-    __syncthreads();
-    const int64_t mt_end = mt0 + len / 128;
-#pragma unroll 2
-    for (int64_t mt = mt0; mt < mt_end; ++mt) {
-      uint32_t words[2][8];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint4* row = reinterpret_cast<const uint4*>(
-            tiles_s + ((st0 + h) * s_ld + mt) * kTileBytes + (int64_t)r * 32);
-        const uint4 h0 = __ldg(row), h1 = __ldg(row + 1);
-        words[h][0] = h0.x; words[h][1] = h0.y; words[h][2] = h0.z; words[h][3] = h0.w;
-        words[h][4] = h1.x; words[h][5] = h1.y; words[h][6] = h1.z; words[h][7] = h1.w;
-      }
-      const int off = (int)(mt - mt0) * 128;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int mk = off + 16 * j;
-        const uint4 w2 = *reinterpret_cast<const uint4*>(sp[0] + mk);
-        const uint4 w1 = *reinterpret_cast<const uint4*>(sp[1] + mk);
-        const uint4 w0 = *reinterpret_cast<const uint4*>(sp[2] + mk);
-        const int W2[4] = {(int)w2.x, (int)w2.y, (int)w2.z, (int)w2.w};
-        const int W1[4] = {(int)w1.x, (int)w1.y, (int)w1.z, (int)w1.w};
-        const int W0[4] = {(int)w0.x, (int)w0.y, (int)w0.z, (int)w0.w};
-        if constexpr (kLists) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            int gbs[4];
-            sr_expand_g(words[h][j], gbs);
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              acc[h][0] = __dp4a(gbs[g], W2[g], acc[h][0]);
-              acc[h][1] = __dp4a(gbs[g], W1[g], acc[h][1]);
-              acc[h][2] = __dp4a(gbs[g], W0[g], acc[h][2]);
-            }
-          }
-        } else {
-          const uint4 c2 = *reinterpret_cast<const uint4*>(sp[kPlanes - 3] + mk);
-          const uint4 c1 = *reinterpret_cast<const uint4*>(sp[kPlanes - 2] + mk);
-          const uint4 c0 = *reinterpret_cast<const uint4*>(sp[kPlanes - 1] + mk);
-          const int C2[4] = {(int)c2.x, (int)c2.y, (int)c2.z, (int)c2.w};
-          const int C1[4] = {(int)c1.x, (int)c1.y, (int)c1.z, (int)c1.w};
-          const int C0[4] = {(int)c0.x, (int)c0.y, (int)c0.z, (int)c0.w};
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            int gbs[4], mbs[4];
-            sr_expand(words[h][j], gbs, mbs);
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              acc[h][0] = __dp4a(gbs[g], W2[g], acc[h][0]);
-              acc[h][1] = __dp4a(gbs[g], W1[g], acc[h][1]);
-              acc[h][2] = __dp4a(gbs[g], W0[g], acc[h][2]);
-              acc[h][kPlanes - 3] = __dp4a(mbs[g], C2[g], acc[h][kPlanes - 3]);
-              acc[h][kPlanes - 2] = __dp4a(mbs[g], C1[g], acc[h][kPlanes - 2]);
-              acc[h][kPlanes - 1] = __dp4a(mbs[g], C0[g], acc[h][kPlanes - 1]);
-            }
-          }
-        }
-      }
-    }
-    if constexpr (kLists) {
-      add_slice(miss_ent, e0, e1, threadIdx.x, 128, bits, 2u * kRows, (uint32_t)clen, mi_s, err,
-                [&](uint32_t mk) { return (long long)sq[mk]; });
+  };
+  if constexpr (kLists) {
+    for (int64_t c = c0; c < c1; ++c) {
+      if (c + 1 < c1) list.stage(c + 1);
+      cp_async_commit();
+      dense(min(t1, (c + 1) * kChunkTiles));
+      cp_async_wait<1>();
+      __syncthreads();
+      list.add(c);
     }
   }
-  if constexpr (kLists) __syncthreads();
-  // this block's integer sums per sample: G (formed with -g) and Mi
-  long long g[2], mi[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    g[h] = 65536LL * acc[h][0] + 256LL * acc[h][1] + (long long)acc[h][2];
+  dense(t1);
+  __syncthreads();  // red is zero
+  sr_add(red, row0, dg, 0, 0);
+  if constexpr (!kLists) sr_add(red, row0, dm, kPassB ? 3 : 0, 3);
+  __syncthreads();
+  // this block's integer sums of row r: G (formed with -g) and Mi
+  const int64_t i = (int64_t)blockIdx.x * kRowsBlk + r;
+  const bool mine = r < kRowsBlk;
+  long long g = 0, mi = 0;
+  if (mine) {
+    const int* d = red[r];
+    g = 65536LL * d[0] + 256LL * d[1] + (long long)d[2];
     if constexpr (kLists)
-      mi[h] = (long long)mi_s[h * kRows + r];
+      mi = list.sum;
     else
-      mi[h] = 65536LL * acc[h][kPlanes - 3] + 256LL * acc[h][kPlanes - 2] +
-              (long long)acc[h][kPlanes - 1];
+      mi = 65536LL * d[3] + 256LL * d[4] + (long long)d[5];
   }
   if (gridDim.y > 1) {
     __shared__ int last_s;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t i = (st0 + h) * 128 + r;
-      atomicAdd(&sums_g[i], (unsigned long long)g[h]);
-      atomicAdd(&sums_m[i], (unsigned long long)mi[h]);
+    if (mine) {
+      atomicAdd(&a.sums_g[i], (unsigned long long)g);
+      atomicAdd(&a.sums_m[i], (unsigned long long)mi);
     }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-      const bool last = atomicAdd(&tickets[blockIdx.x], 1u) == gridDim.y - 1;
-      if (last) tickets[blockIdx.x] = 0u;
+      const bool last = atomicAdd(&a.tickets[blockIdx.x], 1u) == gridDim.y - 1;
+      if (last) a.tickets[blockIdx.x] = 0u;
       last_s = last ? 1 : 0;
     }
     __syncthreads();
     if (!last_s) return;
     __threadfence();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t i = (st0 + h) * 128 + r;
-      g[h] = (long long)__ldcg(&sums_g[i]);
-      mi[h] = (long long)__ldcg(&sums_m[i]);
-      sums_g[i] = 0ull;
-      sums_m[i] = 0ull;
+    if (mine) {
+      g = (long long)__ldcg(&a.sums_g[i]);
+      mi = (long long)__ldcg(&a.sums_m[i]);
+      a.sums_g[i] = 0ull;
+      a.sums_m[i] = 0ull;
     }
   }
-  const double S = (double)(long long)sum_c[0];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    // both integers are below 2^53: exact in FP64, as the limb sums of the tensor-core
-    // epilogue are
-    const double G = -(double)g[h];
-    const double Mi = (double)mi[h];
-    out[(st0 + h) * 128 + r] = __dmul_rn(
-        out_scale, __dsub_rn(__dmul_rn(scale_w[0], G), __dmul_rn(scale_c[0], S - Mi)));
+  if (!mine) return;
+  // both integers are below 2^53: exact in FP64, as the limb sums of the block path's
+  // epilogue are
+  const double S = (double)(long long)a.sum_q[0];
+  const double G = -(double)g, Mi = (double)mi;
+  if constexpr (kPassB) {
+    a.out[i] = __dmul_rn(a.out_scale, __dsub_rn(__dmul_rn(a.scale_g[0], G),
+                                                __dmul_rn(a.scale_m[0], S - Mi)));
+  } else {
+    const double tt = __dsub_rn(G, __dmul_rn(a.two_p[i], S - Mi));
+    a.out[i] = __dmul_rn(a.inv_s[i], __dmul_rn(a.scale_g[0], tt));
   }
 }
 
@@ -1513,20 +1466,25 @@ struct TcPlan {
   int sms = 0;
   int64_t s_ld = 0;  // tiles_s: marker tiles per sample tile (>= m_pad / 128)
   bool tracing = false;
-  // one-column products: the missing-call lists and qc as int32 (m_pad) for pass B's
-  // sums over them
-  MissLists miss;
-  DevBuf sr_qc;
-  DevBuf sr_sums;  // pass B's sums over its marker splits and its tickets: zero between products
+  MissLists miss;  // one-column products: the missing-call lists
+  DevBuf sr_q32;   // with them: the quantised v (n_pad) and c (m_pad) as int32
+  DevBuf sr_sums;  // the divided passes' sums and tickets: zero between launches
 };
 
 // The missing-call lists cost about two products' time to build (four passes over the
 // codes) and 8 bytes per missing call, while a fit runs four or five one-column products:
-// a handle builds them at the first one-column product of its second AI-REML fit, so a
-// single fit (with its variance ratio) keeps the dense flag sums and repeated fits on a
-// handle (refits, LOCO) take the lists.
+// a handle counts its missing calls at the first one-column product of its second AI-REML
+// fit, and lists them if the lists are then the cheaper of the two.  The flags cost about
+// 0.5 ms per pass at 200,000 x 148,979 whatever the calls; the lists 1.1-1.4 ms at 1 %
+// missing, in proportion to the calls (9,001 x 21,011: 28 and 25 us against 20 and 18): the
+// line is 0.3 %.  In handles of a few million entries the launch is most of either (3,000 x
+// 779 at 1 %: 5.6 + 6.4 us against 4.7 + 5.1), and the lists are kept, as their statistics
+// report them.
 // SAIGE_SR_LISTS: 0 keeps the dense missing-flag sums, 2 builds the lists at a handle's
-// first one-column product, otherwise (default) in its second fit.
+// first one-column product, otherwise (default) by the rule above.
+constexpr double kSrListFrac = 0.003;
+constexpr int64_t kSrListSmall = (int64_t)1 << 22;
+
 static int sr_lists_mode() {
   const char* e = getenv("SAIGE_SR_LISTS");
   if (!e || !e[0]) return 1;
@@ -1604,10 +1562,14 @@ static Status tc_plan_new(TcPlan** out) {
     if (e != cudaSuccess)
       return bail(fail(SAIGE_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)));
   }
-  for (bool lists : {false, true}) {
-    cudaError_t e = cudaFuncSetAttribute(
-        lists ? sr_pass_a_kernel<true> : sr_pass_a_kernel<false>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr_pass_a_smem(lists));
+  {
+    cudaError_t e = cudaFuncSetAttribute(sr_pass_kernel<false, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sr_list_smem(kSrChunkA, kSrRowsA));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(sr_pass_kernel<true, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sr_list_smem(kSrChunkB, kSrRowsB));
     if (e != cudaSuccess)
       return bail(fail(SAIGE_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)));
   }
@@ -1923,15 +1885,19 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     int8_t* planes_b = p->img_w.as<int8_t>();  // 6 x m_pad limb planes of qw, qc
     double* u = p->u.as<double>();
     const int lmode = sr_lists_mode();
-    if (p->miss.state == 0 && (lmode == 2 || (lmode == 1 && h->n_fits >= 2)))
-      SG_TRY(miss_lists_build(h, p->tiles_s.as<uint8_t>(), p->s_ld,
-                              MissShape{kSrBlockMarkers, kSrWords, 2 * kRows, kSrChunk}, &p->miss,
-                              st));
+    if ((p->miss.state == 0 && (lmode == 2 || (lmode == 1 && h->n_fits >= 2))) ||
+        (p->miss.state == kMissListsLeft && lmode == 2))
+      SG_TRY(miss_lists_build(
+          h, p->tiles_s.as<uint8_t>(), p->s_ld,
+          MissShape{kSrRowsA, kSrChunkA / 16, kSrRowsB, kSrChunkB},
+          lmode == 2 || h->m_pad * h->n_pad <= kSrListSmall ? kMissListMaxFrac : kSrListFrac,
+          &p->miss, st));
     const bool lists = p->miss.state == 1 && lmode != 0;
-    int32_t* qc32 = nullptr;
+    int32_t *qv32 = nullptr, *qc32 = nullptr;
     if (lists) {
-      SG_TRY(p->sr_qc.reserve((size_t)h->m_pad * sizeof(int32_t)));
-      qc32 = p->sr_qc.as<int32_t>();
+      SG_TRY(p->sr_q32.reserve((size_t)(h->n_pad + h->m_pad) * sizeof(int32_t)));
+      qv32 = p->sr_q32.as<int32_t>();
+      qc32 = qv32 + h->n_pad;
     }
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     SG_TRY(mark(&t0));
@@ -1941,48 +1907,72 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     amax_v_kernel<<<(unsigned)ceil_div(h->n, kAmaxRows), 256, 0, st>>>(v, h->n_pad, h->n, cm,
                                                                        sc.amax_v);
     sr_quant_v_kernel<<<(unsigned)ceil_div(h->n_pad, 256), 256, 0, st>>>(
-        v + (int64_t)cols[0] * h->n_pad, h->n, h->n_pad, sc.amax_v, sc.scale_v, planes_a, sc.sum_v);
+        v + (int64_t)cols[0] * h->n_pad, h->n, h->n_pad, sc.amax_v, sc.scale_v, planes_a, qv32,
+        sc.sum_v);
+    const unsigned blocks_a = (unsigned)(h->m_pad / kSrRowsA);
+    const unsigned blocks_b = (unsigned)(h->n_pad / kSrRowsB);  // (n_pad: a multiple of 512)
+    SrArgs a{};
+    a.split = sr_split(blocks_a, n_stages_a, p->sms, 12, 26);
+    SrArgs b{};
+    b.split = sr_split(blocks_b, n_stages_b, p->sms, 5, 5);
+    if ((a.split.blocks > 1 || b.split.blocks > 1) && !p->sr_sums.ptr) {
+      const size_t bytes = (size_t)std::max(h->n_pad, h->m_pad) * 16 +
+                           (size_t)std::max(blocks_a, blocks_b) * 4;
+      SG_TRY(p->sr_sums.reserve(bytes));
+      SG_CUDA(cudaMemsetAsync(p->sr_sums.ptr, 0, bytes, st));
+    }
+    a.sums_g = p->sr_sums.as<unsigned long long>();
+    a.sums_m = a.sums_g + std::max(h->n_pad, h->m_pad);
+    a.tickets = reinterpret_cast<unsigned int*>(a.sums_m + std::max(h->n_pad, h->m_pad));
+    b.sums_g = a.sums_g;
+    b.sums_m = a.sums_m;
+    b.tickets = a.tickets;
+    a.tiles = p->tiles_m.as<uint8_t>();
+    a.ld = n_stages_a;
+    a.n_kt = n_stages_a;
+    a.planes = planes_a;
+    a.q32 = qv32;
+    a.ent = p->miss.a_ent.as<uint32_t>();
+    a.seg = p->miss.a_seg.as<int64_t>();
+    a.nch = p->miss.a_nch;
+    a.bits = p->miss.a_bits;
+    a.err = sc.err;
+    a.sum_q = sc.sum_v;
+    a.scale_g = sc.scale_v;
+    a.two_p = h->two_p;
+    a.inv_s = h->inv_s;
+    a.out = u;
+    const dim3 grid_a(blocks_a, a.split.blocks);
     if (lists)
-      sr_pass_a_kernel<true><<<(unsigned)(h->m_pad / kSrBlockMarkers), 256, sr_pass_a_smem(true),
-                               st>>>(
-          h->geno, h->wpr, planes_a, h->n_pad, sc.sum_v, sc.scale_v, h->two_p, h->inv_s,
-          p->miss.a_ent.as<uint32_t>(), p->miss.a_seg.as<int64_t>(), p->miss.a_nch, p->miss.a_bits,
-          sc.err, u);
+      sr_pass_kernel<false, true><<<grid_a, 256, sr_list_smem(kSrChunkA, kSrRowsA), st>>>(a);
     else
-      sr_pass_a_kernel<false><<<(unsigned)(h->m_pad / kSrBlockMarkers), 256, sr_pass_a_smem(false),
-                                st>>>(
-          h->geno, h->wpr, planes_a, h->n_pad, sc.sum_v, sc.scale_v, h->two_p, h->inv_s, nullptr,
-          nullptr, 0, 0, nullptr, u);
+      sr_pass_kernel<false, false><<<grid_a, 256, 0, st>>>(a);
     SG_CHECK_LAUNCH();
     amax_wc_kernel<<<(unsigned)ceil_div(h->m_pad, kAmaxRows), 256, 0, st>>>(
         u, h->m_pad, h->m_pad, h->inv_s, h->two_p, excl, h->m, sc.amax_w, sc.amax_c);
     sr_quant_wc_kernel<<<(unsigned)ceil_div(h->m_pad, 256), 256, 0, st>>>(
         u, h->m_pad, h->inv_s, h->two_p, sc.amax_w, sc.amax_c, sc.scale_w, sc.scale_c, planes_b,
         qc32, sc.sum_c);
-    // two sample tiles per block (n_pad is a multiple of 512: an even tile count)
-    const SrSplitB split = sr_split_b(h->n_pad, h->m_pad);
-    const unsigned pairs = (unsigned)(h->n_pad / (2 * kRows));
-    const dim3 grid_b(pairs, split.blocks);
-    if (split.blocks > 1 && !p->sr_sums.ptr) {
-      const size_t bytes = (size_t)h->n_pad * 16 + (size_t)pairs * 4;
-      SG_TRY(p->sr_sums.reserve(bytes));
-      SG_CUDA(cudaMemsetAsync(p->sr_sums.ptr, 0, bytes, st));
-    }
-    unsigned long long* sums = p->sr_sums.as<unsigned long long>();
-    unsigned int* tickets = reinterpret_cast<unsigned int*>(sums + 2 * h->n_pad);
-    const double out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
-    double* out = kp + (int64_t)cols[0] * h->n_pad;
+    b.tiles = p->tiles_s.as<uint8_t>();
+    b.ld = p->s_ld;
+    b.n_kt = n_stages_b;
+    b.planes = planes_b;
+    b.q32 = qc32;
+    b.ent = p->miss.b_ent.as<uint32_t>();
+    b.seg = p->miss.b_seg.as<int64_t>();
+    b.nch = p->miss.b_nch;
+    b.bits = p->miss.b_bits;
+    b.err = sc.err;
+    b.sum_q = sc.sum_c;
+    b.scale_g = sc.scale_w;
+    b.scale_m = sc.scale_c;
+    b.out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
+    b.out = kp + (int64_t)cols[0] * h->n_pad;
+    const dim3 grid_b(blocks_b, b.split.blocks);
     if (lists)
-      sr_pass_b_kernel<true><<<grid_b, kRows, 0, st>>>(
-          p->tiles_s.as<uint8_t>(), h->m_pad / kRows, p->s_ld, planes_b, h->m_pad, sc.sum_c,
-          sc.scale_w, sc.scale_c, qc32, p->miss.b_ent.as<uint32_t>(), p->miss.b_seg.as<int64_t>(),
-          p->miss.b_nch, p->miss.b_bits, sc.err, split, sums, sums + h->n_pad, tickets, out_scale,
-          out);
+      sr_pass_kernel<true, true><<<grid_b, 256, sr_list_smem(kSrChunkB, kSrRowsB), st>>>(b);
     else
-      sr_pass_b_kernel<false><<<grid_b, kRows, 0, st>>>(
-          p->tiles_s.as<uint8_t>(), h->m_pad / kRows, p->s_ld, planes_b, h->m_pad, sc.sum_c,
-          sc.scale_w, sc.scale_c, nullptr, nullptr, nullptr, 0, 0, nullptr, split, sums,
-          sums + h->n_pad, tickets, out_scale, out);
+      sr_pass_kernel<true, false><<<grid_b, 256, 0, st>>>(b);
     SG_CHECK_LAUNCH();
     count_launches(6);
     SG_TRY(mark(&t1));

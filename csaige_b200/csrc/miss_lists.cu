@@ -2,12 +2,12 @@
 //
 // A one-column MIXED product forms, per marker (pass A) or per sample (pass B), the
 // integer sums G = sum g q over the calls and Mi = sum q over the missing calls
-// (kernels_tc.cu).  With ~1 % of calls missing, the dense missing-flag sums cost a
-// third of the kernels' instructions (one byte permute and three dp4a per four
-// entries) for a sum over a few entries.  With these lists the one-column kernels form
-// Mi instead as an exact int64 sum of the quantised vector over each row's missing
-// calls, read from the chunk of the vector they already hold in shared memory.  The
-// integer is the one the dense sums form, so the products do not change by a bit.
+// (kernels_tc.cu).  The dense missing-flag sums cost a second unpack and a second set of
+// matrix instructions for a sum over a few entries.  With these lists the one-column kernels
+// form Mi instead as an exact int64 sum of the quantised vector over each row's missing
+// calls, read from the chunk of the vector they hold in shared memory: cheaper up to about
+// 0.3 % of the calls missing.  The integer is the one the dense sums form, so the products
+// do not change by a bit.
 #include <algorithm>
 #include <vector>
 
@@ -185,7 +185,7 @@ std::vector<int64_t> offsets(const int32_t* cnt, int64_t n) {
 }  // namespace
 
 Status miss_lists_build(saige_grm* h, const uint8_t* tiles_s, int64_t s_ld, const MissShape& sh,
-                        MissLists* L, cudaStream_t st) {
+                        double max_frac, MissLists* L, cudaStream_t st) {
   L->state = -1;
   const int64_t m_pad = h->m_pad, n_pad = h->n_pad, n_mt = m_pad / kTileRows;
   const int a_bits = log2_exact(16 * sh.a_chunk_words), b_bits = log2_exact(sh.b_chunk);
@@ -214,7 +214,11 @@ Status miss_lists_build(saige_grm* h, const uint8_t* tiles_s, int64_t s_ld, cons
   if (ob.back() != total)
     return fail(SAIGE_ECUDA, "missing-call lists: %lld calls by marker, %lld by sample",
                 (long long)total, (long long)ob.back());
-  if ((double)total > kMissListMaxFrac * (double)h->m * (double)h->n) return Status();
+  const double calls = (double)h->m * (double)h->n;
+  if ((double)total > max_frac * calls) {
+    if ((double)total <= kMissListMaxFrac * calls) L->state = kMissListsLeft;
+    return Status();
+  }
   const size_t ent_bytes = (size_t)std::max<int64_t>(total, 1) * sizeof(uint32_t);
   // the lists are optional: declined rather than have an allocation flush the block cache
   // (freeing every cached block) when the free memory would not hold them with room over
