@@ -461,7 +461,6 @@ Status pcg_scratch(saige_grm* h, int q, PcgScratch& s) {
   double* cb = h->ws_cols.as<double>();
   s.cols.rz = cb;
   s.cols.rr = cb + q;
-  s.cols.pap = cb + 2 * q;
   s.cols.tol_abs = cb + 3 * q;
   s.small = cb + 4 * q;  // 4q doubles
   int32_t* ib = reinterpret_cast<int32_t*>(cb + 8 * q);

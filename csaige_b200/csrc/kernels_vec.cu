@@ -81,11 +81,36 @@ __global__ void cross_dots_kernel(const double* __restrict__ a, const double* __
   if (threadIdx.x == 0) partial[(int64_t)pair * gridDim.x + blockIdx.x] = s;
 }
 
-__global__ void pcg_start_kernel(const double* __restrict__ b, const double* __restrict__ x0,
-                                 const double* __restrict__ ax0, const double* __restrict__ d,
-                                 double* __restrict__ x, double* __restrict__ r,
-                                 double* __restrict__ z, double* __restrict__ p, int64_t n,
-                                 int64_t ld, double* __restrict__ partial) {
+// The PCG kernels' elementwise loops are bound by the latency of their loads: at n = 9,001 a
+// column has three blocks (the partition fixes the order of its sums), and a thread eleven
+// rows.  It takes kPcgBatch rows at a time, all loads before the first use, and adds to its
+// sums in row order as before (31 columns of 9,001: pcg_update 23.8 -> 8.2 us,
+// pcg_apply 11.7 -> 4.9, pcg_start 8.4 -> 5.5).  The sums over the blocks are formed by the
+// kernel that needs them, in every block alike, instead of a launch each (2.4 and 1.8 us, and
+// their gaps; pcg_p 2.3 -> 4.6).
+constexpr int kPcgBatch = 4;
+
+// Into sh, for every thread of the block: the sums of nb partials of up to three quantities
+// (NULL: none), a warp each, in the order of reduce_partials.
+__device__ __forceinline__ void block_partials(const double* a, const double* b, const double* c,
+                                               int nb, double* sh) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const double* from = w == 0 ? a : (w == 1 ? b : (w == 2 ? c : nullptr));
+  if (from) {
+    double s = 0.0;
+    for (int k = l; k < nb; k += 32) s += from[k];
+    s = warp_sum(s);
+    if (l == 0) sh[w] = s;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kT)
+    pcg_start_kernel(const double* __restrict__ b, const double* __restrict__ x0,
+                     const double* __restrict__ ax0, const double* __restrict__ d,
+                     double* __restrict__ x, double* __restrict__ r, double* __restrict__ z,
+                     double* __restrict__ p, int64_t n, int64_t ld,
+                     double* __restrict__ partial) {
   __shared__ double sh[kT / 32];
   const int c = blockIdx.y;
   const int64_t off = (int64_t)c * ld;
@@ -93,18 +118,31 @@ __global__ void pcg_start_kernel(const double* __restrict__ b, const double* __r
   int64_t hi = lo + ch;
   if (hi > n) hi = n;
   double s_rz = 0.0, s_rr = 0.0, s_bb = 0.0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += kT) {
-    const double bi = b[off + i];
-    const double xi = x0 ? x0[off + i] : 0.0;
-    const double ri = bi - (ax0 ? ax0[off + i] : 0.0);
-    const double zi = ri / d[i];
-    x[off + i] = xi;
-    r[off + i] = ri;
-    z[off + i] = zi;
-    p[off + i] = zi;
-    s_rz += ri * zi;
-    s_rr += ri * ri;
-    s_bb += bi * bi;
+  for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kPcgBatch * kT) {
+    double bi[kPcgBatch], xi[kPcgBatch], ai[kPcgBatch], di[kPcgBatch];
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      const bool in = i < hi;
+      bi[k] = in ? b[off + i] : 0.0;
+      xi[k] = in && x0 ? x0[off + i] : 0.0;
+      ai[k] = in && ax0 ? ax0[off + i] : 0.0;
+      di[k] = in ? d[i] : 1.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      if (i >= hi) break;
+      const double ri = bi[k] - ai[k];
+      const double zi = ri / di[k];
+      x[off + i] = xi[k];
+      r[off + i] = ri;
+      z[off + i] = zi;
+      p[off + i] = zi;
+      s_rz += ri * zi;
+      s_rr += ri * ri;
+      s_bb += bi[k] * bi[k];
+    }
   }
   const int nb = gridDim.x, q = gridDim.y;
   s_rz = block_sum(s_rz, sh);
@@ -118,7 +156,7 @@ __global__ void pcg_start_kernel(const double* __restrict__ b, const double* __r
 }
 
 __global__ void pcg_start_finish(const double* __restrict__ sums, int q, double tol, int force_step,
-                                 PcgCols cols) {
+                                 PcgCols cols, unsigned int* __restrict__ tickets) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= q) return;
   const double rz = sums[c], rr = sums[q + c], bb = sums[2 * q + c];
@@ -128,16 +166,18 @@ __global__ void pcg_start_finish(const double* __restrict__ sums, int q, double 
   cols.rr[c] = rr;
   cols.tol_abs[c] = tol_abs;
   cols.iters[c] = 0;
+  tickets[c] = 0u;
   // a warm-started column takes at least one CG step (force_step), so a start
   // that already meets the tolerance is still refined against the current operator
   cols.state[c] = (!force_step && sqrt(rr) < tol_abs) ? kColConverged : kColActive;
 }
 
 template <bool kWInverse>
-__global__ void pcg_apply_kernel(const double* __restrict__ p, const double* __restrict__ kp,
-                                 const double* __restrict__ wv, double tau0, double tau1,
-                                 double* __restrict__ ap, int64_t n, int64_t ld,
-                                 const int32_t* __restrict__ state, double* __restrict__ partial) {
+__global__ void __launch_bounds__(kT)
+    pcg_apply_kernel(const double* __restrict__ p, const double* __restrict__ kp,
+                     const double* __restrict__ wv, double tau0, double tau1,
+                     double* __restrict__ ap, int64_t n, int64_t ld,
+                     const int32_t* __restrict__ state, double* __restrict__ partial) {
   __shared__ double sh[kT / 32];
   const int c = blockIdx.y;
   if (state[c] != kColActive) return;
@@ -146,58 +186,93 @@ __global__ void pcg_apply_kernel(const double* __restrict__ p, const double* __r
   int64_t hi = lo + ch;
   if (hi > n) hi = n;
   double s = 0.0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += kT) {
-    const double pi = p[off + i];
-    // ai_reml.rs:147 (tau0 v / max(w,1e-30) + tau1 Kv) or pcg.rs:56 (tau0 w v + tau1 Kv)
-    const double a = kWInverse ? tau0 * pi / wv[i] + tau1 * kp[off + i]
-                               : tau0 * wv[i] * pi + tau1 * kp[off + i];
-    ap[off + i] = a;
-    s += pi * a;
+  for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kPcgBatch * kT) {
+    double pk[kPcgBatch], kk[kPcgBatch], wk[kPcgBatch];
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      const bool in = i < hi;
+      pk[k] = in ? p[off + i] : 0.0;
+      kk[k] = in ? kp[off + i] : 0.0;
+      wk[k] = in ? wv[i] : 1.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      if (i >= hi) break;
+      const double pi = pk[k];
+      // ai_reml.rs:147 (tau0 v / max(w,1e-30) + tau1 Kv) or pcg.rs:56 (tau0 w v + tau1 Kv)
+      const double a = kWInverse ? tau0 * pi / wk[k] + tau1 * kk[k]
+                                 : tau0 * wk[k] * pi + tau1 * kk[k];
+      ap[off + i] = a;
+      s += pi * a;
+    }
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) partial[(int64_t)c * gridDim.x + blockIdx.x] = s;
 }
 
-__global__ void pcg_apply_finish(const double* __restrict__ partial, int nb, int q, PcgCols cols) {
-  const int c = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (c >= q) return;
-  if (cols.state[c] != kColActive) return;
-  const int l = threadIdx.x & 31;
-  double s = 0.0;
-  for (int b = l; b < nb; b += 32) s += partial[(int64_t)c * nb + b];
-  s = warp_sum(s);
-  if (l == 0) {
-    cols.pap[c] = s;
-    if (fabs(s) < 1e-30) cols.state[c] = kColStopped;  // decomposition.rs:257-264
-  }
-}
-
-__global__ void pcg_update_kernel(double* __restrict__ x, double* __restrict__ r,
-                                  double* __restrict__ z, const double* __restrict__ p,
-                                  const double* __restrict__ ap, const double* __restrict__ d,
-                                  int64_t n, int64_t ld, PcgCols cols,
-                                  double* __restrict__ partial, double* __restrict__ kx,
-                                  const double* __restrict__ kp) {
+// pap: pcg_apply's partials, whose sums every block forms for itself.  A column with |pap| <
+// 1e-30 stops (decomposition.rs:257-264): pcg_p_kernel says so.
+__global__ void __launch_bounds__(kT)
+    pcg_update_kernel(double* __restrict__ x, double* __restrict__ r, double* __restrict__ z,
+                      const double* __restrict__ p, const double* __restrict__ ap,
+                      const double* __restrict__ d, int64_t n, int64_t ld, PcgCols cols,
+                      const double* __restrict__ pap_partial, double* __restrict__ partial,
+                      double* __restrict__ kx, const double* __restrict__ kp) {
   __shared__ double sh[kT / 32];
   const int c = blockIdx.y;
+  const int nb = gridDim.x, q = gridDim.y;
   if (cols.state[c] != kColActive) return;
-  const double alpha = cols.rz[c] / cols.pap[c];
+  block_partials(pap_partial + (int64_t)c * nb, nullptr, nullptr, nb, sh);
+  const double pap = sh[0];
+  if (fabs(pap) < 1e-30) return;
+  __syncthreads();  // sh is free again
+  const double alpha = cols.rz[c] / pap;
   const int64_t off = (int64_t)c * ld;
   const int64_t ch = part_chunk(n), lo = (int64_t)blockIdx.x * ch;
   int64_t hi = lo + ch;
   if (hi > n) hi = n;
   double s_rz = 0.0, s_rr = 0.0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += kT) {
-    x[off + i] += alpha * p[off + i];
-    if (kx) kx[off + i] += alpha * kp[off + i];  // K x follows x: K x += alpha K p
-    const double ri = r[off + i] - alpha * ap[off + i];
-    r[off + i] = ri;
-    const double zi = ri / d[i];
-    z[off + i] = zi;
-    s_rz += ri * zi;
-    s_rr += ri * ri;
+  for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kPcgBatch * kT) {
+    double pk[kPcgBatch], xk[kPcgBatch], rk[kPcgBatch], ak[kPcgBatch], dk[kPcgBatch];
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      const bool in = i < hi;
+      pk[k] = in ? p[off + i] : 0.0;
+      xk[k] = in ? x[off + i] : 0.0;
+      rk[k] = in ? r[off + i] : 0.0;
+      ak[k] = in ? ap[off + i] : 0.0;
+      dk[k] = in ? d[i] : 1.0;
+    }
+    if (kx) {  // K x follows x: K x += alpha K p
+      double kxk[kPcgBatch], kpk[kPcgBatch];
+#pragma unroll
+      for (int k = 0; k < kPcgBatch; ++k) {
+        const int64_t i = i0 + k * kT;
+        kxk[k] = i < hi ? kx[off + i] : 0.0;
+        kpk[k] = i < hi ? kp[off + i] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < kPcgBatch; ++k) {
+        const int64_t i = i0 + k * kT;
+        if (i < hi) kx[off + i] = kxk[k] + alpha * kpk[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPcgBatch; ++k) {
+      const int64_t i = i0 + k * kT;
+      if (i >= hi) break;
+      x[off + i] = xk[k] + alpha * pk[k];
+      const double ri = rk[k] - alpha * ak[k];
+      r[off + i] = ri;
+      const double zi = ri / dk[k];
+      z[off + i] = zi;
+      s_rz += ri * zi;
+      s_rr += ri * ri;
+    }
   }
-  const int nb = gridDim.x, q = gridDim.y;
   s_rz = block_sum(s_rz, sh);
   s_rr = block_sum(s_rr, sh);
   if (threadIdx.x == 0) {
@@ -206,40 +281,41 @@ __global__ void pcg_update_kernel(double* __restrict__ x, double* __restrict__ r
   }
 }
 
-__global__ void pcg_update_finish(const double* __restrict__ partial, int nb, int q,
-                                  int max_iter, PcgCols cols, double* __restrict__ beta) {
-  const int c = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (c >= q) return;
+// p = z + beta p of the columns that go on.  Every block forms beta and the next state from
+// the nb partials of pcg_apply and pcg_update; the one that takes the column's last ticket,
+// when no block reads the old ones any more, writes them.
+__global__ void __launch_bounds__(kT)
+    pcg_p_kernel(double* __restrict__ p, const double* __restrict__ z, int64_t n, int64_t ld,
+                 const double* __restrict__ pap_partial, const double* __restrict__ partial,
+                 int nb, int max_iter, PcgCols cols, unsigned int* __restrict__ tickets) {
+  __shared__ double sh[3];
+  const int c = blockIdx.y, q = gridDim.y;
   if (cols.state[c] != kColActive) return;
-  const int l = threadIdx.x & 31;
-  double s_rz = 0.0, s_rr = 0.0;
-  for (int b = l; b < nb; b += 32) {
-    s_rz += partial[((int64_t)0 * q + c) * nb + b];
-    s_rr += partial[((int64_t)1 * q + c) * nb + b];
+  block_partials(partial + ((int64_t)0 * q + c) * nb, partial + ((int64_t)1 * q + c) * nb,
+                 pap_partial + (int64_t)c * nb, nb, sh);
+  const double s_rz = sh[0], s_rr = sh[1];
+  const bool stop = fabs(sh[2]) < 1e-30;  // (pcg_update left no sums of such a column)
+  const double beta = s_rz / cols.rz[c];
+  const int it = cols.iters[c] + 1;
+  const int next = stop                            ? kColStopped
+                   : sqrt(s_rr) < cols.tol_abs[c] ? kColConverged
+                   : it >= max_iter               ? kColMaxIter
+                                                  : kColActive;
+  if (next == kColActive) {
+    const int64_t off = (int64_t)c * ld;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+      p[off + i] = z[off + i] + beta * p[off + i];
   }
-  s_rz = warp_sum(s_rz);
-  s_rr = warp_sum(s_rr);
-  if (l == 0) {
-    beta[c] = s_rz / cols.rz[c];
-    cols.rz[c] = s_rz;
-    cols.rr[c] = s_rr;
-    const int it = cols.iters[c] + 1;
-    cols.iters[c] = it;
-    if (sqrt(s_rr) < cols.tol_abs[c]) cols.state[c] = kColConverged;
-    else if (it >= max_iter) cols.state[c] = kColMaxIter;
-  }
-}
-
-__global__ void pcg_p_kernel(double* __restrict__ p, const double* __restrict__ z, int64_t n,
-                             int64_t ld, const int32_t* __restrict__ state,
-                             const double* __restrict__ beta) {
-  const int c = blockIdx.y;
-  if (state[c] != kColActive) return;
-  const double bt = beta[c];
-  const int64_t off = (int64_t)c * ld;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    p[off + i] = z[off + i] + bt * p[off + i];
+  __syncthreads();  // the block has read the column's scalars
+  if (threadIdx.x != 0) return;
+  if (atomicAdd(&tickets[c], 1u) != gridDim.x - 1) return;
+  tickets[c] = 0u;
+  cols.state[c] = next;
+  if (stop) return;
+  cols.rz[c] = s_rz;
+  cols.rr[c] = s_rr;
+  cols.iters[c] = it;
 }
 
 __global__ void sigma_diag_kernel(const double* __restrict__ w, double tau0, double tau1,
@@ -413,12 +489,13 @@ cudaError_t cross_dots(const double* a, int p, const double* b, int q, const dou
 cudaError_t pcg_start(const double* b, const double* x0, const double* ax0, const double* d,
                       double* x, double* r, double* z, double* p, int64_t n, int64_t ld, int q,
                       double tol, bool force_step, PcgCols cols, double* partial,
-                      double* scratch3q, cudaStream_t st) {
+                      double* scratch4q, cudaStream_t st) {
   const int nb = red_blocks(n);
   pcg_start_kernel<<<dim3(nb, q), kT, 0, st>>>(b, x0, ax0, d, x, r, z, p, n, ld, partial);
-  reduce_partials<<<(unsigned)ceil_div(3 * q, 8), 256, 0, st>>>(partial, nb, 3 * q, scratch3q);
-  pcg_start_finish<<<(unsigned)ceil_div(q, 64), 64, 0, st>>>(scratch3q, q, tol, force_step ? 1 : 0,
-                                                             cols);
+  reduce_partials<<<(unsigned)ceil_div(3 * q, 8), 256, 0, st>>>(partial, nb, 3 * q, scratch4q);
+  pcg_start_finish<<<(unsigned)ceil_div(q, 64), 64, 0, st>>>(
+      scratch4q, q, tol, force_step ? 1 : 0, cols,
+      reinterpret_cast<unsigned int*>(scratch4q + 3 * (size_t)q));
   count_launches(3);
   return cudaGetLastError();
 }
@@ -429,8 +506,7 @@ cudaError_t pcg_apply(const double* p, const double* kp, const double* wmax, dou
   const int nb = red_blocks(n);
   pcg_apply_kernel<true><<<dim3(nb, q), kT, 0, st>>>(p, kp, wmax, tau0, tau1, ap, n, ld,
                                                      cols.state, partial);
-  pcg_apply_finish<<<(unsigned)ceil_div(q, 8), 256, 0, st>>>(partial, nb, q, cols);
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 
@@ -440,22 +516,24 @@ cudaError_t pcg_apply_w(const double* p, const double* kp, const double* w, doub
   const int nb = red_blocks(n);
   pcg_apply_kernel<false><<<dim3(nb, q), kT, 0, st>>>(p, kp, w, tau0, tau1, ap, n, ld,
                                                       cols.state, partial);
-  pcg_apply_finish<<<(unsigned)ceil_div(q, 8), 256, 0, st>>>(partial, nb, q, cols);
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t pcg_step(double* x, double* r, double* z, double* p, const double* ap,
                      const double* d, int64_t n, int64_t ld, int q, int max_iter, PcgCols cols,
-                     double* partial, double* scratch2q, cudaStream_t st, double* kx, const double* kp) {
+                     double* partial, double* scratch4q, cudaStream_t st, double* kx,
+                     const double* kp) {
   const int nb = red_blocks(n);
-  pcg_update_kernel<<<dim3(nb, q), kT, 0, st>>>(x, r, z, p, ap, d, n, ld, cols, partial, kx, kp);
-  pcg_update_finish<<<(unsigned)ceil_div(q, 8), 256, 0, st>>>(partial, nb, q, max_iter, cols,
-                                                              scratch2q);
+  double* sums = partial + (int64_t)nb * q;  // after pcg_apply's
+  pcg_update_kernel<<<dim3(nb, q), kT, 0, st>>>(x, r, z, p, ap, d, n, ld, cols, partial, sums, kx,
+                                                kp);
   unsigned gx = (unsigned)ceil_div(n, kT);
   if (gx > 1024) gx = 1024;
-  pcg_p_kernel<<<dim3(gx, q), kT, 0, st>>>(p, z, n, ld, cols.state, scratch2q);
-  count_launches(3);
+  pcg_p_kernel<<<dim3(gx, q), kT, 0, st>>>(p, z, n, ld, partial, sums, nb, max_iter, cols,
+                                           reinterpret_cast<unsigned int*>(scratch4q +
+                                                                           3 * (size_t)q));
+  count_launches(2);
   return cudaGetLastError();
 }
 

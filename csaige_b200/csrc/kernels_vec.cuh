@@ -12,7 +12,6 @@ enum : int32_t { kColActive = 0, kColConverged = 1, kColStopped = 2, kColMaxIter
 struct PcgCols {
   double* rz;       // r'z
   double* rr;       // r'r
-  double* pap;      // p'Ap
   double* tol_abs;  // tol * max(||b||, 1)
   int32_t* state;   // kCol*
   int32_t* iters;
@@ -38,8 +37,9 @@ cudaError_t cross_dots(const double* a, int p, const double* b, int q, const dou
 cudaError_t pcg_start(const double* b, const double* x0, const double* ax0, const double* d,
                       double* x, double* r, double* z, double* p, int64_t n, int64_t ld, int q,
                       double tol, bool force_step, PcgCols cols, double* partial,
-                      double* scratch3q, cudaStream_t st);
-// ap = tau0 p / wmax + tau1 kp, pap = p'ap; columns with |pap| < 1e-30 stop.
+                      double* scratch4q, cudaStream_t st);
+// ap = tau0 p / wmax + tau1 kp, and the partial sums of p'ap, which pcg_step takes from
+// partial.
 cudaError_t pcg_apply(const double* p, const double* kp, const double* wmax, double tau0,
                       double tau1, double* ap, int64_t n, int64_t ld, int q, PcgCols cols,
                       double* partial, cudaStream_t st);
@@ -47,11 +47,12 @@ cudaError_t pcg_apply(const double* p, const double* kp, const double* wmax, dou
 cudaError_t pcg_apply_w(const double* p, const double* kp, const double* w, double tau0,
                         double tau1, double* ap, int64_t n, int64_t ld, int q, PcgCols cols,
                         double* partial, cudaStream_t st);
-// x += alpha p, r -= alpha ap, z = r / d, then beta, ||r|| test, p = z + beta p;
+// Columns with |p'ap| < 1e-30 stop; x += alpha p, r -= alpha ap, z = r / d, then beta, ||r||
+// test, p = z + beta p; scratch4q: as pcg_start left it (its tickets are zero);
 // with kx, also kx += alpha kp (K x kept beside x from the products K p).
 cudaError_t pcg_step(double* x, double* r, double* z, double* p, const double* ap,
                      const double* d, int64_t n, int64_t ld, int q, int max_iter, PcgCols cols,
-                     double* partial, double* scratch2q, cudaStream_t st, double* kx = nullptr,
+                     double* partial, double* scratch4q, cudaStream_t st, double* kx = nullptr,
                      const double* kp = nullptr);
 
 // Elementwise helpers for the AI-REML loop.
