@@ -857,13 +857,12 @@ static Status fit_impl(saige_grm* h, const double* y, const double* x, int64_t n
     double score_e = 0.0, ai_00 = 0.0, ai_01 = 0.0;
     if (!fix_tau_e) {
       // trace of P W^-1 (ai_reml.rs:281-299): the probe solves repeat the ones above
-      for (int k = 0; k < f.nrv; ++k)
-        SG_CUDA(div_w(U + (size_t)k * ld, f.w, f.tmpq + (size_t)k * ld, n, f.st));
+      SG_CUDA(div_w(U, f.w, f.tmpq, n, ld, f.nrv, f.st));
       SG_TRY(coldots(f, f.tmpq, f.pu, f.nrv, tr));
       double tw = 0.0;
       for (int k = 0; k < f.nrv; ++k) tw += tr[(size_t)k];
       const double trace_w = tw / (double)f.nrv;
-      SG_CUDA(div_w(f.py, f.w, f.invw_py, n, f.st));
+      SG_CUDA(div_w(f.py, f.w, f.invw_py, n, ld, 1, f.st));
       SG_TRY(coldots(f, f.py, f.invw_py, 1, r1));
       score_e = r1[0] - trace_w;
       if (recyc && cfg->solve == SAIGE_SOLVE_BLOCK) {

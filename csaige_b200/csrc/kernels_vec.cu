@@ -408,11 +408,29 @@ __global__ void sub_combo_kernel(double* __restrict__ y, int q, const double* __
 }
 
 __global__ void div_w_kernel(const double* __restrict__ v, const double* __restrict__ w,
-                             double* __restrict__ out, int64_t n) {
+                             double* __restrict__ out, int64_t n, int64_t ld) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const int64_t off = (int64_t)blockIdx.y * ld;
   const double wm = w[i] > 1e-30 ? w[i] : 1e-30;
-  out[i] = v[i] / wm;
+  out[off + i] = v[off + i] / wm;
+}
+
+// Column blockIdx.y of the list from two blocks of vectors to the slots from `slot` on.  One
+// launch in place of two copies per column: the copies of five columns of 9,001 doubles took
+// 1.9 us each on the device and longer to issue.
+__global__ void __launch_bounds__(kT)
+    keep_cols_kernel(const double* __restrict__ a, const double* __restrict__ b, KeepCols cols,
+                     double* __restrict__ a_out, double* __restrict__ b_out, int slot,
+                     int64_t ld) {
+  const int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x;  // pairs of doubles (ld is even)
+  if (2 * i >= ld) return;
+  const int64_t from = (int64_t)cols.c[blockIdx.y] * ld + 2 * i;
+  const int64_t to = (int64_t)(slot + blockIdx.y) * ld + 2 * i;
+  const double2 x = *reinterpret_cast<const double2*>(a + from);
+  const double2 y = *reinterpret_cast<const double2*>(b + from);
+  *reinterpret_cast<double2*>(a_out + to) = x;
+  *reinterpret_cast<double2*>(b_out + to) = y;
 }
 
 struct Key8 {
@@ -579,8 +597,18 @@ cudaError_t sub_combo(double* y, int q, const double* a, int p, const double* co
   return cudaGetLastError();
 }
 
-cudaError_t div_w(const double* v, const double* w, double* out, int64_t n, cudaStream_t st) {
-  div_w_kernel<<<g1(n), kT, 0, st>>>(v, w, out, n);
+cudaError_t div_w(const double* v, const double* w, double* out, int64_t n, int64_t ld, int q,
+                  cudaStream_t st) {
+  div_w_kernel<<<dim3(g1(n), q), kT, 0, st>>>(v, w, out, n, ld);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t keep_cols(const double* a, const double* b, const KeepCols& cols, int k, double* a_out,
+                      double* b_out, int slot, int64_t ld, cudaStream_t st) {
+  if (k <= 0) return cudaSuccess;
+  keep_cols_kernel<<<dim3((unsigned)ceil_div(ld / 2, kT), k), kT, 0, st>>>(a, b, cols, a_out, b_out,
+                                                                           slot, ld);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -76,7 +76,16 @@ cudaError_t init_mu(const double* y, int trait, double* mu, double* eta, int64_t
 cudaError_t sub_combo(double* y, int q, const double* a, int p, const double* coef, int64_t n,
                       int64_t ld, cudaStream_t st);
 // out = v / max(w,1e-30)
-cudaError_t div_w(const double* v, const double* w, double* out, int64_t n, cudaStream_t st);
+cudaError_t div_w(const double* v, const double* w, double* out, int64_t n, int64_t ld, int q,
+                  cudaStream_t st);
+// Columns cols.c[0 .. k) (k <= kKeepMax) of a and of b, ld apart (a multiple of 2), to the
+// columns from `slot` on of a_out and b_out.
+constexpr int kKeepMax = 64;
+struct KeepCols {
+  int c[kKeepMax];
+};
+cudaError_t keep_cols(const double* a, const double* b, const KeepCols& cols, int k, double* a_out,
+                      double* b_out, int slot, int64_t ld, cudaStream_t st);
 // nrv Rademacher probe columns (ld apart, padding rows zeroed) from the ChaCha8
 // stream with the given key (ai_reml.rs:121-130).
 cudaError_t rademacher_probes_dev(const uint32_t* key, double* out, int64_t n, int64_t ld, int nrv,

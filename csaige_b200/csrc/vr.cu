@@ -133,6 +133,23 @@ __global__ void vr_bed_decode_kernel(const uint8_t* __restrict__ rows, int64_t b
   out[(int64_t)c * ld + i] = code == 0 ? 2.0 : (code == 2 ? 1.0 : (code == 3 ? 0.0 : (double)NAN));
 }
 
+// Row rows[blockIdx.x] of the raw .bed (bpm bytes at any alignment) to row blockIdx.x of out.
+// One launch in place of a copy per candidate row: 1,100 copies of 12.5 KB took 2.1 ms.
+__global__ void __launch_bounds__(kT)
+    vr_gather_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
+                     const int64_t* __restrict__ rows, uint8_t* __restrict__ out) {
+  const uint8_t* from = bed + 3 + rows[blockIdx.x] * bpm;
+  uint8_t* to = out + (int64_t)blockIdx.x * bpm;
+  for (int64_t i0 = threadIdx.x; i0 < bpm; i0 += 8 * kT) {
+    uint8_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = i0 + k * kT < bpm ? from[i0 + k * kT] : 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (i0 + k * kT < bpm) to[i0 + k * kT] = v[k];
+  }
+}
+
 inline unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + kT - 1) / kT); }
 
 // variance_ratio.rs:260-272: (sd / mean) / n, infinity for n <= 1 or |mean| < 1e-30.
@@ -403,11 +420,16 @@ Status vr_gather_rows(const uint8_t* bed_dev, int64_t bpm, const int64_t* vidx, 
   out.bpm = bpm;
   out.m = m_vr;
   out.has_sidx = sample_idx != nullptr;
+  DevBuf idx;
   if (m_vr > 0) {
     SG_TRY(out.rows.reserve((size_t)m_vr * (size_t)bpm));
-    for (int64_t j = 0; j < m_vr; ++j)
-      SG_CUDA(cudaMemcpyAsync(out.rows.as<uint8_t>() + j * bpm, bed_dev + 3 + vidx[j] * bpm,
-                              (size_t)bpm, cudaMemcpyDeviceToDevice, st));
+    SG_TRY(idx.reserve((size_t)m_vr * sizeof(int64_t)));
+    SG_CUDA(cudaMemcpyAsync(idx.ptr, vidx, (size_t)m_vr * sizeof(int64_t), cudaMemcpyHostToDevice,
+                            st));
+    vr_gather_kernel<<<(unsigned)m_vr, kT, 0, st>>>(bed_dev, bpm, idx.as<int64_t>(),
+                                                    out.rows.as<uint8_t>());
+    count_launches(1);
+    SG_CUDA(cudaGetLastError());
   }
   if (sample_idx) {
     SG_TRY(out.sidx.reserve((size_t)n * sizeof(int64_t)));

@@ -139,7 +139,19 @@ __global__ void combo_kernel(const double* __restrict__ V, int m, const double* 
   double acc[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) acc[c] = (add && c0 + c < q) ? Y[(int64_t)(c0 + c) * ld + i] : 0.0;
-  for (int j = 0; j < m; ++j) {
+  // eight columns' loads at a time: at n = 9,001 a thread's chain of loads is what the
+  // kernel takes (7.9 -> 6.5 us)
+  int j = 0;
+  for (; j + 8 <= m; j += 8) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = V[(int64_t)(j + k) * ld + i];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[c] += v[k] * g[(j + k) * 8 + c];
+  }
+  for (; j < m; ++j) {
     const double v = V[(int64_t)j * ld + i];
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[c] += v * g[j * 8 + c];
