@@ -77,18 +77,14 @@ Status dots(Fit& f, const double* a, int pa, const double* b, int qb, const doub
   double* dout = f.dsmall;
   SG_CUDA(cross_dots(a, pa, b, qb, wv, f.n, f.ld, f.partial, dout, f.st));
   out.resize((size_t)pa * qb);
-  SG_CUDA(cudaMemcpyAsync(out.data(), dout, out.size() * 8, cudaMemcpyDeviceToHost, f.st));
-  SG_CUDA(cudaStreamSynchronize(f.st));
-  return Status();
+  return read_back(f.h, out.data(), dout, out.size() * 8, f.st);
 }
 
 Status coldots(Fit& f, const double* a, const double* b, int q, std::vector<double>& out) {
   double* dout = f.dsmall;
   SG_CUDA(col_dots(a, b, f.n, f.ld, q, f.partial, dout, f.st));
   out.resize((size_t)q);
-  SG_CUDA(cudaMemcpyAsync(out.data(), dout, out.size() * 8, cudaMemcpyDeviceToHost, f.st));
-  SG_CUDA(cudaStreamSynchronize(f.st));
-  return Status();
+  return read_back(f.h, out.data(), dout, out.size() * 8, f.st);
 }
 
 // PCG of Sigma = tau0 W^-1 + tau1 K on q columns of b into x (x0 optional).
@@ -366,8 +362,7 @@ Status galerkin_start(Fit& f, Recycle& rc, int mb, int q, bool& ok) {
   const int64_t ld = f.ld;
   SG_CUDA(gram(rc.v, mb, rc.av, mb + q, f.n, ld, rc.gpart, rc.gout, f.st));
   std::vector<double> gall((size_t)mb * (mb + q)), gam;
-  SG_CUDA(cudaMemcpyAsync(gall.data(), rc.gout, gall.size() * 8, cudaMemcpyDeviceToHost, f.st));
-  SG_CUDA(cudaStreamSynchronize(f.st));
+  SG_TRY(read_back(f.h, gall.data(), rc.gout, gall.size() * 8, f.st));
   ok = galerkin_coeffs(gall, mb, q, gam);
   if (!ok) {
     ++rc.fallbacks;

@@ -94,8 +94,51 @@ size_t cache_flush(int dev) {
 }
 }  // namespace
 
+namespace {
+std::mutex g_pin_mu;
+std::vector<void*> g_pins;  // free blocks
+}  // namespace
+
+void* PinBuf::get() {
+  if (ptr || tried) return ptr;
+  tried = true;
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (!g_pins.empty()) {
+      ptr = g_pins.back();
+      g_pins.pop_back();
+      return ptr;
+    }
+  }
+  if (cudaHostAlloc(&ptr, kPinBytes, cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ptr = nullptr;
+  }
+  return ptr;
+}
+
+void PinBuf::release() {
+  if (!ptr) return;
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (g_pins.size() < kPinKept) {
+      g_pins.push_back(ptr);
+      ptr = nullptr;
+    }
+  }
+  if (ptr) cudaFreeHost(ptr);
+  ptr = nullptr;
+  tried = false;
+}
+
 void release_cached_blocks() {
   cache_flush(-1);
+  std::vector<void*> pins;
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    pins.swap(g_pins);
+  }
+  for (void* p : pins) cudaFreeHost(p);
   // the sub-cohort build's host-mapped block, unless a build is using it
   release_cohort_mapped();
   // the streamed build's host-mapped block, unless a build is using it
@@ -428,8 +471,21 @@ static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
   return Status();
 }
 
+Status read_back(saige_grm* h, void* dst, const void* dev, size_t bytes, cudaStream_t st) {
+  void* p = bytes <= kPinBytes ? h->pin.get() : nullptr;
+  SG_CUDA(cudaMemcpyAsync(p ? p : dst, dev, bytes, cudaMemcpyDeviceToHost, st));
+  SG_CUDA(cudaStreamSynchronize(st));
+  if (p) memcpy(dst, p, bytes);
+  return Status();
+}
+
+Status grm_product_check(saige_grm* h, unsigned int err, cudaStream_t st) {
+  return err ? tc_product_failed(h, err, st) : Status();
+}
+
 Status grm_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
-                   int precision, cudaStream_t st) {
+                   int precision, cudaStream_t st, unsigned int* later) {
+  if (later) *later = 0u;
   if (h->m_eff == 0 || (h->masked && h->m_active == 0)) {
     // pcg.rs:132-134: no markers -> zero vector
     for (int c = 0; c < q; ++c)
@@ -438,7 +494,7 @@ Status grm_product(saige_grm* h, const double* v, double* kp, int q, const int32
     return Status();
   }
   if (precision == SAIGE_PREC_FP32) return grm_product_fp32(h, v, kp, q, active, st);
-  if (precision == SAIGE_PREC_MIXED) return tc_product(h, v, kp, q, active, st);
+  if (precision == SAIGE_PREC_MIXED) return tc_product(h, v, kp, q, active, st, later);
   return fail(SAIGE_EINVAL, "unknown precision %d", precision);
 }
 
@@ -450,7 +506,7 @@ Status pcg_scratch(saige_grm* h, int q, PcgScratch& s) {
   const int nb = red_blocks(h->n);
   SG_TRY(h->ws_vec.reserve((size_t)5 * ld * q * sizeof(double)));
   SG_TRY(h->ws_red.reserve((size_t)nb * 3 * q * sizeof(double) + 64));
-  SG_TRY(h->ws_cols.reserve((size_t)q * (8 * sizeof(double) + 2 * sizeof(int32_t)) + 256));
+  SG_TRY(h->ws_cols.reserve((size_t)q * (9 * sizeof(double) + 2 * sizeof(int32_t)) + 256));
   double* base = h->ws_vec.as<double>();
   s.r = base;
   s.z = base + (int64_t)1 * ld * q;
@@ -460,10 +516,11 @@ Status pcg_scratch(saige_grm* h, int q, PcgScratch& s) {
   s.partial = h->ws_red.as<double>();
   double* cb = h->ws_cols.as<double>();
   s.cols.rz = cb;
-  s.cols.rr = cb + q;
   s.cols.tol_abs = cb + 3 * q;
   s.small = cb + 4 * q;  // 4q doubles
-  int32_t* ib = reinterpret_cast<int32_t*>(cb + 8 * q);
+  // read together: 16 bytes per column from rr on
+  s.cols.rr = cb + 8 * q;
+  int32_t* ib = reinterpret_cast<int32_t*>(cb + 9 * q);
   s.cols.state = ib;
   s.cols.iters = ib + q;
   return Status();
@@ -478,6 +535,28 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   SG_TRY(pcg_scratch(h, q + ne, s));  // room for the extra columns in p and kp
   std::vector<int32_t> state((size_t)q, kColActive);
   bool extra_done = ne == 0;
+  // The columns' state after each iteration, and the error word of its product, are read
+  // together: one wait per iteration (a wait after the product, and both reads into pageable
+  // memory, left the device idle for about a fifth of a refit of 9,001 samples).
+  const size_t per = 16, cols_bytes = per * (size_t)(q + ne);
+  std::vector<char> pageable;
+  char* landing = cols_bytes + 8 <= kPinBytes ? static_cast<char*>(h->pin.get()) : nullptr;
+  unsigned int* later = landing ? reinterpret_cast<unsigned int*>(landing + cols_bytes) : nullptr;
+  if (later) *later = 0u;
+  if (!landing) {
+    pageable.resize(cols_bytes);
+    landing = pageable.data();
+  }
+  const double* h_rr = reinterpret_cast<const double*>(landing);
+  const int32_t* h_state = reinterpret_cast<const int32_t*>(h_rr + q + ne);
+  const int32_t* h_iters = h_state + q + ne;
+  auto read_cols = [&]() -> Status {
+    SG_CUDA(cudaMemcpyAsync(landing, s.cols.rr, cols_bytes, cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    if (later) SG_TRY(grm_product_check(h, *later, st));
+    std::copy(h_state, h_state + q, state.begin());
+    return Status();
+  };
   // With tau1 = 0 the operator is tau0 W^-1 (or tau0 W): tau1 K v contributes only
   // zeros, so no GRM product is formed and K v reads as 0.
   const bool no_k = run.tau1 == 0.0;
@@ -510,13 +589,10 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
                     run.force_step && run.x0 != nullptr, s.cols, s.partial, s.small, st));
   if (run.max_iter <= 0) {
     // the loop body never runs; converged is the initial test
-    SG_CUDA(cudaMemcpyAsync(state.data(), s.cols.state, (size_t)q * 4, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(read_cols());
   } else {
     for (;;) {
-      SG_CUDA(cudaMemcpyAsync(state.data(), s.cols.state, (size_t)q * 4, cudaMemcpyDeviceToHost,
-                              st));
-      SG_CUDA(cudaStreamSynchronize(st));
+      SG_TRY(read_cols());
       bool any = false;
       for (int c = 0; c < q; ++c) any |= state[(size_t)c] == kColActive;
       if (!any) break;
@@ -526,12 +602,12 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
                                 cudaMemcpyDeviceToDevice, st));
         std::vector<int32_t> st2 = state;
         st2.resize((size_t)(q + ne), kColActive);
-        SG_TRY(grm_product(h, s.p, s.kp, q + ne, st2.data(), run.precision, st));
+        SG_TRY(grm_product(h, s.p, s.kp, q + ne, st2.data(), run.precision, st, later));
         SG_CUDA(cudaMemcpyAsync(run.extra_out, s.kp + (size_t)q * ld, (size_t)ld * ne * sizeof(double),
                                 cudaMemcpyDeviceToDevice, st));
         extra_done = true;
       } else if (!no_k) {
-        SG_TRY(grm_product(h, s.p, s.kp, q, state.data(), run.precision, st));
+        SG_TRY(grm_product(h, s.p, s.kp, q, state.data(), run.precision, st, later));
       }
       if (!no_k && run.keep_p && run.keep_kp) {
         KeepCols kc;
@@ -559,24 +635,20 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
                        s.partial, s.small, st, run.kx_valid ? run.kx : nullptr, s.kp));
     }
   }
+  run.iters.assign(h_iters, h_iters + q);
+  run.state = state;
+  run.resid.resize((size_t)q);
+  run.total_iters = 0;
+  for (int c = 0; c < q; ++c) {
+    run.resid[(size_t)c] = sqrt(h_rr[c]);
+    if (run.max_iter <= 0 && state[(size_t)c] == kColActive) run.state[(size_t)c] = kColMaxIter;
+    run.total_iters += run.iters[(size_t)c];
+  }
   if (!extra_done)
     SG_TRY(grm_product(h, run.extra_in, run.extra_out, ne, nullptr, run.precision, st));
   if (run.r_out)
     SG_CUDA(cudaMemcpyAsync(run.r_out, s.r, (size_t)ld * q * sizeof(double),
                             cudaMemcpyDeviceToDevice, st));
-  std::vector<double> rr((size_t)q);
-  run.iters.assign((size_t)q, 0);
-  run.state = state;
-  SG_CUDA(cudaMemcpyAsync(run.iters.data(), s.cols.iters, (size_t)q * 4, cudaMemcpyDeviceToHost, st));
-  SG_CUDA(cudaMemcpyAsync(rr.data(), s.cols.rr, (size_t)q * 8, cudaMemcpyDeviceToHost, st));
-  SG_CUDA(cudaStreamSynchronize(st));
-  run.resid.resize((size_t)q);
-  run.total_iters = 0;
-  for (int c = 0; c < q; ++c) {
-    run.resid[(size_t)c] = sqrt(rr[(size_t)c]);
-    if (run.max_iter <= 0 && state[(size_t)c] == kColActive) run.state[(size_t)c] = kColMaxIter;
-    run.total_iters += run.iters[(size_t)c];
-  }
   if (run.count_columns) h->n_kv_launches = launches0 + (h->n_kv - kv0);
   return Status();
 }

@@ -47,6 +47,20 @@ struct DevBuf {
 };
 
 void release_cached_blocks();
+
+// A page-locked block of kPinBytes that a handle's small device-to-host reads land in: a read
+// into pageable memory goes through the driver's own staging and waits for itself.  Blocks
+// come from a free list of at most kPinKept, which release_cached_blocks() empties.
+constexpr size_t kPinBytes = (size_t)1 << 18;
+constexpr size_t kPinKept = 16;
+struct PinBuf {
+  void* ptr = nullptr;
+  bool tried = false;
+  // kPinBytes at ptr, or NULL when none can be had (the reads are pageable then)
+  void* get();
+  void release();
+  ~PinBuf() { release(); }
+};
 // Frees the sub-cohort build's host-mapped block unless a call is using it (cohorts.cu).
 void release_cohort_mapped();
 
@@ -128,6 +142,7 @@ struct saige_grm {
   saige::TcPlan* tc = nullptr;
   // generic workspaces
   saige::DevBuf ws_vec, ws_red, ws_cols, ws_io;
+  saige::PinBuf pin;  // small reads, under mu
   // Leave-one-chromosome-out: while `masked`, products skip the markers flagged in
   // excl (m_pad bytes, 1 = left out) and scale by 1/m_active.  Set and cleared only
   // inside saige_fit_loco, under mu.
@@ -165,8 +180,14 @@ bool marker_qc_pass(double af, int64_t n_valid, int64_t n, double min_maf, doubl
 
 // Kv for q columns of v (ld = h->n_pad, padding rows zero) into kp.
 // active (host, length q, may be NULL) selects columns; others are skipped.
+// With `later` (page-locked), a MIXED product returns without waiting, its error word (0: none)
+// to arrive there in stream order, and the caller passes it to grm_product_check once st has
+// been synchronised; timed and traced products wait all the same.
 Status grm_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
-                   int precision, cudaStream_t st);
+                   int precision, cudaStream_t st, unsigned int* later = nullptr);
+Status grm_product_check(saige_grm* h, unsigned int err, cudaStream_t st);
+// Copies `bytes` from the device to dst, synchronising st.
+Status read_back(saige_grm* h, void* dst, const void* dev, size_t bytes, cudaStream_t st);
 
 struct PcgRun {
   // inputs (device, ld = n_pad)

@@ -1839,8 +1839,23 @@ static unsigned set_work(TcArgs* a, int64_t tiles, int sms) {
   return (unsigned)w.grid;
 }
 
+// The sums and counts of tiles that CTAs share: one slot per CTA (see TcWork).
+static size_t part_bytes(const TcPlan* p) {
+  return (size_t)p->sms * (2 * kMaxR * kRows * 8 + 4);
+}
+
+Status tc_product_failed(saige_grm* h, unsigned int err, cudaStream_t st) {
+  if (err & kSrListErr)
+    return fail(SAIGE_ECUDA, "one-column GRM product: a missing-call list entry out of range");
+  // shared tiles may be left half summed
+  TcPlan* p = h->tc;
+  if (p->part.ptr) SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes(p), st));
+  SG_CUDA(cudaStreamSynchronize(st));
+  return fail(SAIGE_TIMEOUT, "tensor-core GRM product: a pipeline wait timed out");
+}
+
 Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
-                  cudaStream_t st) {
+                  cudaStream_t st, unsigned int* later) {
   SG_TRY(tc_init(h));
   TcPlan* p = h->tc;
   std::vector<int> cols;
@@ -1983,10 +1998,9 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
   }
   // a slot for every tile that CTAs share (at most one per CTA boundary)
   const size_t part_slots = (size_t)p->sms;
-  const size_t part_bytes = part_slots * (2 * kMaxR * kRows * 8 + 4);
   if (!single && !p->part.ptr) {
-    SG_TRY(p->part.reserve(part_bytes));
-    SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes, st));
+    SG_TRY(p->part.reserve(part_bytes(p)));
+    SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes(p), st));
   }
   for (size_t c0 = 0; c0 < (single ? 0 : cols.size()); c0 += kMaxR) {
     const int r = (int)std::min<size_t>(kMaxR, cols.size() - c0);
@@ -2079,9 +2093,12 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->n_kv += r;
   }
   h->n_kv_launches += 1;
+  if (later && !h->profiling && !p->tracing) {
+    SG_CUDA(cudaMemcpyAsync(later, sc.err, sizeof(*later), cudaMemcpyDeviceToHost, st));
+    return Status();
+  }
   unsigned int err = 0;
-  SG_CUDA(cudaMemcpyAsync(&err, sc.err, sizeof(err), cudaMemcpyDeviceToHost, st));
-  SG_CUDA(cudaStreamSynchronize(st));
+  SG_TRY(read_back(h, &err, sc.err, sizeof(err), st));
   for (auto& pr : ev_a) {
     float ms = 0.f;
     SG_CUDA(cudaEventElapsedTime(&ms, pr.first, pr.second));
@@ -2098,15 +2115,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->stats.sc_ms += ms;
   }
   for (cudaEvent_t e : ev) cudaEventDestroy(e);
-  if (err & kSrListErr)
-    return fail(SAIGE_ECUDA, "one-column GRM product: a missing-call list entry out of range");
-  if (err) {
-    // shared tiles may be left half summed
-    if (p->part.ptr) SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes, st));
-    SG_CUDA(cudaStreamSynchronize(st));
-    return fail(SAIGE_TIMEOUT, "tensor-core GRM product: a pipeline wait timed out");
-  }
-  return Status();
+  return err ? tc_product_failed(h, err, st) : Status();
 }
 
 }  // namespace saige

@@ -11,8 +11,11 @@ namespace saige {
 constexpr int kTcFastCols = 42;
 
 // Kv for q columns (ld = h->n_pad) through the int8-limb tensor-core kernels.
+// later: see grm_product.
 Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
-                  cudaStream_t st);
+                  cudaStream_t st, unsigned int* later = nullptr);
+// A product's error word other than 0: its error, the state of its pipeline put right.
+Status tc_product_failed(saige_grm* h, unsigned int err, cudaStream_t st);
 void tc_destroy(saige_grm* h);
 // Streamed build: reserves the code tiles for up to rows_cap marker rows (the
 // sample-major tiles keep that many marker tiles per sample tile), then builds the

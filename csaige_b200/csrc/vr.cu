@@ -316,8 +316,7 @@ Status vr_run(saige_grm* h, const VrFill& fill, int64_t n_cand, const double* ma
     SG_CHECK_LAUNCH();
     std::vector<double> stats(2 * (size_t)q), fillv((size_t)q), ac((size_t)q);
     std::vector<int32_t> flip((size_t)q);
-    SG_CUDA(cudaMemcpyAsync(stats.data(), dStats, 2 * (size_t)q * 8, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(read_back(h, stats.data(), dStats, 2 * (size_t)q * 8, st));
     for (int c = 0; c < q; ++c) {
       const double s_nm = stats[2 * (size_t)c], n_nm = stats[2 * (size_t)c + 1];
       fillv[(size_t)c] = n_nm > 0.0 ? 2.0 * (s_nm / (2.0 * n_nm)) : 0.0;
@@ -356,8 +355,7 @@ Status vr_run(saige_grm* h, const VrFill& fill, int64_t n_cand, const double* ma
     SG_CUDA(col_dots(dTmp, dG, n, ld, q, dPart, dDots + q, st));
     count_launches(3);
     std::vector<double> dots(2 * (size_t)q);
-    SG_CUDA(cudaMemcpyAsync(dots.data(), dDots, 2 * (size_t)q * 8, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(read_back(h, dots.data(), dDots, 2 * (size_t)q * 8, st));
     // the reference's rules, marker by marker in shuffled order (variance_ratio.rs:139-210)
     for (int c = 0; c < q && !stop; ++c) {
       if (ac[(size_t)c] < 1.0) continue;
