@@ -625,14 +625,9 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
         }
         SG_TRY(keep());
       }
-      if (run.w_inverse)
-        SG_CUDA(pcg_apply(s.p, s.kp, run.wv, run.tau0, run.tau1, s.ap, n, ld, q, s.cols,
-                          s.partial, st));
-      else
-        SG_CUDA(pcg_apply_w(s.p, s.kp, run.wv, run.tau0, run.tau1, s.ap, n, ld, q, s.cols,
-                            s.partial, st));
-      SG_CUDA(pcg_step(run.x, s.r, s.z, s.p, s.ap, run.d, n, ld, q, run.max_iter, s.cols,
-                       s.partial, s.small, st, run.kx_valid ? run.kx : nullptr, s.kp));
+      SG_CUDA(pcg_iteration(run.x, s.r, s.z, s.p, s.kp, s.ap, run.w_inverse, run.wv, run.tau0,
+                            run.tau1, run.d, n, ld, q, run.max_iter, s.cols, s.partial, s.small,
+                            st, run.kx_valid ? run.kx : nullptr));
     }
   }
   run.iters.assign(h_iters, h_iters + q);

@@ -55,6 +55,14 @@ cudaError_t pcg_step(double* x, double* r, double* z, double* p, const double* a
                      double* partial, double* scratch4q, cudaStream_t st, double* kx = nullptr,
                      const double* kp = nullptr);
 
+// pcg_apply (w_inverse) or pcg_apply_w, and pcg_step: one launch for columns of up to eight row
+// blocks, which leave ap and z as they were.
+cudaError_t pcg_iteration(double* x, double* r, double* z, double* p, const double* kp, double* ap,
+                          bool w_inverse, const double* wv, double tau0, double tau1,
+                          const double* d, int64_t n, int64_t ld, int q, int max_iter,
+                          PcgCols cols, double* partial, double* scratch4q, cudaStream_t st,
+                          double* kx = nullptr);
+
 // Elementwise helpers for the AI-REML loop.
 // Jacobi diagonal of fit-null: wmax = max(w,1e-30), d = tau0/wmax + tau1 (1 when |d| <= 1e-30);
 // with diagk, d = tau0/wmax + tau1 diagk[i].

@@ -1,6 +1,7 @@
 """The PCG's vector kernels at the edges of their row blocks and batches.
 
-A row block has up to 4,096 rows, a thread takes every 256th of them, four at a time.  The
+A row block has up to 4,096 rows, a thread takes every 256th of them, four at a time; columns
+of up to eight row blocks (32,768 rows) take one launch per iteration.  The
 solves are compared with a numpy PCG over the same products; MIXED products differ by their
 quantisation (about 1e-7 of the largest entry) when the search directions differ by rounding,
 far below the solves' tolerance of 1e-5."""
@@ -38,7 +39,7 @@ def _pcg(grm, w, tau, b, x0, tol):
     raise AssertionError("no convergence")
 
 
-@pytest.mark.parametrize("n", [33, 255, 257, 1023, 1025, 4096, 4097, 9001, 13000])
+@pytest.mark.parametrize("n", [33, 255, 257, 1023, 1025, 4096, 4097, 9001, 13000, 16385, 32768, 32769])
 @pytest.mark.parametrize("warm", [False, True])
 def test_pcg_over_row_blocks(n, warm):
     grm = _grm(n)
