@@ -407,8 +407,16 @@ Status bed_gather_dev(const uint8_t* bed_dev, int64_t n_fam, const std::vector<i
                             cudaMemcpyHostToDevice, st));
     sp = d_sidx.as<int32_t>();
   }
+  DevBuf d_mask;
+  SubsetMask mask;
+  const bool steps = geno_out && !counts_dev && subset_compress_pays(n, n_fam);
+  const bool masked = sp && (steps || (counts_dev && !geno_out));
+  if (masked) {
+    SG_TRY(d_mask.reserve(subset_mask_words(n_fam, steps) * sizeof(uint32_t)));
+    SG_CUDA(launch_subset_mask(sp, n, n_fam, steps, d_mask.as<uint32_t>(), &mask, st));
+  }
   SG_CUDA(launch_bed_gather(bed_dev, (n_fam + 3) / 4, d_rows.as<int64_t>(), (int64_t)rows.size(),
-                            sp, n, geno_out, wpr, counts_dev, st));
+                            sp, n, geno_out, wpr, counts_dev, st, masked ? &mask : nullptr));
   SG_CUDA(cudaStreamSynchronize(st));
   return Status();
 }

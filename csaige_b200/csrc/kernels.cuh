@@ -11,10 +11,28 @@ namespace saige {
 // geno_out != NULL the 2-bit codes are written to row r of geno_out (pitch
 // words_per_row 32-bit words; padding samples coded 01 = missing).  counts
 // (2 per row, may be NULL) receive {alt-allele count, missing count}.
+// With the subset's mask, counts alone are formed without the gather.
+struct SubsetMask {
+  const uint32_t* others = nullptr;       // both bits of every sample outside the subset
+  const unsigned int* repeats = nullptr;  // not 0: the subset names a sample twice
+  // for subsets in ascending order: per word of 16 samples, how to move its kept codes
+  // together (the four steps of a bit compress) and where they go
+  const uint4* steps = nullptr;
+  const int32_t* place = nullptr;
+  const unsigned int* unsorted = nullptr;  // not 0: the subset is not strictly ascending
+  int64_t n_fam = 0;
+};
 cudaError_t launch_bed_gather(const uint8_t* bed, int64_t bytes_per_marker, const int64_t* src_rows,
                               int64_t n_rows, const int32_t* sample_idx, int64_t n,
                               uint32_t* geno_out, int64_t words_per_row, int64_t* counts,
-                              cudaStream_t st);
+                              cudaStream_t st, const SubsetMask* mask = nullptr);
+// The mask of sidx[0 .. n) among n_fam samples, in `words` (subset_mask_words(n_fam, steps) of
+// them, 16-byte aligned), with the steps of an ascending subset when asked for.
+size_t subset_mask_words(int64_t n_fam, bool steps);
+cudaError_t launch_subset_mask(const int32_t* sidx, int64_t n, int64_t n_fam, bool steps,
+                               uint32_t* words, SubsetMask* mask, cudaStream_t st);
+// Whether launch_bed_gather takes the steps for rows of n out of n_fam samples.
+bool subset_compress_pays(int64_t n, int64_t n_fam);
 
 // Alt-allele and missing counts of rows j0 .. j0 + n_rows of the raw .bed for several
 // sample subsets at once: subset c is sidx[offs[c] .. offs[c] + ns[c]) (offs[c] a

@@ -153,11 +153,15 @@ __device__ __forceinline__ void store_counts(long long alt, long long miss, int6
 // planes together, the low plane, and their product).  40,000 rows of 200,000 samples:
 // counts 1.35 ms with a byte per load, 64-bit counters and every word handled as if it
 // were the last; now 0.48 ms with a block per row, 0.39 ms with a warp (5.1 TB/s).
-template <int kGroup, bool kOut, bool kCounts>
+// kMask: the counts of a sample subset without repeats, whose other samples the mask turns
+// into 11 (which counts as nothing).
+template <int kGroup, bool kOut, bool kCounts, bool kMask = false>
 __global__ void __launch_bounds__(kThreads)
     bed_rows_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
                     const int64_t* __restrict__ src_rows, int64_t n_rows, int64_t n,
-                    uint32_t* __restrict__ out, int64_t wpr, int64_t* __restrict__ counts) {
+                    uint32_t* __restrict__ out, int64_t wpr, int64_t* __restrict__ counts,
+                    const SubsetMask mask = SubsetMask()) {
+  if (kMask && *mask.repeats) return;  // bed_subset_kernel counts
   const int64_t r = (int64_t)blockIdx.x * (kThreads / kGroup) + threadIdx.x / kGroup;
   if (r >= n_rows) return;  // whole warps (kGroup 32) or, never, whole blocks
   const uint8_t* row = bed + 3 + src_rows[r] * bpm;
@@ -173,7 +177,8 @@ __global__ void __launch_bounds__(kThreads)
   const int first = j;
 #pragma unroll 8
   for (; j < n_fast; j += kGroup) {
-    const uint32_t w = __funnelshift_r(__ldg(base + j), __ldg(base + j + 1), 8 * off);
+    uint32_t w = __funnelshift_r(__ldg(base + j), __ldg(base + j + 1), 8 * off);
+    if (kMask) w |= __ldg(mask.others + j);
     if (kCounts) {
       const uint32_t lo = w & 0x55555555u;
       both += __popc(w);
@@ -201,6 +206,7 @@ __global__ void __launch_bounds__(kThreads)
         const int64_t bi = 4 * (int64_t)j + b;
         if (bi < bpm) word |= (uint32_t)row[bi] << (8 * b);
       }
+      if (kMask) word |= __ldg(mask.others + j);
       const uint32_t keep = left >= 16 ? 0xFFFFFFFFu : ((1u << (2 * (int)left)) - 1u);
       if (kCounts) count_word(word, keep & 0x55555555u, alt, miss);
       w = to_device_layout((word & keep) | ~keep);
@@ -214,7 +220,7 @@ __global__ void __launch_bounds__(kThreads)
 // read from global memory, for rows too long to stage): each thread loads the 16 sample
 // indices of a packed word once and gathers that word from every staged row.  Bound: the
 // index loads (64 bytes from L2 per 4-byte word and row with a row per block) and the bank
-// conflicts of the byte gathers.  40,000 rows of 60,013 of 150,001 samples: 2.10 ms with a
+// conflicts of the byte gathers.  39,001 rows of 60,000 of 150,001 samples: 2.10 ms with a
 // row per block, 1.59 ms with three.  (Lane = sample with two ballots per 32 samples has no
 // bank conflicts but took 2.37 ms: the votes bound it.)
 constexpr int kSubsetThreads = 512;
@@ -224,8 +230,10 @@ __global__ void __launch_bounds__(kSubsetThreads, 2)
     bed_subset_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
                       const int64_t* __restrict__ src_rows, int64_t n_rows,
                       const int32_t* __restrict__ sidx, int64_t n, uint32_t* __restrict__ out,
-                      int64_t wpr, int64_t* __restrict__ counts) {
+                      int64_t wpr, int64_t* __restrict__ counts,
+                      const unsigned int* __restrict__ only_if) {
   constexpr int R = kRows ? kRows : 1;
+  if (only_if && !*only_if) return;  // counted through the mask, or compressed
   extern __shared__ __align__(16) uint8_t row_s[];
   __shared__ int red[2 * R][kSubsetThreads / 32];
   const int64_t r0 = (int64_t)blockIdx.x * R;
@@ -474,11 +482,238 @@ cudaError_t launch_bed_count_cohorts(const uint8_t* bed, int64_t bpm, int64_t j0
   return cudaGetLastError();
 }
 
+__global__ void subset_mask_kernel(const int32_t* __restrict__ sidx, int64_t n,
+                                   uint32_t* __restrict__ others,
+                                   unsigned int* __restrict__ repeats,
+                                   unsigned int* __restrict__ unsorted) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t s = sidx[i];
+  const uint32_t bits = 3u << (2 * (s & 15));
+  if (!(atomicAnd(&others[s >> 4], ~bits) & bits)) *repeats = 1u;
+  if (i + 1 < n && sidx[i + 1] <= s) *unsorted = 1u;
+}
+
+// The even bits 0, 2, .. of x as bits 0, 1, ..; and each of 16 bits as a pair.
+__device__ __forceinline__ uint32_t gather_even(uint32_t x) {
+  x &= 0x55555555u;
+  x = (x | (x >> 1)) & 0x33333333u;
+  x = (x | (x >> 2)) & 0x0F0F0F0Fu;
+  x = (x | (x >> 4)) & 0x00FF00FFu;
+  return (x | (x >> 8)) & 0xFFFFu;
+}
+__device__ __forceinline__ uint32_t pairs_of(uint32_t m) {
+  m = (m | (m << 8)) & 0x00FF00FFu;
+  m = (m | (m << 4)) & 0x0F0F0F0Fu;
+  m = (m | (m << 2)) & 0x33333333u;
+  m = (m | (m << 1)) & 0x55555555u;
+  return m | (m << 1);
+}
+
+// The compress steps of each word (the parallel-prefix method of Warren, Hacker's Delight,
+// 7-4): step e moves by 2^e places the codes whose count of left-out samples below them has
+// bit e set.  And how many of the (ascending) subset's samples lie below the word.
+__global__ void subset_steps_kernel(const int32_t* __restrict__ sidx, int64_t n,
+                                    const uint32_t* __restrict__ others, int64_t n_words,
+                                    uint4* __restrict__ steps, int32_t* __restrict__ place) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n_words) return;
+  uint32_t m = ~gather_even(others[j]) & 0xFFFFu, mk = (~m << 1) & 0xFFFFu;
+  uint32_t mv[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    uint32_t mp = mk ^ (mk << 1);
+    mp ^= mp << 2;
+    mp ^= mp << 4;
+    mp ^= mp << 8;
+    const uint32_t move = mp & m;
+    mv[e] = pairs_of(move & 0xFFFFu);
+    m = (m ^ move) | (move >> (1 << e));
+    mk &= ~mp;
+  }
+  steps[j] = make_uint4(mv[0], mv[1], mv[2], mv[3]);
+  int64_t lo = 0, hi = n;  // first index with sidx >= 16 j
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) / 2;
+    if (sidx[mid] < 16 * j)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  place[j] = (int32_t)lo;
+}
+
+size_t subset_mask_words(int64_t n_fam, bool steps) {
+  const size_t k = (size_t)round_up(ceil_div(n_fam, (int64_t)16), (int64_t)4);
+  return k + 4 + (steps ? 5 * k : 0);
+}
+
+cudaError_t launch_subset_mask(const int32_t* sidx, int64_t n, int64_t n_fam, bool steps,
+                               uint32_t* words, SubsetMask* mask, cudaStream_t st) {
+  const int64_t n_words = ceil_div(n_fam, (int64_t)16);
+  const size_t k = (size_t)round_up(n_words, (int64_t)4);
+  unsigned int* flags = words + k;
+  mask->others = words;
+  mask->repeats = flags;
+  mask->unsorted = flags + 1;
+  mask->n_fam = n_fam;
+  cudaError_t e = cudaMemsetAsync(words, 0xFF, k * 4, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 16, st);
+  if (e != cudaSuccess) return e;
+  subset_mask_kernel<<<(unsigned)ceil_div(n, (int64_t)256), 256, 0, st>>>(sidx, n, words, flags,
+                                                                         flags + 1);
+  count_launches(1);
+  if (steps) {
+    uint4* s4 = reinterpret_cast<uint4*>(flags + 4);
+    int32_t* place = reinterpret_cast<int32_t*>(s4 + k);
+    subset_steps_kernel<<<(unsigned)ceil_div(n_words, (int64_t)128), 128, 0, st>>>(
+        sidx, n, words, n_words, s4, place);
+    count_launches(1);
+    mask->steps = s4;
+    mask->place = place;
+  }
+  return cudaGetLastError();
+}
+
+// The packed rows of an ascending subset, kRows rows per block: each thread compresses a word
+// of 16 samples at a time (its steps loaded once for the rows) and ORs the kept codes into the
+// rows' packed words in shared memory.  Bound by the latency of a word's loads and by the ORs
+// (kCompressThreads 256: 0.83 ms where the packed rows leave room for more blocks, 1.27 at 40 %
+// kept; 1,024: 1.33).
+constexpr int kCompressThreads = 512;
+template <int kRows>
+__global__ void __launch_bounds__(kCompressThreads)
+    bed_compress_kernel(const uint8_t* __restrict__ bed, int64_t bpm,
+                        const int64_t* __restrict__ src_rows, int64_t n_rows,
+                        const SubsetMask mask, int64_t n, uint32_t* __restrict__ out,
+                        int64_t wpr) {
+  extern __shared__ __align__(16) uint32_t packed[];  // kRows x stride
+  if (*mask.unsorted) return;  // bed_subset_kernel gathers
+  const int64_t r0 = (int64_t)blockIdx.x * kRows;
+  const int nr = n_rows - r0 < kRows ? (int)(n_rows - r0) : kRows;
+  const int n_real = (int)((n + 15) / 16), stride = n_real + 1;
+  for (int i = threadIdx.x; i < kRows * stride; i += kCompressThreads) packed[i] = 0u;
+  const uint8_t* row[kRows];
+  const uint32_t* base[kRows];
+  int off[kRows];
+  int n_fast = (int)(mask.n_fam / 16);
+#pragma unroll
+  for (int q = 0; q < kRows; ++q) {
+    row[q] = bed + 3 + src_rows[r0 + (q < nr ? q : 0)] * bpm;
+    off[q] = (int)(reinterpret_cast<uintptr_t>(row[q]) & 3u);
+    base[q] = reinterpret_cast<const uint32_t*>(row[q] - off[q]);
+    // words whose two aligned words end inside the row
+    const int64_t safe = bpm + off[q] >= 8 ? (bpm + off[q] - 8) / 4 + 1 : 0;
+    if (safe < n_fast) n_fast = (int)safe;
+  }
+  __syncthreads();
+  const int n_src = (int)((mask.n_fam + 15) / 16);
+#pragma unroll 2
+  for (int j = threadIdx.x; j < n_src; j += kCompressThreads) {
+    const uint32_t keep = ~__ldg(mask.others + j);
+    if (!keep) continue;
+    uint32_t w[kRows];
+    if (j < n_fast) {
+#pragma unroll
+      for (int q = 0; q < kRows; ++q)
+        w[q] = __funnelshift_r(__ldg(base[q] + j), __ldg(base[q] + j + 1), 8 * off[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) {
+        w[q] = 0u;
+        for (int b = 0; b < 4; ++b) {
+          const int64_t bi = 4 * (int64_t)j + b;
+          if (bi < bpm) w[q] |= (uint32_t)row[q][bi] << (8 * b);
+        }
+      }
+    }
+    const uint4 mv = __ldg(mask.steps + j);
+    const int at = __ldg(mask.place + j), sh = 2 * (at & 15);
+    uint32_t* to = packed + (at >> 4);
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      uint32_t x = w[q] & keep, t;
+      t = x & mv.x;
+      x = (x ^ t) | (t >> 2);
+      t = x & mv.y;
+      x = (x ^ t) | (t >> 4);
+      t = x & mv.z;
+      x = (x ^ t) | (t >> 8);
+      t = x & mv.w;
+      x = (x ^ t) | (t >> 16);
+      const uint32_t lo = x << sh, hi = __funnelshift_l(x, 0u, sh);
+      if (lo) atomicOr(to + q * stride, lo);
+      if (hi) atomicOr(to + q * stride + 1, hi);  // (at most n codes: the spare word stays 0)
+    }
+  }
+  __syncthreads();
+  for (int q = 0; q < nr; ++q)
+    for (int64_t j = threadIdx.x; j < wpr; j += kCompressThreads) {
+      uint32_t w = 0xFFFFFFFFu;  // padding samples: code 11
+      if (j < n_real) {
+        const int64_t left = n - 16 * j;
+        const uint32_t keep = left >= 16 ? 0xFFFFFFFFu : ((1u << (2 * (int)left)) - 1u);
+        w = to_device_layout((packed[q * stride + j] & keep) | ~keep);
+      }
+      out[(r0 + q) * wpr + j] = w;
+    }
+}
+
+// 39,001 rows of 150,001 samples, compressed against gathered: 0.99 against 1.08 ms with 17 % of
+// the samples kept, 1.03 / 1.26 with 25 %, 1.09 / 1.58 with 40 %, 1.27 / 2.17 with 70 %, 1.52 /
+// 2.67 with 95 %.  The gather's time goes with the samples kept, the compress's with all.
+bool subset_compress_pays(int64_t n, int64_t n_fam) {
+  return 6 * n >= n_fam && (n + 31) / 16 * 4 <= kSmemRowMax;
+}
+
 cudaError_t launch_bed_gather(const uint8_t* bed, int64_t bpm, const int64_t* src_rows,
                               int64_t n_rows, const int32_t* sample_idx, int64_t n,
                               uint32_t* geno_out, int64_t words_per_row, int64_t* counts,
-                              cudaStream_t st) {
+                              cudaStream_t st, const SubsetMask* mask) {
   if (n_rows <= 0 || (!geno_out && !counts)) return cudaSuccess;
+  // Counts alone need no gather: the whole row is read against the subset's mask, as the
+  // gather's staging reads it whole (40,000 rows, 60,013 of 150,001 samples: 1.59 ms gathered,
+  // 0.41 ms masked).  A small subset of rows too long to stage is gathered from global
+  // memory: it touches at most n of the row's sectors.
+  const bool masked = sample_idx && mask && counts && !geno_out &&
+                      (bpm <= kSmemRowMax || 32 * n >= bpm);
+  if (masked) {
+    const int64_t n_fam = mask->n_fam;
+    const bool shortrow = bpm <= 2048 || n_rows >= 148 * 16;
+    const unsigned grid =
+        (unsigned)(shortrow ? ceil_div(n_rows, (int64_t)(kThreads / 32)) : n_rows);
+    if (shortrow)
+      bed_rows_kernel<32, false, true, true><<<grid, kThreads, 0, st>>>(
+          bed, bpm, src_rows, n_rows, n_fam, nullptr, 0, counts, *mask);
+    else
+      bed_rows_kernel<kThreads, false, true, true><<<grid, kThreads, 0, st>>>(
+          bed, bpm, src_rows, n_rows, n_fam, nullptr, 0, counts, *mask);
+    count_launches(1);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  const bool compressed =
+      sample_idx && mask && mask->steps && geno_out && !counts && subset_compress_pays(n, mask->n_fam);
+  if (compressed) {
+    const int64_t per_row = ((n + 15) / 16 + 1) * 4;
+    const int rows = 4 * per_row <= kSmemHalf ? 4 : (2 * per_row <= kSmemHalf ? 2 : 1);
+    auto go = [&](auto kern) -> cudaError_t {
+      const size_t smem = (size_t)(per_row * rows);
+      if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (e != cudaSuccess) return e;
+      }
+      kern<<<(unsigned)ceil_div(n_rows, (int64_t)rows), kCompressThreads, smem, st>>>(
+          bed, bpm, src_rows, n_rows, *mask, n, geno_out, words_per_row);
+      return cudaGetLastError();
+    };
+    count_launches(1);
+    cudaError_t e = rows == 4   ? go(bed_compress_kernel<4>)
+                    : rows == 2 ? go(bed_compress_kernel<2>)
+                                : go(bed_compress_kernel<1>);
+    if (e != cudaSuccess) return e;
+  }
   if (sample_idx) {
     // as many rows per block as half an SM's shared memory holds (two blocks of 16 warps
     // per SM, so that one stages while the other gathers), at most four; a row beyond
@@ -494,7 +729,8 @@ cudaError_t launch_bed_gather(const uint8_t* bed, int64_t bpm, const int64_t* sr
         if (e != cudaSuccess) return e;
       }
       kern<<<(unsigned)ceil_div(n_rows, (int64_t)per), kSubsetThreads, smem, st>>>(
-          bed, bpm, src_rows, n_rows, sample_idx, n, geno_out, words_per_row, counts);
+          bed, bpm, src_rows, n_rows, sample_idx, n, geno_out, words_per_row, counts,
+          masked ? mask->repeats : (compressed ? mask->unsorted : nullptr));
       return cudaGetLastError();
     };
     cudaError_t e = rows == 4   ? go(bed_subset_kernel<4>, 4)
@@ -513,7 +749,8 @@ cudaError_t launch_bed_gather(const uint8_t* bed, int64_t bpm, const int64_t* sr
   const bool shortrow = bpm <= 2048 || (n_rows >= 148 * 16 && (!geno_out || bpm <= 16 * 1024));
   const unsigned grid = (unsigned)(shortrow ? ceil_div(n_rows, (int64_t)(kThreads / 32)) : n_rows);
   auto go = [&](auto kern) {
-    kern<<<grid, kThreads, 0, st>>>(bed, bpm, src_rows, n_rows, n, geno_out, words_per_row, counts);
+    kern<<<grid, kThreads, 0, st>>>(bed, bpm, src_rows, n_rows, n, geno_out, words_per_row, counts,
+                                    SubsetMask());
   };
   if (shortrow) {
     if (geno_out && counts) go(bed_rows_kernel<32, true, true>);
