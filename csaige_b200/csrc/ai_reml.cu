@@ -188,9 +188,16 @@ Status solve_each(Fit& f, const double* x0, const double tau[2]) {
   return Status();
 }
 
-// P-projection (ai_reml.rs:242-251) of q solved columns sol (in place):
-// sol -= SinvX C^-1 (SinvX' u).
-Status p_project(Fit& f, double* sol, const double* u, int q, const std::vector<double>& l) {
+// P-projection (ai_reml.rs:242-251) of q solved columns: out = sol - SinvX C^-1 (SinvX' u); the
+// coefficients stay in f.dsmall.
+Status p_project(Fit& f, const double* sol, double* out, const double* u, int q,
+                 const std::vector<double>& l) {
+  if (f.p <= kCholMax) {
+    SG_CUDA(cross_dots(f.sol + f.ld, f.p, u, q, nullptr, f.n, f.ld, f.partial, f.dsmall, f.st));
+    SG_CUDA(chol_cols(l.data(), f.p, f.dsmall, q, f.st));
+    SG_CUDA(sub_combo(sol, out, q, f.sol + f.ld, f.p, f.dsmall, f.n, f.ld, f.st));
+    return Status();
+  }
   std::vector<double> t;
   SG_TRY(dots(f, f.sol + f.ld, f.p, u, q, nullptr, t));  // p x q
   std::vector<double> coef((size_t)f.p * q), col((size_t)f.p), corr((size_t)f.p);
@@ -200,7 +207,7 @@ Status p_project(Fit& f, double* sol, const double* u, int q, const std::vector<
     for (int j = 0; j < f.p; ++j) coef[(size_t)j * q + c] = corr[(size_t)j];
   }
   SG_CUDA(cudaMemcpyAsync(f.dsmall, coef.data(), coef.size() * 8, cudaMemcpyHostToDevice, f.st));
-  SG_CUDA(sub_combo(sol, q, f.sol + f.ld, f.p, f.dsmall, f.n, f.ld, f.st));
+  SG_CUDA(sub_combo(sol, out, q, f.sol + f.ld, f.p, f.dsmall, f.n, f.ld, f.st));
   return Status();
 }
 
@@ -381,9 +388,8 @@ Status basis_cols(Fit& f, Recycle& rc, int at, const double* x, const double* kx
                   const double tau[2]) {
   const int64_t ld = f.ld;
   if (at + k > rc.mb_max) return fail(SAIGE_EINVAL, "start basis beyond its %d columns", rc.mb_max);
-  SG_TRY(copy_cols(f, x, rc.v + (size_t)at * ld, k));
-  SG_TRY(copy_cols(f, kx, rc.kv + (size_t)at * ld, k));
-  SG_CUDA(sigma_image(x, kx, f.wmax, tau[0], tau[1], rc.av + (size_t)at * ld, f.n, ld, k, f.st));
+  SG_CUDA(sigma_image(x, kx, f.wmax, tau[0], tau[1], rc.v + (size_t)at * ld,
+                      rc.kv + (size_t)at * ld, rc.av + (size_t)at * ld, f.n, ld, k, f.st));
   return Status();
 }
 
@@ -448,8 +454,7 @@ Status block_solve_recycled(Fit& f, Recycle& rc, const double* x0_prev, const do
 // scratch also takes dot results).
 Status kpy_combine(Fit& f, Recycle& rc, const std::vector<double>& alpha) {
   SG_CUDA(cudaMemcpyAsync(f.dsmall, alpha.data(), (size_t)f.p * 8, cudaMemcpyHostToDevice, f.st));
-  SG_TRY(copy_cols(f, rc.kblock, f.kpy, 1));
-  SG_CUDA(sub_combo(f.kpy, 1, rc.kblock + f.ld, f.p, f.dsmall, f.n, f.ld, f.st));
+  SG_CUDA(sub_combo(rc.kblock, f.kpy, 1, rc.kblock + f.ld, f.p, f.dsmall, f.n, f.ld, f.st));
   return Status();
 }
 
@@ -802,8 +807,7 @@ static Status fit_impl(saige_grm* h, const double* y, const double* x, int64_t n
     SG_CUDA(eta_mu(f.x, p, f.dsmall, trait, f.eta, f.mu, n, ld, f.st));
 
     // P y = Sinv y - SinvX alpha; YPAPY = Py' K Py (ai_reml.rs:221-232)
-    SG_TRY(copy_cols(f, SinvY, f.py, 1));
-    SG_CUDA(sub_combo(f.py, 1, SinvX, p, f.dsmall, n, ld, f.st));
+    SG_CUDA(sub_combo(SinvY, f.py, 1, SinvX, p, f.dsmall, n, ld, f.st));
     if (recyc && cfg->solve == SAIGE_SOLVE_BLOCK && block_kx && !rc.learned) {
       SG_TRY(kpy_from_block(f, rc, alpha));  // K X*_t and K Py without a launch
     } else if (recyc && cfg->solve == SAIGE_SOLVE_BLOCK) {
@@ -817,16 +821,15 @@ static Status fit_impl(saige_grm* h, const double* y, const double* x, int64_t n
     const double ypapy = r1[0];
 
     // Hutchinson trace of P K (ai_reml.rs:237-258)
-    SG_TRY(copy_cols(f, SinvU, f.pu, f.nrv));
-    SG_TRY(p_project(f, f.pu, U, f.nrv, l));
+    SG_TRY(p_project(f, SinvU, f.pu, U, f.nrv, l));
     std::vector<double> tr;
     if (rc.kxu_ok) {
       SG_TRY(coldots(f, f.ku, f.pu, f.nrv, tr));  // (K u)' P u
     } else {
       // u' K P u with K P u = K Sinv U - K Sinv X coef (coef of the projection above,
       // still in f.dsmall; rc.kblock = K [Sinv y | Sinv X | Sinv U] of this iteration)
-      SG_TRY(copy_cols(f, rc.kblock + (size_t)(1 + p) * ld, f.tmpq, f.nrv));
-      SG_CUDA(sub_combo(f.tmpq, f.nrv, rc.kblock + ld, p, f.dsmall, n, ld, f.st));
+      SG_CUDA(sub_combo(rc.kblock + (size_t)(1 + p) * ld, f.tmpq, f.nrv, rc.kblock + ld, p, f.dsmall,
+                        n, ld, f.st));
       SG_TRY(coldots(f, U, f.tmpq, f.nrv, tr));
     }
     double trace_sum = 0.0;
@@ -844,8 +847,7 @@ static Status fit_impl(saige_grm* h, const double* y, const double* x, int64_t n
     }
     f.have_prev_pk = true;
     tm.mark("  ai solve");
-    SG_TRY(copy_cols(f, f.pk_raw, f.pk, 1));
-    SG_TRY(p_project(f, f.pk, f.kpy, 1, l));
+    SG_TRY(p_project(f, f.pk_raw, f.pk, f.kpy, 1, l));
     SG_TRY(coldots(f, f.kpy, f.pk, 1, r1));
     const double ai_11 = r1[0];
 
@@ -867,8 +869,7 @@ static Status fit_impl(saige_grm* h, const double* y, const double* x, int64_t n
         SG_TRY(solve(f, f.invw_py, f.pw_raw, (warm && f.have_prev_pw) ? f.tmpq : nullptr, 1, tau));
       }
       f.have_prev_pw = true;
-      SG_TRY(copy_cols(f, f.pw_raw, f.pw, 1));
-      SG_TRY(p_project(f, f.pw, f.invw_py, 1, l));
+      SG_TRY(p_project(f, f.pw_raw, f.pw, f.invw_py, 1, l));
       SG_TRY(coldots(f, f.invw_py, f.pw, 1, r1));
       ai_00 = r1[0];
       SG_TRY(coldots(f, f.invw_py, f.pk, 1, r1));

@@ -1355,8 +1355,11 @@ SG_API int32_t saige_grm_matvec(saige_grm* h, const double* v, double* out, int6
     SG_TRY(h->ws_io.reserve(2 * blk));
     double* dv = h->ws_io.as<double>();
     double* dk = dv + (size_t)h->n_pad * nrhs;
-    SG_TRY(upload_block(h, v, dv, nrhs, h->stream));
+    // (products read n rows)
+    SG_CUDA(cudaMemcpy2DAsync(dv, (size_t)h->n_pad * 8, v, (size_t)n * 8, (size_t)n * 8,
+                              (size_t)nrhs, cudaMemcpyHostToDevice, h->stream));
     SG_TRY(grm_product(h, dv, dk, nrhs, nullptr, precision, h->stream));
+    if (nrhs == 1) return read_back(h, out, dk, (size_t)n * 8, h->stream);
     SG_TRY(download_block(h, dk, out, nrhs, h->stream));
     SG_CUDA(cudaStreamSynchronize(h->stream));
     return Status();
@@ -1380,8 +1383,7 @@ SG_API int32_t saige_grm_matvec_dev(saige_grm* h, const double* v_dev, double* o
     SG_TRY(h->ws_io.reserve(2 * blk));
     double* dv = h->ws_io.as<double>();
     double* dk = dv + (size_t)h->n_pad * nrhs;
-    SG_TRY(devcopy_block(h, v_dev, h->n, dv, h->n_pad, nrhs, st));
-    SG_CUDA(zero_pad(dv, h->n, h->n_pad, nrhs, st));
+    SG_TRY(devcopy_block(h, v_dev, h->n, dv, h->n_pad, nrhs, st));  // (products read n rows)
     SG_TRY(grm_product(h, dv, dk, nrhs, nullptr, precision, st));
     SG_TRY(devcopy_block(h, dk, h->n_pad, out_dev, h->n, nrhs, st));
     SG_CUDA(cudaStreamSynchronize(st));

@@ -178,7 +178,7 @@ Status grm_stream_rows_finish(saige_grm* h, const std::vector<int64_t>& pass, co
 // fit_null.rs:209-222's marker QC over n samples (MAF and call rate).
 bool marker_qc_pass(double af, int64_t n_valid, int64_t n, double min_maf, double max_missing);
 
-// Kv for q columns of v (ld = h->n_pad, padding rows zero) into kp.
+// Kv for q columns of v (ld = h->n_pad; rows n .. ld - 1 are not read) into kp.
 // active (host, length q, may be NULL) selects columns; others are skipped.
 // With `later` (page-locked), a MIXED product returns without waiting, its error word (0: none)
 // to arrive there in stream order, and the caller passes it to grm_product_check once st has

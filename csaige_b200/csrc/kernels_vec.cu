@@ -6,6 +6,8 @@
 #include <cooperative_groups.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels_vec.cuh"
 #include "rng.hpp"
@@ -645,15 +647,38 @@ __global__ void init_mu_kernel(const double* __restrict__ y, int t, double* __re
   eta[i] = e;
 }
 
-__global__ void sub_combo_kernel(double* __restrict__ y, int q, const double* __restrict__ a,
-                                 int p, const double* __restrict__ coef, int64_t n, int64_t ld) {
+// y = from - A coef (from may be y); rows n .. ld - 1 become from's.
+__global__ void sub_combo_kernel(const double* from, double* y, int q,
+                                 const double* __restrict__ a, int p,
+                                 const double* __restrict__ coef, int64_t n, int64_t ld) {
   const int c = blockIdx.y;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = y[(int64_t)c * ld + i];
+  if (i >= ld) return;
+  double v = from[(int64_t)c * ld + i];
   // ai_reml.rs:247-251: one subtraction per covariate column, in order
-  for (int j = 0; j < p; ++j) v -= a[(int64_t)j * ld + i] * coef[j * q + c];
+  if (i < n)
+    for (int j = 0; j < p; ++j) v -= a[(int64_t)j * ld + i] * coef[j * q + c];
   y[(int64_t)c * ld + i] = v;
+}
+
+// t (p x q, row-major): each column's solve with the Cholesky factor l, with the host's
+// operations in the host's order (decomposition.rs:64-89).  A few hundred operations: a
+// microsecond or two, in place of a read, a wait and a copy back.
+__global__ void __launch_bounds__(64)
+    chol_cols_kernel(const CholFactor l, int p, double* __restrict__ t, int q) {
+  const int c = blockIdx.x * 64 + threadIdx.x;
+  if (c >= q) return;
+  double y[kCholMax];
+  for (int i = 0; i < p; ++i) {
+    double s = 0.0;
+    for (int j = 0; j < i; ++j) s = __dadd_rn(s, __dmul_rn(l.v[i * p + j], y[j]));
+    y[i] = __ddiv_rn(__dsub_rn(t[i * q + c], s), l.v[i * p + i]);
+  }
+  for (int i = p - 1; i >= 0; --i) {
+    double s = 0.0;
+    for (int j = i + 1; j < p; ++j) s = __dadd_rn(s, __dmul_rn(l.v[j * p + i], t[j * q + c]));
+    t[i * q + c] = __ddiv_rn(__dsub_rn(y[i], s), l.v[i * p + i]);
+  }
 }
 
 __global__ void div_w_kernel(const double* __restrict__ v, const double* __restrict__ w,
@@ -888,9 +913,18 @@ cudaError_t init_mu(const double* y, int trait, double* mu, double* eta, int64_t
   return cudaGetLastError();
 }
 
-cudaError_t sub_combo(double* y, int q, const double* a, int p, const double* coef, int64_t n,
-                      int64_t ld, cudaStream_t st) {
-  sub_combo_kernel<<<dim3(g1(n), q), kT, 0, st>>>(y, q, a, p, coef, n, ld);
+cudaError_t sub_combo(const double* from, double* y, int q, const double* a, int p,
+                      const double* coef, int64_t n, int64_t ld, cudaStream_t st) {
+  sub_combo_kernel<<<dim3(g1(ld), q), kT, 0, st>>>(from, y, q, a, p, coef, n, ld);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t chol_cols(const double* l, int p, double* t, int q, cudaStream_t st) {
+  if (p > kCholMax) return cudaErrorInvalidValue;
+  CholFactor f{};
+  std::copy(l, l + p * p, f.v);
+  chol_cols_kernel<<<(unsigned)ceil_div(q, 64), 64, 0, st>>>(f, p, t, q);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -80,9 +80,16 @@ cudaError_t work_vectors(const double* y, const double* eta, const double* mu, i
 // mu = initialize_mu(y), eta = link(mu)  (family.rs:23-45)
 cudaError_t init_mu(const double* y, int trait, double* mu, double* eta, int64_t n,
                     cudaStream_t st);
-// Y[:,c] -= sum_j A[:,j] coef[j*q + c]   (A: n x p, Y: n x q)
-cudaError_t sub_combo(double* y, int q, const double* a, int p, const double* coef, int64_t n,
-                      int64_t ld, cudaStream_t st);
+// Y[:,c] = from[:,c] - sum_j A[:,j] coef[j*q + c]   (A: n x p, Y: n x q)
+// (from may be y; otherwise rows n .. ld - 1 of y become from's)
+cudaError_t sub_combo(const double* from, double* y, int q, const double* a, int p,
+                      const double* coef, int64_t n, int64_t ld, cudaStream_t st);
+// t (p x q on the device, row-major; p <= kCholMax) = (L L')^-1 t for the factor l on the host.
+constexpr int kCholMax = 16;
+struct CholFactor {
+  double v[kCholMax * kCholMax];
+};
+cudaError_t chol_cols(const double* l, int p, double* t, int q, cudaStream_t st);
 // out = v / max(w,1e-30)
 cudaError_t div_w(const double* v, const double* w, double* out, int64_t n, int64_t ld, int q,
                   cudaStream_t st);

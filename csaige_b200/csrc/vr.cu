@@ -331,7 +331,7 @@ Status vr_run(saige_grm* h, const VrFill& fill, int64_t n_cand, const double* ma
     SG_CHECK_LAUNCH();
     // X adjustment: G -= X (A' G)
     SG_CUDA(cross_dots(dA, p, dG, q, nullptr, n, ld, dPart, dT, st));
-    SG_CUDA(sub_combo(dG, q, dX, p, dT, n, ld, st));
+    SG_CUDA(sub_combo(dG, dG, q, dX, p, dT, n, ld, st));
     // Sigma^-1 g_tilde for the whole block (PcgSolver::new(1e-5, 500), zero start)
     PcgRun run;
     run.b = dG;

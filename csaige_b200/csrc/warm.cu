@@ -162,13 +162,17 @@ __global__ void combo_kernel(const double* __restrict__ V, int m, const double* 
 }
 
 // out may be kv (each element is read before it is written by the same thread)
-__global__ void sigma_image_kernel(const double* v, const double* kv,
+__global__ void sigma_image_kernel(const double* __restrict__ v, const double* __restrict__ kv,
                                    const double* __restrict__ wmax, double tau0, double tau1,
-                                   double* out, int64_t n, int64_t ld) {
+                                   double* __restrict__ v_out, double* __restrict__ kv_out,
+                                   double* __restrict__ out, int64_t n, int64_t ld) {
   const int64_t c = blockIdx.y;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  out[c * ld + i] = tau0 * v[c * ld + i] / wmax[i] + tau1 * kv[c * ld + i];
+  if (i >= ld) return;
+  const double x = v[c * ld + i], kx = kv[c * ld + i];
+  v_out[c * ld + i] = x;
+  kv_out[c * ld + i] = kx;
+  if (i < n) out[c * ld + i] = tau0 * x / wmax[i] + tau1 * kx;
 }
 
 __global__ void sub_cols_kernel(const double* __restrict__ a, const double* __restrict__ b,
@@ -332,10 +336,11 @@ cudaError_t combo(const double* V, int m, const double* G, int q, double* Y, boo
 }
 
 cudaError_t sigma_image(const double* v, const double* kv, const double* wmax, double tau0,
-                        double tau1, double* out, int64_t n, int64_t ld, int q, cudaStream_t st) {
+                        double tau1, double* v_out, double* kv_out, double* out, int64_t n,
+                        int64_t ld, int q, cudaStream_t st) {
   if (q <= 0) return cudaSuccess;
-  sigma_image_kernel<<<dim3((unsigned)ceil_div(n, 256), (unsigned)q), 256, 0, st>>>(
-      v, kv, wmax, tau0, tau1, out, n, ld);
+  sigma_image_kernel<<<dim3((unsigned)ceil_div(ld, 256), (unsigned)q), 256, 0, st>>>(
+      v, kv, wmax, tau0, tau1, v_out, kv_out, out, n, ld);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -22,9 +22,11 @@ cudaError_t gram(const double* A, int a, const double* B, int b, int64_t n, int6
 cudaError_t combo(const double* V, int m, const double* G, int q, double* Y, bool add, int64_t n,
                   int64_t ld, cudaStream_t st);
 
-// out[:, c] = tau0 v[:, c] / wmax + tau1 kv[:, c]  (the fit-null Sigma applied to v given K v)
+// out[:, c] = tau0 v[:, c] / wmax + tau1 kv[:, c]  (the fit-null Sigma applied to v given K v),
+// and v and kv copied (all ld rows) to v_out and kv_out; none of the outputs overlaps v or kv.
 cudaError_t sigma_image(const double* v, const double* kv, const double* wmax, double tau0,
-                        double tau1, double* out, int64_t n, int64_t ld, int q, cudaStream_t st);
+                        double tau1, double* v_out, double* kv_out, double* out, int64_t n,
+                        int64_t ld, int q, cudaStream_t st);
 
 // out[:, c] = a[:, c] - b[:, c]
 cudaError_t sub_cols(const double* a, const double* b, double* out, int64_t n, int64_t ld, int q,
