@@ -72,18 +72,34 @@ struct Fit {
   bool have_prev = false, have_prev_pk = false, have_prev_pw = false;
 };
 
+// Where k dot products go: the handle's page-locked block when their one launch can write it.
+double* dots_out(Fit& f, size_t k) {
+  void* p = one_launch_columns(f.n) && k * sizeof(double) <= kPinReads ? f.h->pin.get() : nullptr;
+  return p ? static_cast<double*>(p) : f.dsmall;
+}
+
 Status dots(Fit& f, const double* a, int pa, const double* b, int qb, const double* wv,
             std::vector<double>& out) {
-  double* dout = f.dsmall;
-  SG_CUDA(cross_dots(a, pa, b, qb, wv, f.n, f.ld, f.partial, dout, f.st));
   out.resize((size_t)pa * qb);
+  double* dout = dots_out(f, out.size());
+  SG_CUDA(cross_dots(a, pa, b, qb, wv, f.n, f.ld, f.partial, dout, f.st));
+  if (dout != f.dsmall) {
+    SG_CUDA(cudaStreamSynchronize(f.st));
+    std::copy(dout, dout + out.size(), out.begin());
+    return Status();
+  }
   return read_back(f.h, out.data(), dout, out.size() * 8, f.st);
 }
 
 Status coldots(Fit& f, const double* a, const double* b, int q, std::vector<double>& out) {
-  double* dout = f.dsmall;
-  SG_CUDA(col_dots(a, b, f.n, f.ld, q, f.partial, dout, f.st));
   out.resize((size_t)q);
+  double* dout = dots_out(f, out.size());
+  SG_CUDA(col_dots(a, b, f.n, f.ld, q, f.partial, dout, f.st));
+  if (dout != f.dsmall) {
+    SG_CUDA(cudaStreamSynchronize(f.st));
+    std::copy(dout, dout + out.size(), out.begin());
+    return Status();
+  }
   return read_back(f.h, out.data(), dout, out.size() * 8, f.st);
 }
 

@@ -480,7 +480,7 @@ static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
 }
 
 Status read_back(saige_grm* h, void* dst, const void* dev, size_t bytes, cudaStream_t st) {
-  void* p = bytes <= kPinBytes ? h->pin.get() : nullptr;
+  void* p = bytes <= kPinReads ? h->pin.get() : nullptr;
   SG_CUDA(cudaMemcpyAsync(p ? p : dst, dev, bytes, cudaMemcpyDeviceToHost, st));
   SG_CUDA(cudaStreamSynchronize(st));
   if (p) memcpy(dst, p, bytes);
@@ -545,10 +545,13 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   bool extra_done = ne == 0;
   // The columns' state after each iteration, and the error word of its product, are read
   // together: one wait per iteration (a wait after the product, and both reads into pageable
-  // memory, left the device idle for about a fifth of a refit of 9,001 samples).
+  // memory, left the device idle for about a fifth of a refit of 9,001 samples).  Where an
+  // iteration is one launch, that launch writes the state where the host reads it.
   const size_t per = 16, cols_bytes = per * (size_t)(q + ne);
   std::vector<char> pageable;
-  char* landing = cols_bytes + 8 <= kPinBytes ? static_cast<char*>(h->pin.get()) : nullptr;
+  char* landing =
+      cols_bytes + 8 <= kPinBytes - kPinReads ? static_cast<char*>(h->pin.get()) : nullptr;
+  if (landing) landing += kPinReads;
   unsigned int* later = landing ? reinterpret_cast<unsigned int*>(landing + cols_bytes) : nullptr;
   if (later) *later = 0u;
   if (!landing) {
@@ -558,8 +561,13 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   const double* h_rr = reinterpret_cast<const double*>(landing);
   const int32_t* h_state = reinterpret_cast<const int32_t*>(h_rr + q + ne);
   const int32_t* h_iters = h_state + q + ne;
+  const bool written = later && one_launch_columns(n);
+  const PcgSeen seen = written ? PcgSeen{const_cast<double*>(h_rr), const_cast<int32_t*>(h_state),
+                                         const_cast<int32_t*>(h_iters)}
+                               : PcgSeen();
   auto read_cols = [&]() -> Status {
-    SG_CUDA(cudaMemcpyAsync(landing, s.cols.rr, cols_bytes, cudaMemcpyDeviceToHost, st));
+    if (!written)
+      SG_CUDA(cudaMemcpyAsync(landing, s.cols.rr, cols_bytes, cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
     if (later) SG_TRY(grm_product_check(h, *later, st));
     std::copy(h_state, h_state + q, state.begin());
@@ -594,7 +602,7 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   }
   run.kx_valid = run.kx && !no_k && (!run.x0 || !run.ax0 || run.kx0);
   SG_CUDA(pcg_start(run.b, run.x0, ax0, run.d, run.x, s.r, s.z, s.p, n, ld, q, run.tol,
-                    run.force_step && run.x0 != nullptr, s.cols, s.partial, s.small, st));
+                    run.force_step && run.x0 != nullptr, s.cols, s.partial, s.small, st, seen));
   if (run.max_iter <= 0) {
     // the loop body never runs; converged is the initial test
     SG_TRY(read_cols());
@@ -635,7 +643,7 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
       }
       SG_CUDA(pcg_iteration(run.x, s.r, s.z, s.p, s.kp, s.ap, run.w_inverse, run.wv, run.tau0,
                             run.tau1, run.d, n, ld, q, run.max_iter, s.cols, s.partial, s.small,
-                            st, run.kx_valid ? run.kx : nullptr));
+                            st, run.kx_valid ? run.kx : nullptr, seen));
     }
   }
   run.iters.assign(h_iters, h_iters + q);

@@ -51,7 +51,8 @@ void release_cached_blocks();
 // A page-locked block of kPinBytes that a handle's small device-to-host reads land in: a read
 // into pageable memory goes through the driver's own staging and waits for itself.  Blocks
 // come from a free list of at most kPinKept, which release_cached_blocks() empties.
-constexpr size_t kPinBytes = (size_t)1 << 18;
+// The first kPinReads bytes are read_back's, the rest a solve's.
+constexpr size_t kPinBytes = (size_t)1 << 18, kPinReads = (size_t)1 << 17;
 constexpr size_t kPinKept = 16;
 struct PinBuf {
   void* ptr = nullptr;

@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(kT)
     pcg_iteration_kernel(double* __restrict__ x, double* __restrict__ r, double* __restrict__ p,
                          const double* __restrict__ kp, const double* __restrict__ wv,
                          double tau0, double tau1, const double* __restrict__ d, int64_t n,
-                         int64_t ld, int max_iter, PcgCols cols, double* __restrict__ kx) {
+                         int64_t ld, int max_iter, PcgCols cols, double* __restrict__ kx,
+                         const PcgSeen seen) {
   extern __shared__ double az[];  // the row block's a = (Sigma p), then z
   __shared__ double sh[2 * 9], part[3];
   const int c = blockIdx.y;
@@ -418,7 +419,10 @@ __global__ void __launch_bounds__(kT)
   column_sums(pap, sh, part);
   if (fabs(pap[0]) < 1e-30) {  // decomposition.rs:257-264
     column_barrier();  // every block has read the partial sums and the column's state
-    if (blockIdx.x == 0 && threadIdx.x == 0) cols.state[c] = kColStopped;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      cols.state[c] = kColStopped;
+      if (seen.state) seen.state[c] = kColStopped;
+    }
     return;
   }
   const double rz = cols.rz[c], alpha = rz / pap[0];
@@ -486,6 +490,11 @@ __global__ void __launch_bounds__(kT)
     cols.rr[c] = sums[1];
     cols.iters[c] = it;
     cols.state[c] = next;
+    if (seen.state) {
+      seen.rr[c] = sums[1];
+      seen.iters[c] = it;
+      seen.state[c] = next;
+    }
   }
 }
 
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(kT)
                             const double* __restrict__ ax0, const double* __restrict__ d,
                             double* __restrict__ x, double* __restrict__ r,
                             double* __restrict__ p, int64_t n, int64_t ld, double tol,
-                            int force_step, PcgCols cols) {
+                            int force_step, PcgCols cols, const PcgSeen seen) {
   __shared__ double sh[3 * 9], part[3];
   const int c = blockIdx.y;
   const int64_t off = (int64_t)c * ld;
@@ -529,8 +538,14 @@ __global__ void __launch_bounds__(kT)
   }
   column_sums(sums, sh, part);
   column_barrier();  // the partial sums are read
-  if (blockIdx.x == 0 && threadIdx.x == 0)
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     pcg_first_state(c, sums[0], sums[1], sums[2], tol, force_step, cols);
+    if (seen.state) {
+      seen.rr[c] = sums[1];
+      seen.iters[c] = 0;
+      seen.state[c] = cols.state[c];
+    }
+  }
 }
 
 // out[column or pair] in one launch: col_dots_kernel or cross_dots_kernel and reduce_partials.
@@ -753,6 +768,8 @@ inline unsigned g1(int64_t n) { return (unsigned)ceil_div(n, kT); }
 
 }  // namespace
 
+bool one_launch_columns(int64_t n) { return red_blocks(n) <= kClusterRows; }
+
 int red_blocks(int64_t n) {
   int64_t b = ceil_div(n, 4096);
   if (b < 1) b = 1;
@@ -807,11 +824,11 @@ cudaError_t cross_dots(const double* a, int p, const double* b, int q, const dou
 cudaError_t pcg_start(const double* b, const double* x0, const double* ax0, const double* d,
                       double* x, double* r, double* z, double* p, int64_t n, int64_t ld, int q,
                       double tol, bool force_step, PcgCols cols, double* partial,
-                      double* scratch4q, cudaStream_t st) {
+                      double* scratch4q, cudaStream_t st, PcgSeen seen) {
   const int nb = red_blocks(n);
   if (nb <= kClusterRows) {
     return launch_columns(pcg_start_column_kernel, nb, q, 0, st, b, x0, ax0, d, x, r, p, n, ld, tol,
-                          force_step ? 1 : 0, cols);
+                          force_step ? 1 : 0, cols, seen);
   }
   pcg_start_kernel<<<dim3(nb, q), kT, 0, st>>>(b, x0, ax0, d, x, r, z, p, n, ld, partial);
   reduce_partials<<<(unsigned)ceil_div(3 * q, 8), 256, 0, st>>>(partial, nb, 3 * q, scratch4q);
@@ -846,13 +863,13 @@ cudaError_t pcg_iteration(double* x, double* r, double* z, double* p, const doub
                           bool w_inverse, const double* wv, double tau0, double tau1,
                           const double* d, int64_t n, int64_t ld, int q, int max_iter,
                           PcgCols cols, double* partial, double* scratch4q, cudaStream_t st,
-                          double* kx) {
+                          double* kx, PcgSeen seen) {
   const int nb = red_blocks(n);
   if (nb <= kClusterRows) {
     auto k = w_inverse ? pcg_iteration_kernel<true> : pcg_iteration_kernel<false>;
     const size_t smem = (size_t)ceil_div(n, nb) * sizeof(double);  // at most 32 KB
     return launch_columns(k, nb, q, smem, st, x, r, p, kp, wv, tau0, tau1, d, n, ld, max_iter, cols,
-                          kx);
+                          kx, seen);
   }
   cudaError_t e =
       w_inverse ? pcg_apply(p, kp, wv, tau0, tau1, ap, n, ld, q, cols, partial, st)

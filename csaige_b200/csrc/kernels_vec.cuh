@@ -19,6 +19,15 @@ struct PcgCols {
 
 // Number of partial-sum blocks used by the reductions below.
 int red_blocks(int64_t n);
+// Whether columns of n rows are a cluster's work (see kernels_vec.cu): dot products are then one
+// launch, whose out may be page-locked host memory, and a PCG iteration too, which writes the
+// columns' rr, state and iteration counts to `seen` (page-locked, or all NULL) as well.
+bool one_launch_columns(int64_t n);
+struct PcgSeen {
+  double* rr;
+  int32_t* state;
+  int32_t* iters;
+};
 
 // out[c] = sum_i a[i,c] * b[i,c] for c < q (two-stage, fixed order).
 // partial must hold red_blocks(n) * q doubles.
@@ -37,7 +46,7 @@ cudaError_t cross_dots(const double* a, int p, const double* b, int q, const dou
 cudaError_t pcg_start(const double* b, const double* x0, const double* ax0, const double* d,
                       double* x, double* r, double* z, double* p, int64_t n, int64_t ld, int q,
                       double tol, bool force_step, PcgCols cols, double* partial,
-                      double* scratch4q, cudaStream_t st);
+                      double* scratch4q, cudaStream_t st, PcgSeen seen = PcgSeen());
 // ap = tau0 p / wmax + tau1 kp, and the partial sums of p'ap, which pcg_step takes from
 // partial.
 cudaError_t pcg_apply(const double* p, const double* kp, const double* wmax, double tau0,
@@ -61,7 +70,7 @@ cudaError_t pcg_iteration(double* x, double* r, double* z, double* p, const doub
                           bool w_inverse, const double* wv, double tau0, double tau1,
                           const double* d, int64_t n, int64_t ld, int q, int max_iter,
                           PcgCols cols, double* partial, double* scratch4q, cudaStream_t st,
-                          double* kx = nullptr);
+                          double* kx = nullptr, PcgSeen seen = PcgSeen());
 
 // Elementwise helpers for the AI-REML loop.
 // Jacobi diagonal of fit-null: wmax = max(w,1e-30), d = tau0/wmax + tau1 (1 when |d| <= 1e-30);
