@@ -383,9 +383,17 @@ bool galerkin_coeffs(const std::vector<double>& gall, int mb, int q, std::vector
 // cannot be factorised (no start).
 Status galerkin_start(Fit& f, Recycle& rc, int mb, int q, bool& ok) {
   const int64_t ld = f.ld;
-  SG_CUDA(gram(rc.v, mb, rc.av, mb + q, f.n, ld, rc.gpart, rc.gout, f.st));
   std::vector<double> gall((size_t)mb * (mb + q)), gam;
-  SG_TRY(read_back(f.h, gall.data(), rc.gout, gall.size() * 8, f.st));
+  // the Gram block's last kernel writes it where the host reads it, when it fits there
+  double* landing =
+      gall.size() * 8 <= kPinReads ? static_cast<double*>(f.h->pin.get()) : nullptr;
+  SG_CUDA(gram(rc.v, mb, rc.av, mb + q, f.n, ld, rc.gpart, landing ? landing : rc.gout, f.st));
+  if (landing) {
+    SG_CUDA(cudaStreamSynchronize(f.st));
+    std::copy(landing, landing + gall.size(), gall.begin());
+  } else {
+    SG_TRY(read_back(f.h, gall.data(), rc.gout, gall.size() * 8, f.st));
+  }
   ok = galerkin_coeffs(gall, mb, q, gam);
   if (!ok) {
     ++rc.fallbacks;
