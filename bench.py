@@ -186,8 +186,8 @@ class ClockSampler:
 
 def single_column_modes(grm, n: int, reps: int = 4) -> dict:
     """Device ms per one-column product on the bench's handle (after its timed fits) with
-    the dense missing-flag sums (SAIGE_SR_LISTS=0) and with the missing-call lists the
-    handle built in its second warm-up fit: the same products to the bit."""
+    the dense missing-flag sums (SAIGE_SR_LISTS=0) and by the library's own rule (the
+    missing-call lists, where they are the cheaper): the same products to the bit."""
     import numpy as np
 
     v = np.random.default_rng(3).standard_normal((1, n))
@@ -709,7 +709,7 @@ def run_ours(args, world, rank, local):
     tot_ms, nl = passes[dom]
     avg_s = (tot_ms / max(nl, 1)) * 1e-3
     m_grm = grm.n_markers
-    # right-hand sides per tensor-core launch (single columns run on the CUDA cores)
+    # right-hand sides per block launch (single columns have kernels of their own)
     cols = (st["n_kv"] - st["sc_launches"]) / max(st["tc_pass_a_launches"], 1)
     bytes_launch = m_grm * ((n + 3) // 4)                # packed genotypes read once per pass
     flops_launch = 2.0 * n * m_grm * cols                 # one GEMM of an N x M by M x r product
@@ -732,11 +732,11 @@ def run_ours(args, world, rank, local):
     roof["avg_launch_ms"] = avg_s * 1e3
     roof["share_of_step"] = (st["tc_pass_a_ms"] + st["tc_pass_b_ms"]) / 1e3 / (step_s * args.steps)
     if st["sc_launches"]:
-        # one-column products (dp4a on the CUDA cores): both passes read the codes once
+        # one-column products: both passes read the codes once
         sc_avg = st["sc_ms"] / st["sc_launches"] * 1e-3
         listed = st["missing_listed"]
         roof["single_column"] = {
-            "kernels": ("sr_pass_a_kernel + sr_pass_b_kernel (+ quantisation)"
+            "kernels": ("sr_pass_kernel, passes A and B (+ quantisation)"
                         + (", summing over the missing-call lists" if st["sc_list_launches"]
                            else "")),
             "missing_lists": {"products": st["sc_list_launches"], "calls": listed,

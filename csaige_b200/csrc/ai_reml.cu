@@ -453,8 +453,8 @@ Status block_solve_recycled(Fit& f, Recycle& rc, const double* x0_prev, const do
   // in the first product of this solve, for this iteration's AI starts
   Extra ex;
   if (!rc.learned && tau[1] != 0.0) {
-    // (measured: leaving them out to keep this product at kTcFastCols columns cost the
-    // AI solve one more product than the slower launch shape costs)
+    // (measured: leaving them out to keep this product at 42 columns cost the AI solve one
+    // more product, which is more than the 43rd column costs)
     const bool need_pk = f.have_prev_pk && !rc.have_kpk;
     const bool need_pw = rc.with_pw && f.have_prev_pw && !rc.have_kpw;
     if (need_pk && need_pw) ex = Extra{f.pk_raw, rc.kpk, 2};  // adjacent columns

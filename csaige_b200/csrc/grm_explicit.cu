@@ -66,8 +66,7 @@ struct SyrkArgs {
   const double* z = nullptr;       // f64 z rows (m_pad x ldz), zero padded
   int64_t ldz = 0;
   int64_t n = 0, m_pad = 0;        // samples; markers (a multiple of kKc, padding z = 0)
-  const SyrkItem* items = nullptr;  // bi <= bj
-  double* carry = nullptr;          // slots of kT x kT accumulators
+  const int2* tiles = nullptr;     // (bi, bj), bi <= bj
   double scale = 0.0;              // 1 / n_used (0 when no marker is used)
   double* dense = nullptr;         // n x n
   int32_t* rows = nullptr;         // sparse triplets
@@ -76,6 +75,9 @@ struct SyrkArgs {
   unsigned long long* count = nullptr;
   int64_t cap = 0;
   double cutoff = 0.0;
+  // plans with shared tiles: items in place of tiles
+  const SyrkItem* items = nullptr;
+  double* carry = nullptr;         // slots of kT x kT accumulators
 };
 
 // Bit offset of entry e (0..15) of a packed word: e = 4j + i sits at
@@ -85,7 +87,9 @@ __device__ __forceinline__ int code_shift(int e) {
   return 16 * (j >> 1) + 2 * (j & 1) + 4 * i;
 }
 
-template <bool kPacked, bool kFma, bool kSparse>
+// kCarry: items of shared tiles may be among the block's.  (That code costs every tile 3 %, 6 %
+// with the marker loop unrolled by two; plans without shared tiles run without it.)
+template <bool kPacked, bool kFma, bool kSparse, bool kCarry>
 __global__ void __launch_bounds__(kThr, 1) grm_syrk_kernel(const SyrkArgs a) {
   // Two stages in flight: while the threads multiply stage c out of zs[c & 1], each
   // k-step also decodes 1/32 of stage c + 1 into zs[(c + 1) & 1], from the packed
@@ -99,10 +103,17 @@ __global__ void __launch_bounds__(kThr, 1) grm_syrk_kernel(const SyrkArgs a) {
   constexpr int kZ = 2 * kKc * kT;         // doubles per z buffer
   constexpr int kRaw = 2 * kKc * kWordsSide;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const SyrkItem item = a.items[blockIdx.x];
-  const int64_t i0 = (int64_t)item.bi * kT, j0 = (int64_t)item.bj * kT;
-  const int nch = item.c1 - item.c0;
-  const int64_t k0 = (int64_t)item.c0 * kKc;  // stages count from the item's first
+  SyrkItem item{};
+  if constexpr (kCarry) item = a.items[blockIdx.x];
+  int2 tile;
+  if constexpr (kCarry)
+    tile = make_int2(item.bi, item.bj);
+  else
+    tile = a.tiles[blockIdx.x];
+  const int64_t i0 = (int64_t)tile.x * kT, j0 = (int64_t)tile.y * kT;
+  // stages count from the item's first
+  const int nch = kCarry ? item.c1 - item.c0 : (int)(a.m_pad / kKc);
+  const int64_t k0 = kCarry ? (int64_t)item.c0 * kKc : 0;
 
   uint32_t wreg0 = 0, wreg1 = 0;
   double lreg = 0.0;
@@ -150,7 +161,7 @@ __global__ void __launch_bounds__(kThr, 1) grm_syrk_kernel(const SyrkArgs a) {
 #pragma unroll
   for (int r = 0; r < 8; ++r)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[r][q] = item.c0 > 0 ? carry[(r * 8 + q) * kThr] : 0.0;
+    for (int q = 0; q < 8; ++q) acc[r][q] = kCarry && item.c0 > 0 ? carry[(r * 8 + q) * kThr] : 0.0;
 
   // prologue: stage 0 decoded, the words of stage 1 in shared memory
   fetch(0);
@@ -167,7 +178,9 @@ __global__ void __launch_bounds__(kThr, 1) grm_syrk_kernel(const SyrkArgs a) {
     if (c + 2 < nch) fetch(c + 2);
     const double* zi = zs + (c & 1) * kZ + ty;
     const double* zj = zs + (c & 1) * kZ + kKc * kT + tx;
-#pragma unroll 8
+    // (n = 12,001, m = 3,000: 27.6 ms by two, 18.3 ms with FMA by four, 19.4 by two)
+    constexpr int kUnroll = kCarry ? 8 : (kFma ? 4 : 2);
+#pragma unroll kUnroll
     for (int k = 0; k < kKc; ++k) {
       double x[8], y[8];
 #pragma unroll
@@ -190,14 +203,14 @@ __global__ void __launch_bounds__(kThr, 1) grm_syrk_kernel(const SyrkArgs a) {
     __syncthreads();
   }
 
-  if (item.c1 < (int)(a.m_pad / kKc)) {
+  if (kCarry && item.c1 < (int)(a.m_pad / kKc)) {
 #pragma unroll
     for (int r = 0; r < 8; ++r)
 #pragma unroll
       for (int q = 0; q < 8; ++q) carry[(r * 8 + q) * kThr] = acc[r][q];
     return;
   }
-  const bool diag = item.bi == item.bj;
+  const bool diag = tile.x == tile.y;
   const int lane = tid & 31;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
@@ -256,15 +269,21 @@ __global__ void grm_standardize_kernel(const double* __restrict__ dos, int64_t n
   }
 }
 
-template <bool kPacked, bool kFma, bool kSparse>
-cudaError_t launch_syrk_t(const SyrkArgs& a, int64_t n_items, cudaStream_t st) {
-  auto k = grm_syrk_kernel<kPacked, kFma, kSparse>;
+template <bool kPacked, bool kFma, bool kSparse, bool kCarry>
+cudaError_t launch_one(const SyrkArgs& a, int64_t n_items, cudaStream_t st) {
+  auto k = grm_syrk_kernel<kPacked, kFma, kSparse, kCarry>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSmemBytes);
   if (e != cudaSuccess) return e;
   k<<<(unsigned)n_items, kThr, kSmemBytes, st>>>(a);
   count_launches(1);
   return cudaGetLastError();
+}
+
+template <bool kPacked, bool kFma, bool kSparse>
+cudaError_t launch_syrk_t(const SyrkArgs& a, int64_t n_items, cudaStream_t st) {
+  return a.carry ? launch_one<kPacked, kFma, kSparse, true>(a, n_items, st)
+                 : launch_one<kPacked, kFma, kSparse, false>(a, n_items, st);
 }
 
 cudaError_t launch_syrk(const SyrkArgs& a, bool packed, bool fma, bool sparse, int64_t n_items,
@@ -301,7 +320,7 @@ struct Events {
 // its stages can be shared by two launches.  With w whole waves of tiles and a rest, the second
 // launch takes the last 1 - 1/k of one tile per SM, and the first, after all other tiles, these
 // tiles' first 1/k in the time that w waves leave: w + 1 - 1/k waves in place of w + 1.
-// n = 4,001, m = 6,007 (528 tiles on 148 SMs): 4 waves in 7.10 ms, 3 2/3 in 6.68.
+// n = 4,001, m = 6,007 (528 tiles on 148 SMs): 4 waves in 7.15 ms, 3 2/3 in 6.71.
 struct SyrkPlan {
   std::vector<SyrkItem> items;  // the first launch's, then one per slot
   int64_t first = 0, slots = 0;
@@ -311,7 +330,8 @@ SyrkPlan syrk_plan(int64_t nb, int64_t nch, int sms) {
   const int64_t tiles = nb * (nb + 1) / 2, w = tiles / sms, rest = tiles % sms;
   // (sms - rest): the SMs that the last of w + 1 waves would leave idle
   int64_t k = w >= 1 && rest > 0 ? ceil_div((int64_t)sms, sms - rest) : 0;
-  if (k > 10 || nch < 4 * k) k = 0;  // one launch
+  // one launch where two would save less than a twentieth of the waves
+  if (nch < 4 * k || k * (w + 1) > 20) k = 0;
   const int64_t whole = k ? tiles - sms : tiles;
   const int c = k ? (int)(nch / k) : 0;
   std::vector<SyrkItem> head, tail;
@@ -343,11 +363,20 @@ Status run_syrk(SyrkArgs a, int64_t n, int64_t n_pad, bool packed, int32_t arith
   SG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const SyrkPlan plan = syrk_plan(nb, a.m_pad / kKc, sms);
   DevBuf d_items, d_carry;
-  SG_TRY(d_items.reserve(plan.items.size() * sizeof(SyrkItem)));
-  SG_CUDA(cudaMemcpyAsync(d_items.ptr, plan.items.data(), plan.items.size() * sizeof(SyrkItem),
-                          cudaMemcpyHostToDevice, st));
-  if (plan.slots > 0) SG_TRY(d_carry.reserve((size_t)plan.slots * kT * kT * sizeof(double)));
-  a.carry = d_carry.as<double>();
+  std::vector<int2> tiles;
+  if (plan.slots > 0) {
+    SG_TRY(d_items.reserve(plan.items.size() * sizeof(SyrkItem)));
+    SG_CUDA(cudaMemcpyAsync(d_items.ptr, plan.items.data(), plan.items.size() * sizeof(SyrkItem),
+                            cudaMemcpyHostToDevice, st));
+    SG_TRY(d_carry.reserve((size_t)plan.slots * kT * kT * sizeof(double)));
+    a.carry = d_carry.as<double>();
+  } else {
+    for (const SyrkItem& t : plan.items) tiles.push_back(make_int2(t.bi, t.bj));
+    SG_TRY(d_items.reserve(tiles.size() * sizeof(int2)));
+    SG_CUDA(cudaMemcpyAsync(d_items.ptr, tiles.data(), tiles.size() * sizeof(int2),
+                            cudaMemcpyHostToDevice, st));
+    a.tiles = d_items.as<int2>();
+  }
   a.n = n;
   a.cutoff = cutoff;
   const bool fma = arith == SAIGE_GRM_ARITH_FMA;

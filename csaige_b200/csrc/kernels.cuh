@@ -9,7 +9,7 @@ namespace saige {
 // For each selected row r: src marker src_rows[r] of the raw .bed (header at
 // bed[0]), samples gathered in sample_idx order (NULL = identity).  When
 // geno_out != NULL the 2-bit codes are written to row r of geno_out (pitch
-// words_per_row 32-bit words; padding samples coded 01 = missing).  counts
+// words_per_row 32-bit words; padding samples coded 11, genotype 0).  counts
 // (2 per row, may be NULL) receive {alt-allele count, missing count}.
 // With the subset's mask, counts alone are formed without the gather.
 struct SubsetMask {

@@ -1895,7 +1895,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
   const char* sc_env = getenv("SAIGE_SC");
   const bool single = cols.size() == 1 && !(sc_env && sc_env[0] == '0');
   if (single) {
-    // one column: both passes on the CUDA cores (same integer sums, same epilogue)
+    // one column: both passes by sr_pass_kernel (same integer sums, same epilogue)
     int8_t* planes_a = p->img_a.as<int8_t>();  // 3 x n_pad limb planes of q
     int8_t* planes_b = p->img_w.as<int8_t>();  // 6 x m_pad limb planes of qw, qc
     double* u = p->u.as<double>();

@@ -372,7 +372,9 @@ typedef struct {
   int32_t converged;
   double log_likelihood;
   int64_t n_kv;            /* GRM products (columns) performed               */
-  int64_t n_kv_launches;   /* GRM product launches (a block counts once)     */
+  int64_t n_kv_launches;   /* GRM product launches (a block counts once; in  */
+                           /* SAIGE_SOLVE_SINGLE each column counts, though  */
+                           /* its right-hand sides are solved side by side)  */
   int64_t pcg_iters;       /* sum over solves of PCG iterations              */
   double seconds;          /* device wall time of the fit                    */
   int32_t learned_trainings; /* SAIGE_WARM_LEARNED: training rounds of the MLP  */
