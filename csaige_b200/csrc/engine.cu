@@ -550,7 +550,7 @@ Status pcg_run(saige_grm* h, PcgRun& run, cudaStream_t st) {
   const size_t per = 16, cols_bytes = per * (size_t)(q + ne);
   std::vector<char> pageable;
   char* landing =
-      cols_bytes + 8 <= kPinBytes - kPinReads ? static_cast<char*>(h->pin.get()) : nullptr;
+      cols_bytes + 8 <= kPinBytes - kPinReads - kPinWord ? static_cast<char*>(h->pin.get()) : nullptr;
   if (landing) landing += kPinReads;
   unsigned int* later = landing ? reinterpret_cast<unsigned int*>(landing + cols_bytes) : nullptr;
   if (later) *later = 0u;

@@ -51,8 +51,9 @@ void release_cached_blocks();
 // A page-locked block of kPinBytes that a handle's small device-to-host reads land in: a read
 // into pageable memory goes through the driver's own staging and waits for itself.  Blocks
 // come from a free list of at most kPinKept, which release_cached_blocks() empties.
-// The first kPinReads bytes are read_back's, the rest a solve's.
-constexpr size_t kPinBytes = (size_t)1 << 18, kPinReads = (size_t)1 << 17;
+// The first kPinReads bytes are read_back's, the last kPinWord a product's error word, the rest a
+// solve's.
+constexpr size_t kPinBytes = (size_t)1 << 18, kPinReads = (size_t)1 << 17, kPinWord = 64;
 constexpr size_t kPinKept = 16;
 struct PinBuf {
   void* ptr = nullptr;
@@ -181,8 +182,8 @@ bool marker_qc_pass(double af, int64_t n_valid, int64_t n, double min_maf, doubl
 
 // Kv for q columns of v (ld = h->n_pad; rows n .. ld - 1 are not read) into kp.
 // active (host, length q, may be NULL) selects columns; others are skipped.
-// With `later` (page-locked), a MIXED product returns without waiting, its error word (0: none)
-// to arrive there in stream order, and the caller passes it to grm_product_check once st has
+// With `later` (page-locked), a MIXED product returns without waiting, its kernels write an error
+// (0: none) there, and the caller passes it to grm_product_check once st has
 // been synchronised; timed and traced products wait all the same.
 Status grm_product(saige_grm* h, const double* v, double* kp, int q, const int32_t* active,
                    int precision, cudaStream_t st, unsigned int* later = nullptr);

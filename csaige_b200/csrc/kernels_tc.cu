@@ -1032,7 +1032,7 @@ struct SrList {
         if (i + j >= hi) break;
         const uint32_t g = x[j] >> bits;
         if (g >= (uint32_t)kRows_ || (int)(x[j] & pmask) >= n) {
-          atomicOr(err, kSrListErr);
+          report_error(err, kSrListErr);
           continue;
         }
         if ((int)g != row) {
@@ -1882,6 +1882,18 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
   SG_TRY(p->scal.reserve(scal_bytes));
   const uint8_t* excl = h->masked ? h->excl.as<uint8_t>() : nullptr;
   Scal sc = carve(p);
+  // The kernels write the error word where the host reads it: `later`, or a word of the handle's
+  // page-locked block (idle here: every product's word is read after a wait), or, without one,
+  // device memory.
+  if (h->profiling || p->tracing) later = nullptr;
+  unsigned int* word = later;
+  if (!word)
+    if (char* pin = static_cast<char*>(h->pin.get()))
+      word = reinterpret_cast<unsigned int*>(pin + kPinBytes - kPinWord);
+  if (word) {
+    *word = 0u;
+    sc.err = word;
+  }
   // per-pass CUDA-event timing when profiling is on (events on the launching stream)
   std::vector<cudaEvent_t> ev;
   auto mark = [&](cudaEvent_t* e) -> Status {
@@ -2093,12 +2105,14 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->n_kv += r;
   }
   h->n_kv_launches += 1;
-  if (later && !h->profiling && !p->tracing) {
-    SG_CUDA(cudaMemcpyAsync(later, sc.err, sizeof(*later), cudaMemcpyDeviceToHost, st));
-    return Status();
-  }
+  if (later) return Status();
   unsigned int err = 0;
-  SG_TRY(read_back(h, &err, sc.err, sizeof(err), st));
+  if (word) {
+    SG_CUDA(cudaStreamSynchronize(st));
+    err = *word;
+  } else {
+    SG_TRY(read_back(h, &err, sc.err, sizeof(err), st));
+  }
   for (auto& pr : ev_a) {
     float ms = 0.f;
     SG_CUDA(cudaEventElapsedTime(&ms, pr.first, pr.second));

@@ -189,7 +189,7 @@ struct LayerArgs {
   float* hbuf;            // optional: unrounded tanh activations, rows x 256 FP32
   float* y;               // output layer: rows outputs
   long long wait_cycles;  // budget of each pipeline wait
-  unsigned int* err;      // bit 0: a wait ran out; bit 1: a drain ran out
+  unsigned int* err;      // 1: a wait ran out; 2: a drain ran out
 };
 
 // Shared memory: W (128 KB) | A ring (3 x 32 KB) | 14 barriers | TMEM address, abort

@@ -11,6 +11,12 @@ namespace tcx {
 // Budget of a drain wait (work this CTA already issued): ~2 s at 1.9 GHz.
 constexpr long long kWaitCycles = 4000000000LL;
 
+// Sets the error word, which may be page-locked host memory (so a plain store; any code but 0
+// says that the launch failed).
+__device__ __forceinline__ void report_error(unsigned int* err, unsigned int code) {
+  *reinterpret_cast<volatile unsigned int*>(err) = code;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -65,7 +71,7 @@ __device__ __forceinline__ bool mbar_wait_impl(uint32_t bar, uint32_t parity,
   if (budget <= 0) {
     if (mbar_test_wait(bar, parity)) return true;
     *abort_flag = 1;
-    atomicOr(err, 1u);
+    report_error(err, 1u);
     return false;
   }
   if (mbar_try_wait(bar, parity)) return true;
@@ -82,7 +88,7 @@ __device__ __forceinline__ bool mbar_wait_impl(uint32_t bar, uint32_t parity,
       if (*abort_flag) return false;
       if (clock64() - t0 > budget) {
         *abort_flag = 1;
-        atomicOr(err, 1u);
+        report_error(err, 1u);
         return false;
       }
     }
@@ -122,7 +128,7 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, u
     if (mbar_try_wait(bar, parity)) return true;
     __nanosleep(128);
     if ((polls & 63u) == 0 && clock64() - t0 > kWaitCycles) {
-      atomicOr(err, 2u);
+      report_error(err, 2u);
       return false;
     }
   }
