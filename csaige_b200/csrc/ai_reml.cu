@@ -249,6 +249,7 @@ struct Recycle {
   double *kblock, *kpk, *kpw;           // K X* of the latest block solve, K of the AI solutions
   double *kin, *kout;                   // [Py | X*_t | pk' | pw' (| learned)] and its K-image
   double *gam, *gpart, *gout;
+  size_t gpart_cap = 0;                 // doubles at gpart
   bool have_kblock = false, have_kpk = false, have_kpw = false;
   bool kv_ok = true;                    // every basis column of the current start has kv
   // K [X | U] was formed (f.kxu).  Without it (the recycled block fit) [X | U] joins a
@@ -315,7 +316,9 @@ Status recycle_init(Fit& f, Recycle& rc, bool learned, const double* diagk, uint
   }
   const size_t mb = (size_t)rc.mb_max, nk = (size_t)rc.nk;
   const size_t ncol = mb + (mb + q) + 3 * q + 2 * nk + mb + q + q + 2 + 2 * (size_t)rc.keep_cap;
-  const size_t nsmall = mb * q + gram_partial_doubles(f.n, (int)mb, (int)(mb + q)) + mb * (mb + q);
+  // (the starts' bases are of any width up to mb)
+  rc.gpart_cap = gram_partial_most(f.n, (int)mb, (int)(mb + q));
+  const size_t nsmall = mb * q + rc.gpart_cap + mb * (mb + q);
   SG_TRY(rc.mem.reserve((ncol * ld + nsmall) * 8));
   double* b = rc.mem.as<double>();
   SG_CUDA(cudaMemsetAsync(b, 0, ncol * ld * 8, f.st));  // padding rows stay zero
@@ -387,7 +390,8 @@ Status galerkin_start(Fit& f, Recycle& rc, int mb, int q, bool& ok) {
   // the Gram block's last kernel writes it where the host reads it, when it fits there
   double* landing =
       gall.size() * 8 <= kPinReads ? static_cast<double*>(f.h->pin.get()) : nullptr;
-  SG_CUDA(gram(rc.v, mb, rc.av, mb + q, f.n, ld, rc.gpart, landing ? landing : rc.gout, f.st));
+  SG_CUDA(gram(rc.v, mb, rc.av, mb + q, f.n, ld, rc.gpart, rc.gpart_cap,
+               landing ? landing : rc.gout, f.st));
   if (landing) {
     SG_CUDA(cudaStreamSynchronize(f.st));
     std::copy(landing, landing + gall.size(), gall.begin());

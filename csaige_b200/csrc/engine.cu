@@ -848,6 +848,18 @@ SG_API int32_t saige_rademacher_probes(uint64_t seed, int32_t n_vec, int64_t n, 
   SG_GUARD_END
 }
 
+SG_API int32_t saige_gram_workspace(int64_t n, int32_t a, int32_t b, int64_t* needed,
+                                    int64_t* reserved) {
+  SG_GUARD_BEGIN
+  set_error("");
+  if (!needed || !reserved || n <= 0 || a <= 0 || b <= 0)
+    return fail(SAIGE_EINVAL, "null argument or empty size").code;
+  *needed = (int64_t)gram_partial_doubles(n, a, b);
+  *reserved = (int64_t)gram_partial_most(n, a, b);
+  return SAIGE_OK;
+  SG_GUARD_END
+}
+
 // fit_null.rs:209-222: the QC a marker passes to enter the GRM or the variance-ratio
 // candidates.
 static bool qc_pass(double af, int64_t n_valid, int64_t n, double min_maf, double max_missing) {

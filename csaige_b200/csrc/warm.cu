@@ -10,10 +10,13 @@ namespace {
 
 constexpr int kG = 32;  // Gram: rows per stage; the chunks of rows are counted in 32 x 32 tiles
 
+// Row chunks: at least 2,048 rows each, and at most kGramBlocks blocks of 32 x 32 tiles.
+constexpr int kGramBlocks = 148 * 4;
+
 int gram_chunks(int64_t n, int a, int b) {
   const int tiles = ((a + kG - 1) / kG) * ((b + kG - 1) / kG);
   const int64_t by_rows = (n + 2047) / 2048;
-  const int64_t want = std::max<int64_t>(1, 148 * 4 / std::max(tiles, 1));
+  const int64_t want = std::max<int64_t>(1, kGramBlocks / std::max(tiles, 1));
   return (int)std::max<int64_t>(1, std::min(by_rows, want));
 }
 
@@ -307,8 +310,16 @@ size_t gram_partial_doubles(int64_t n, int a, int b) {
   return (size_t)gram_chunks(n, a, b) * (size_t)a * (size_t)b;
 }
 
+// A product is cut into more than one chunk only while chunks x tiles <= kGramBlocks, and has at
+// most kG^2 sums per tile: more than one chunk's sums are at most kGramBlocks kG^2 in all.
+size_t gram_partial_most(int64_t n, int a, int b) {
+  const size_t sums = (size_t)a * (size_t)b, by_rows = (size_t)ceil_div(n, (int64_t)2048);
+  return std::min(by_rows * sums, std::max(sums, (size_t)kGramBlocks * kG * kG));
+}
+
 cudaError_t gram(const double* A, int a, const double* B, int b, int64_t n, int64_t ld,
-                 double* partial, double* out, cudaStream_t st) {
+                 double* partial, size_t cap, double* out, cudaStream_t st) {
+  if (gram_partial_doubles(n, a, b) > cap) return cudaErrorInvalidValue;
   const int nch = gram_chunks(n, a, b);
   const int64_t chunk = round_up(ceil_div(n, nch), kG);
   // 32 x 32 tiles while they give every SM two blocks, else 16 x 16

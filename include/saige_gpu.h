@@ -222,6 +222,12 @@ int32_t saige_release_cached_memory(void);
 int32_t saige_rademacher_probes(uint64_t seed, int32_t n_vec, int64_t n, double* out,
                                 int32_t device);
 
+/* No counterpart in the reference.  Workspace of the Gram products A' B (a and b columns of
+ * n rows) behind the recycled starts, in doubles: what one product's partial sums take, and
+ * what is reserved for every product of at most a x b columns (needs no GPU). */
+int32_t saige_gram_workspace(int64_t n, int32_t a, int32_t b, int64_t* needed,
+                             int64_t* reserved);
+
 /* ---------------------------------------------------------------------
  * GRM operator (OnTheFlyGrm, saige-core/src/glmm/pcg.rs:91-180)
  * ------------------------------------------------------------------- */
