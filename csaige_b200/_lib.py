@@ -287,6 +287,10 @@ SIGNATURES = {
     ),
     "saige_rademacher_probes": (C.c_int32, [C.c_uint64, C.c_int32, C.c_int64, _d, C.c_int32]),
     "saige_gram_workspace": (C.c_int32, [C.c_int64, C.c_int32, C.c_int32, _i64, _i64]),
+    "saige_gram_dev": (
+        C.c_int32,
+        [_vp, C.c_int32, _vp, C.c_int32, C.c_int64, C.c_int64, C.c_int32, _vp, C.c_int32],
+    ),
     "saige_grm_matvec_dev_noalloc": (
         C.c_int32,
         [_vp, _vp, _vp, C.c_int64, C.c_int32, _vp],

@@ -860,6 +860,33 @@ SG_API int32_t saige_gram_workspace(int64_t n, int32_t a, int32_t b, int64_t* ne
   SG_GUARD_END
 }
 
+SG_API int32_t saige_gram_dev(const double* a_dev, int32_t a, const double* b_dev, int32_t b,
+                              int64_t n, int64_t ld, int32_t tile, double* out_dev,
+                              int32_t device) {
+  SG_GUARD_BEGIN
+  set_error("");
+  if (!a_dev || !b_dev || !out_dev || a <= 0 || b <= 0 || n <= 0 || ld < n)
+    return fail(SAIGE_EINVAL, "null argument or bad size").code;
+  // the kernel copies two rows of a column at a time
+  if (ld % 2 || (reinterpret_cast<uintptr_t>(a_dev) | reinterpret_cast<uintptr_t>(b_dev)) % 16)
+    return fail(SAIGE_EINVAL, "columns are not 16-byte aligned").code;
+  if (tile != 0 && tile != 16 && tile != 32)
+    return fail(SAIGE_EINVAL, "tile is 0, 16 or 32").code;
+  int dev = 0;
+  Status ps = pick_device(device, &dev);
+  if (!ps.ok()) return ps.code;
+  auto body = [&]() -> Status {
+    DevBuf part;
+    const size_t cap = gram_partial_doubles(n, a, b);
+    SG_TRY(part.reserve(cap * sizeof(double)));
+    SG_CUDA(gram(a_dev, a, b_dev, b, n, ld, part.as<double>(), cap, out_dev, 0, tile));
+    SG_CUDA(cudaStreamSynchronize(0));
+    return Status();
+  };
+  return body().code;
+  SG_GUARD_END
+}
+
 // fit_null.rs:209-222: the QC a marker passes to enter the GRM or the variance-ratio
 // candidates.
 static bool qc_pass(double af, int64_t n_valid, int64_t n, double min_maf, double max_missing) {

@@ -318,13 +318,13 @@ size_t gram_partial_most(int64_t n, int a, int b) {
 }
 
 cudaError_t gram(const double* A, int a, const double* B, int b, int64_t n, int64_t ld,
-                 double* partial, size_t cap, double* out, cudaStream_t st) {
+                 double* partial, size_t cap, double* out, cudaStream_t st, int tile) {
   if (gram_partial_doubles(n, a, b) > cap) return cudaErrorInvalidValue;
   const int nch = gram_chunks(n, a, b);
   const int64_t chunk = round_up(ceil_div(n, nch), kG);
   // 32 x 32 tiles while they give every SM two blocks, else 16 x 16
   const int64_t tiles4 = ceil_div(a, 32) * ceil_div(b, 32);
-  if (tiles4 * nch >= 296)
+  if (tile ? tile == 32 : tiles4 * nch >= 296)
     gram_kernel<4><<<dim3((unsigned)nch, (unsigned)tiles4), 64, 0, st>>>(A, a, B, b, n, ld, chunk,
                                                                           partial);
   else

@@ -15,10 +15,11 @@ namespace saige {
 // result does not depend on scheduling.  partial holds `cap` doubles; a product that needs more
 // (gram_partial_doubles) is refused.  A narrower product can need more than a wider one: fewer
 // tiles are cut into more row chunks.  gram_partial_most bounds all of at most a x b columns.
+// tile: 16 or 32 columns per side of a block's tile (the same bits), 0 for the one that pays.
 size_t gram_partial_doubles(int64_t n, int a, int b);
 size_t gram_partial_most(int64_t n, int a, int b);
 cudaError_t gram(const double* A, int a, const double* B, int b, int64_t n, int64_t ld,
-                 double* partial, size_t cap, double* out, cudaStream_t st);
+                 double* partial, size_t cap, double* out, cudaStream_t st, int tile = 0);
 
 // Y[:, c] (c < q) = sum_{j < m} V[:, j] G[j*q + c]  (+ Y[:, c] when add); G on the device.
 // Y must not overlap V.  Rows n .. ld-1 are not written.

@@ -228,6 +228,13 @@ int32_t saige_rademacher_probes(uint64_t seed, int32_t n_vec, int64_t n, double*
 int32_t saige_gram_workspace(int64_t n, int32_t a, int32_t b, int64_t* needed,
                              int64_t* reserved);
 
+/* One such product: out (a x b, row-major) = A' B, each entry's rows summed in chunks of a
+ * size that depends on n, a and b only.  Device pointers; columns ld apart (even), 16-byte
+ * aligned.  tile: columns per side of a thread block's tile, 16 or 32 (the same bits), or 0 for
+ * the choice that the recycled starts make.  Runs on the legacy stream. */
+int32_t saige_gram_dev(const double* a_dev, int32_t a, const double* b_dev, int32_t b, int64_t n,
+                       int64_t ld, int32_t tile, double* out_dev, int32_t device);
+
 /* ---------------------------------------------------------------------
  * GRM operator (OnTheFlyGrm, saige-core/src/glmm/pcg.rs:91-180)
  * ------------------------------------------------------------------- */
