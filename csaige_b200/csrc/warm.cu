@@ -240,26 +240,71 @@ __global__ void learn_to_cols_kernel(const float* __restrict__ y, int64_t n, int
   out[(int64_t)c * ld + i] = (double)y[(int64_t)c * n + i];
 }
 
-// Sums of z^2 over a range of markers, for 16 samples per thread (one packed word per
-// marker): z^2 of the four codes (00 -> 2, 10 -> 1, 11 -> 0, 01 missing -> 0; excluded
-// markers 0) sits in shared memory for kDiagChunk markers at a time, so an entry costs a
-// bit-field extract, one 8-byte lookup (four addresses per marker: no bank conflicts)
-// and one FP64 add.  Block y sums the markers [y per, (y + 1) per) into row y of partial;
-// grm_diag_finish adds the rows in order.  Bound: the lookups.  One thread per sample over
-// all markers (a 4-byte load per 2-bit code, one serial chain) took 22.9 ms at n = 60,013,
-// m = 39,000; this takes 0.60 ms.
+// The live rows of a handle, in order: those with a standardised column (1/s != 0) that the
+// mask does not leave out.  Block b's count of kLiveRows rows, then, from the counts, their
+// list and how many there are.
+constexpr int kLiveRows = 1024;
+
+__device__ __forceinline__ bool live_row(const double* inv_s, const uint8_t* excl, int64_t j,
+                                         int64_t m) {
+  return j < m && inv_s[j] != 0.0 && !(excl && excl[j]);
+}
+
+__global__ void __launch_bounds__(kLiveRows)
+    live_count_kernel(const double* __restrict__ inv_s, const uint8_t* __restrict__ excl,
+                      int64_t m, int32_t* __restrict__ counts) {
+  const int c = __syncthreads_count(
+      live_row(inv_s, excl, (int64_t)blockIdx.x * kLiveRows + threadIdx.x, m));
+  if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+
+__global__ void __launch_bounds__(kLiveRows)
+    live_list_kernel(const double* __restrict__ inv_s, const uint8_t* __restrict__ excl,
+                     int64_t m, const int32_t* __restrict__ counts, int32_t* __restrict__ rows,
+                     int32_t* __restrict__ n_live) {
+  __shared__ int before[kLiveRows / 32], in_warp[kLiveRows / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int s = 0;  // rows in the blocks before
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += kLiveRows) s += counts[k];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const int64_t j = (int64_t)blockIdx.x * kLiveRows + threadIdx.x;
+  const bool live = live_row(inv_s, excl, j, m);
+  const unsigned int votes = __ballot_sync(0xffffffffu, live);
+  if (lane == 0) {
+    before[warp] = s;
+    in_warp[warp] = __popc(votes);
+  }
+  __syncthreads();
+  int at = 0;
+  for (int k = 0; k < kLiveRows / 32; ++k) at += before[k] + (k < warp ? in_warp[k] : 0);
+  at += __popc(votes & ((1u << lane) - 1u));
+  if (live) rows[at] = (int32_t)j;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kLiveRows - 1) *n_live = at + (live ? 1 : 0);
+}
+
+// Sums of z^2 over a range of the live rows, for 16 samples per thread (one packed word per
+// row): z^2 of the four codes (00 -> 2, 10 -> 1, 11 -> 0, 01 missing -> 0) sits in shared
+// memory for kDiagChunk rows at a time, so an entry costs a
+// bit-field extract, one 8-byte lookup (four addresses per row: no bank conflicts)
+// and one FP64 add.  Block y sums the live rows [y per, (y + 1) per) into row y of partial;
+// grm_diag_finish adds the rows in order.  The ranges count live rows, so that a handle with
+// markers left out forms the sums of a handle without them, to the bit.  Bound: the lookups.
+// One thread per sample over all markers (a 4-byte load per 2-bit code, one serial chain) took
+// 22.9 ms at n = 60,013, m = 39,000; this takes 0.62 ms (0.64 with the 51 registers that the
+// compiler takes for five blocks per SM), and the list 5 us.
 constexpr int kDiagThreads = 256;
 constexpr int kDiagChunk = 64;
 
-__global__ void __launch_bounds__(kDiagThreads)
+__global__ void __launch_bounds__(kDiagThreads, 4)
     grm_diag_kernel(const uint32_t* __restrict__ geno, int64_t wpr,
                     const double* __restrict__ two_p, const double* __restrict__ inv_s,
-                    const uint8_t* __restrict__ excl, int64_t m, int64_t per,
-                    double* __restrict__ partial) {
+                    const int32_t* __restrict__ rows, const int32_t* __restrict__ n_live,
+                    int64_t per, double* __restrict__ partial) {
   __shared__ double tab[kDiagChunk][4];
+  __shared__ int64_t at[kDiagChunk];  // the rows' first words
   const int64_t w = (int64_t)blockIdx.x * kDiagThreads + threadIdx.x;
   const int64_t lo = (int64_t)blockIdx.y * per;
-  const int64_t hi = lo + per < m ? lo + per : m;
+  const int64_t n_rows = *n_live, hi = lo + per < n_rows ? lo + per : n_rows;
   double acc[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = 0.0;
@@ -269,23 +314,33 @@ __global__ void __launch_bounds__(kDiagThreads)
     {
       const int mk = threadIdx.x >> 2, code = threadIdx.x & 3;
       double z = 0.0;
-      if (mk < cnt && code != 1 && !(excl && excl[c0 + mk])) {
-        const double g = code == 0 ? 2.0 : (code == 2 ? 1.0 : 0.0);
-        z = (g - two_p[c0 + mk]) * inv_s[c0 + mk];
+      if (mk < cnt) {
+        const int32_t j = rows[c0 + mk];
+        if (code != 1) {
+          const double g = code == 0 ? 2.0 : (code == 2 ? 1.0 : 0.0);
+          z = (g - two_p[j]) * inv_s[j];
+        }
+        if (code == 0) at[mk] = j * wpr;
       }
       tab[mk][code] = z * z;
     }
     __syncthreads();
     if (w >= wpr) continue;
-    const uint32_t* p = geno + c0 * wpr + w;
-#pragma unroll 8
-    for (int k = 0; k < cnt; ++k) {
-      const uint32_t x = __ldg(p + (int64_t)k * wpr);
+    auto add = [&](int k, uint32_t x) {
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const int shift = 16 * (e >> 3) + 2 * ((e >> 2) & 1) + 4 * (e & 3);
         acc[e] += tab[k][(x >> shift) & 3u];
       }
+    };
+    // neighbouring rows (most chunks): addresses that do not wait for a lookup (0.78 ms with)
+    const uint32_t* p = geno + at[0] + w;
+    if (at[cnt - 1] - at[0] == (cnt - 1) * wpr) {
+#pragma unroll 8
+      for (int k = 0; k < cnt; ++k) add(k, __ldg(p + (int64_t)k * wpr));
+    } else {
+#pragma unroll 8
+      for (int k = 0; k < cnt; ++k) add(k, __ldg(geno + at[k] + w));
     }
   }
   if (w >= wpr) return;
@@ -393,23 +448,31 @@ Status grm_diag(saige_grm* h, double* out, cudaStream_t st) {
   const int64_t m_used = h->masked ? h->m_active : h->m_eff;
   const double scale = m_used > 0 ? 1.0 / (double)m_used : 0.0;
   // about eight blocks per SM over (windows of 4,096 samples) x (marker ranges)
+  // (at most m_used rows are live)
   const int64_t windows = ceil_div(h->wpr, (int64_t)kDiagThreads);
-  const int64_t most = std::max<int64_t>(1, ceil_div(h->m, (int64_t)kDiagChunk));
+  const int64_t most = std::max<int64_t>(1, ceil_div(m_used, (int64_t)kDiagChunk));
   const int64_t want = std::min(most, ceil_div((int64_t)148 * 8, windows));
-  const int64_t per = round_up(ceil_div(std::max<int64_t>(h->m, 1), want), kDiagChunk);
-  const int64_t splits = std::max<int64_t>(1, ceil_div(h->m, per));
-  DevBuf partial;
+  const int64_t per = round_up(ceil_div(std::max<int64_t>(m_used, 1), want), kDiagChunk);
+  const int64_t splits = std::max<int64_t>(1, ceil_div(m_used, per));
+  const int64_t blocks = std::max<int64_t>(1, ceil_div(h->m, (int64_t)kLiveRows));
+  DevBuf partial, list;
   SG_TRY(partial.reserve((size_t)splits * h->n_pad * sizeof(double)));
-  // the partial sums are used on st only
+  SG_TRY(list.reserve((size_t)(h->m + blocks + 1) * sizeof(int32_t)));
+  int32_t *rows = list.as<int32_t>(), *counts = rows + h->m, *n_live = counts + blocks;
+  const uint8_t* excl = h->masked ? h->excl.as<uint8_t>() : nullptr;
+  // the buffers are used on st only
   ReleaseScope rs(ReleaseMode::kStream, st);
+  live_count_kernel<<<(unsigned)blocks, kLiveRows, 0, st>>>(h->inv_s, excl, h->m, counts);
+  live_list_kernel<<<(unsigned)blocks, kLiveRows, 0, st>>>(h->inv_s, excl, h->m, counts, rows,
+                                                           n_live);
   grm_diag_kernel<<<dim3((unsigned)windows, (unsigned)splits), kDiagThreads, 0, st>>>(
-      h->geno, h->wpr, h->two_p, h->inv_s, h->masked ? h->excl.as<uint8_t>() : nullptr, h->m, per,
-      partial.as<double>());
+      h->geno, h->wpr, h->two_p, h->inv_s, rows, n_live, per, partial.as<double>());
   grm_diag_finish<<<(unsigned)ceil_div(h->n, 256), 256, 0, st>>>(
       partial.as<double>(), (int)splits, h->n_pad, h->n, scale, out);
-  count_launches(2);
+  count_launches(4);
   SG_CHECK_LAUNCH();
   partial.release();
+  list.release();
   return Status();
 }
 
