@@ -233,6 +233,7 @@ SIGNATURES = {
     "saige_tc_set_wait_budget": (C.c_int32, [C.c_int64]),
     "saige_grm_noalloc_scratch_bytes": (C.c_int32, [_vp, P(_sz), P(_sz)]),
     "saige_release_cached_memory": (C.c_int32, []),
+    "saige_pinned_blocks": (C.c_int32, [_i32, _i32]),
     "saige_write_null_model": (C.c_int32, [C.c_char_p, P(NullModelC)]),
     "saige_xvx_inv_xv": (C.c_int32, [_d, _d, C.c_int64, C.c_int32, _d]),
     "saige_fit_null_cohorts": (

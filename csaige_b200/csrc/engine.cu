@@ -828,6 +828,16 @@ SG_API int32_t saige_release_cached_memory(void) {
   SG_GUARD_END
 }
 
+SG_API int32_t saige_pinned_blocks(int32_t* kept, int32_t* most) {
+  SG_GUARD_BEGIN
+  if (!kept || !most) return fail(SAIGE_EINVAL, "null argument").code;
+  std::lock_guard<std::mutex> lk(g_pin_mu);
+  *kept = (int32_t)g_pins.size();
+  *most = (int32_t)kPinKept;
+  return SAIGE_OK;
+  SG_GUARD_END
+}
+
 SG_API int32_t saige_rademacher_probes(uint64_t seed, int32_t n_vec, int64_t n, double* out,
                                       int32_t device) {
   SG_GUARD_BEGIN

@@ -50,11 +50,14 @@ void release_cached_blocks();
 
 // A page-locked block of kPinBytes that a handle's small device-to-host reads land in: a read
 // into pageable memory goes through the driver's own staging and waits for itself.  Blocks
-// come from a free list of at most kPinKept, which release_cached_blocks() empties.
+// come from a free list, which release_cached_blocks() empties.  It keeps as many as were in use
+// at once, up to kPinKept (64 MB; the sub-cohort call has a fit in flight for every second
+// hardware thread): a block beyond that goes back to the driver, which waits for the device, and
+// so for every other fit in flight.
 // The first kPinReads bytes are read_back's, the last kPinWord a product's error word, the rest a
 // solve's.
 constexpr size_t kPinBytes = (size_t)1 << 18, kPinReads = (size_t)1 << 17, kPinWord = 64;
-constexpr size_t kPinKept = 16;
+constexpr size_t kPinKept = 256;
 struct PinBuf {
   void* ptr = nullptr;
   bool tried = false;

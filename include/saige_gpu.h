@@ -215,6 +215,11 @@ int32_t saige_xvx_inv_xv(const double* x, const double* w, int64_t n, int32_t p,
  * fail. */
 int32_t saige_release_cached_memory(void);
 
+/* Page-locked host blocks (256 KB each) that closed handles have left for the next ones, and
+ * how many may be kept: as many as were in use at once, up to `most`.
+ * saige_release_cached_memory frees them. */
+int32_t saige_pinned_blocks(int32_t* kept, int32_t* most);
+
 /* The Rademacher probe vectors of fit_ai_reml (saige-core/src/glmm/ai_reml.rs:121-130):
  * ChaCha8Rng::seed_from_u64(seed), n_vec vectors of n entries drawn in order with
  * gen::<bool>() -> +1 / -1.  Generated on `device` (the stream is counter based)
