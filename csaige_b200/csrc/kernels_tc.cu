@@ -1462,7 +1462,7 @@ TcWork tc_work(int64_t tiles, int64_t nk, int sms) {
 
 struct TcPlan {
   DevBuf tiles_m, tiles_s, img_a, img_w, img_c, u, scal, trace;
-  DevBuf part;  // sums of the tiles that CTAs share, and their counts: zero between launches
+  DevBuf part;  // counts and sums of the tiles that CTAs share: zero between launches
   int sms = 0;
   int64_t s_ld = 0;  // tiles_s: marker tiles per sample tile (>= m_pad / 128)
   bool tracing = false;
@@ -1470,6 +1470,9 @@ struct TcPlan {
   DevBuf sr_q32;   // with them: the quantised v (n_pad) and c (m_pad) as int32
   DevBuf sr_sums;  // the divided passes' sums and tickets: zero between launches
 };
+
+// Bytes of the counts of the tiles that CTAs share.
+static size_t part_counts(const TcPlan* p) { return (size_t)round_up((int64_t)p->sms * 4, 256); }
 
 // The missing-call lists cost about two products' time to build (four passes over the
 // codes) and 8 bytes per missing call, while a fit runs four or five one-column products:
@@ -1830,18 +1833,26 @@ void tc_set_wait_budget(long long cycles) {
 }
 
 // Sets the work division of a launch over `tiles` tiles; returns its grid.
-static unsigned set_work(TcArgs* a, int64_t tiles, int sms) {
-  const TcWork w = tc_work(tiles, a->nk, sms);
+static unsigned set_work(TcArgs* a, int64_t tiles, const TcPlan* p) {
+  const TcWork w = tc_work(tiles, a->nk, p->sms);
   a->whole = w.whole;
   a->extra = w.extra;
   a->tail_tile = w.tail_tile;
   a->tail_units = w.tail_units;
+  // the counts come first: their place does not depend on the columns
+  a->part_done = p->part.as<unsigned int>();
+  a->part = reinterpret_cast<unsigned long long*>(p->part.as<char>() + part_counts(p));
   return (unsigned)w.grid;
 }
 
-// The sums and counts of tiles that CTAs share: one slot per CTA (see TcWork).
-static size_t part_bytes(const TcPlan* p) {
-  return (size_t)p->sms * (2 * kMaxR * kRows * 8 + 4);
+// Room, all zero, for the sums and counts of tiles that CTAs share when r columns are in a
+// launch: a slot per CTA (see TcWork).
+static Status part_reserve(TcPlan* p, int r, cudaStream_t st) {
+  const size_t want = part_counts(p) + (size_t)p->sms * 2 * r * kRows * 8;
+  if (want <= p->part.bytes) return Status();
+  SG_TRY(p->part.reserve(want));
+  SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, p->part.bytes, st));
+  return Status();
 }
 
 Status tc_product_failed(saige_grm* h, unsigned int err, cudaStream_t st) {
@@ -1849,7 +1860,7 @@ Status tc_product_failed(saige_grm* h, unsigned int err, cudaStream_t st) {
     return fail(SAIGE_ECUDA, "one-column GRM product: a missing-call list entry out of range");
   // shared tiles may be left half summed
   TcPlan* p = h->tc;
-  if (p->part.ptr) SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes(p), st));
+  if (p->part.ptr) SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, p->part.bytes, st));
   SG_CUDA(cudaStreamSynchronize(st));
   return fail(SAIGE_TIMEOUT, "tensor-core GRM product: a pipeline wait timed out");
 }
@@ -2008,12 +2019,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->stats.sc_list_launches += lists ? 1 : 0;
     h->n_kv += 1;
   }
-  // a slot for every tile that CTAs share (at most one per CTA boundary)
-  const size_t part_slots = (size_t)p->sms;
-  if (!single && !p->part.ptr) {
-    SG_TRY(p->part.reserve(part_bytes(p)));
-    SG_CUDA(cudaMemsetAsync(p->part.ptr, 0, part_bytes(p), st));
-  }
+  if (!single) SG_TRY(part_reserve(p, rmax, st));
   for (size_t c0 = 0; c0 < (single ? 0 : cols.size()); c0 += kMaxR) {
     const int r = (int)std::min<size_t>(kMaxR, cols.size() - c0);
     const int ng = (int)round_up(3 * r, 16);
@@ -2048,9 +2054,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_ld = h->m_pad;
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = set_work(&a, h->m_pad / kRows, p->sms);
-      a.part = p->part.as<unsigned long long>();
-      a.part_done = reinterpret_cast<unsigned int*>(a.part + part_slots * 2 * kMaxR * kRows);
+      const unsigned grid = set_work(&a, h->m_pad / kRows, p);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<false>(h->device, grid, a, st));
@@ -2091,9 +2095,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = set_work(&a, h->n_pad / kRows, p->sms);
-      a.part = p->part.as<unsigned long long>();
-      a.part_done = reinterpret_cast<unsigned int*>(a.part + part_slots * 2 * kMaxR * kRows);
+      const unsigned grid = set_work(&a, h->n_pad / kRows, p);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<true>(h->device, grid, a, st));
