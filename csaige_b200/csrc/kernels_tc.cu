@@ -1441,7 +1441,7 @@ struct TcWork {
 };
 constexpr int64_t kMinSaved = 24;
 
-TcWork tc_work(int64_t tiles, int64_t nk, int sms) {
+TcWork tc_work(int64_t tiles, int64_t nk, int sms, bool share_tiles) {
   TcWork w;
   w.grid = sms;
   w.whole = (int)(tiles / sms);
@@ -1449,7 +1449,7 @@ TcWork tc_work(int64_t tiles, int64_t nk, int sms) {
   const int64_t rest = tiles - w.tail_tile, share = ceil_div(rest * nk, (int64_t)sms);
   w.extra = 0;
   w.tail_units = 0;
-  if (rest > 0 && nk - share >= kMinSaved) {
+  if (share_tiles && rest > 0 && nk - share >= kMinSaved) {
     w.tail_units = rest * nk;
   } else {
     w.extra = (int)rest;
@@ -1832,9 +1832,10 @@ void tc_set_wait_budget(long long cycles) {
   g_tc_wait_cycles.store(cycles < 0 ? kWaitCycles : cycles, std::memory_order_relaxed);
 }
 
-// Sets the work division of a launch over `tiles` tiles; returns its grid.
-static unsigned set_work(TcArgs* a, int64_t tiles, const TcPlan* p) {
-  const TcWork w = tc_work(tiles, a->nk, p->sms);
+// Sets the work division of a launch over `tiles` tiles, which CTAs share only when there is room
+// for the sums (`share`); returns its grid.
+static unsigned set_work(TcArgs* a, int64_t tiles, const TcPlan* p, bool share) {
+  const TcWork w = tc_work(tiles, a->nk, p->sms, share);
   a->whole = w.whole;
   a->extra = w.extra;
   a->tail_tile = w.tail_tile;
@@ -1956,8 +1957,16 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     if ((a.split.blocks > 1 || b.split.blocks > 1) && !p->sr_sums.ptr) {
       const size_t bytes = (size_t)std::max(h->n_pad, h->m_pad) * 16 +
                            (size_t)std::max(blocks_a, blocks_b) * 4;
-      SG_TRY(p->sr_sums.reserve(bytes));
-      SG_CUDA(cudaMemsetAsync(p->sr_sums.ptr, 0, bytes, st));
+      const Status ss = p->sr_sums.reserve(bytes);
+      if (ss.ok()) {
+        SG_CUDA(cudaMemsetAsync(p->sr_sums.ptr, 0, bytes, st));
+      } else if (ss.code == SAIGE_ENOMEM) {  // undivided, for the same sums
+        set_error("");
+        a.split = SrSplit{n_stages_a, 1};
+        b.split = SrSplit{n_stages_b, 1};
+      } else {
+        return ss;
+      }
     }
     a.sums_g = p->sr_sums.as<unsigned long long>();
     a.sums_m = a.sums_g + std::max(h->n_pad, h->m_pad);
@@ -2019,7 +2028,14 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     h->stats.sc_list_launches += lists ? 1 : 0;
     h->n_kv += 1;
   }
-  if (!single) SG_TRY(part_reserve(p, rmax, st));
+  bool share = false;
+  if (!single) {
+    // short of memory: no tile is shared, for the same sums
+    const Status ps = part_reserve(p, rmax, st);
+    if (!ps.ok() && ps.code != SAIGE_ENOMEM) return ps;
+    if (!ps.ok()) set_error("");
+    share = ps.ok();
+  }
   for (size_t c0 = 0; c0 < (single ? 0 : cols.size()); c0 += kMaxR) {
     const int r = (int)std::min<size_t>(kMaxR, cols.size() - c0);
     const int ng = (int)round_up(3 * r, 16);
@@ -2054,7 +2070,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_ld = h->m_pad;
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = set_work(&a, h->m_pad / kRows, p);
+      const unsigned grid = set_work(&a, h->m_pad / kRows, p, share);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<false>(h->device, grid, a, st));
@@ -2095,7 +2111,7 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
       a.out_scale = 1.0 / (double)(h->masked ? h->m_active : h->m_eff);
       a.err = sc.err;
       a.trace = p->tracing ? p->trace.as<unsigned long long>() : nullptr;
-      const unsigned grid = set_work(&a, h->n_pad / kRows, p);
+      const unsigned grid = set_work(&a, h->n_pad / kRows, p, share);
       cudaEvent_t t0 = nullptr, t1 = nullptr;
       SG_TRY(mark(&t0));
       SG_TRY(launch_tc_tuned<true>(h->device, grid, a, st));
