@@ -429,11 +429,25 @@ static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
   std::vector<int> act;
   for (int c = 0; c < q; ++c)
     if (!active || active[c] == kColActive) act.push_back(c);
-  // the active columns in groups of up to kFp32Cols that share one decode of the codes
-  const size_t group = std::min<size_t>(std::max<size_t>(act.size(), 1), kFp32Cols);
-  SG_TRY(h->v32.reserve(group * h->n_pad * sizeof(float)));
-  SG_TRY(h->u32.reserve(group * h->m_pad * sizeof(float)));
-  SG_TRY(h->ypart.reserve(std::min<size_t>(group, kFp32ColsB) * h->n_splits * h->n_pad * sizeof(float)));
+  // the active columns in groups of up to kFp32Cols that share one decode of the codes; smaller
+  // ones, for the same bits, when memory is short of their scratch
+  size_t group = std::min<size_t>(std::max<size_t>(act.size(), 1), kFp32Cols);
+  auto scratch = [&]() -> Status {
+    SG_TRY(h->v32.reserve(group * h->n_pad * sizeof(float)));
+    SG_TRY(h->u32.reserve(group * h->m_pad * sizeof(float)));
+    return h->ypart.reserve(std::min<size_t>(group, kFp32ColsB) * h->n_splits * h->n_pad *
+                            sizeof(float));
+  };
+  Status room = scratch();
+  while (room.code == SAIGE_ENOMEM && group > 1) {
+    h->v32.release();
+    h->u32.release();
+    h->ypart.release();
+    group /= 2;
+    set_error("");
+    room = scratch();
+  }
+  SG_TRY(room);
   const float scale = 1.0f / (float)(h->masked ? h->m_active : h->m_eff);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->profiling) {
@@ -441,8 +455,8 @@ static Status grm_product_fp32(saige_grm* h, const double* v, double* kp, int q,
     SG_CUDA(cudaEventCreate(&e1));
     SG_CUDA(cudaEventRecord(e0, st));
   }
-  for (size_t c0 = 0; c0 < act.size(); c0 += kFp32Cols) {
-    const int nc = (int)std::min<size_t>(kFp32Cols, act.size() - c0);
+  for (size_t c0 = 0; c0 < act.size(); c0 += group) {
+    const int nc = (int)std::min<size_t>(group, act.size() - c0);
     Fp32Cols cols{};
     for (int k = 0; k < nc; ++k) {
       cols.v[k] = v + (int64_t)act[c0 + k] * h->n_pad;

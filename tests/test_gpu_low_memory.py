@@ -78,3 +78,10 @@ def test_mixed_column_without_room_for_divided_passes():
         return g
 
     _same_when_short(make, lambda g: g.mat_vec(v[0]), 4 * MB)
+
+
+def test_fp32_columns_without_room_for_a_shared_decode():
+    # 13 MB of vectors; scratch of 7 MB for a column, 31 MB for eight
+    n, m = 100000, 2000
+    v = np.random.default_rng(3).standard_normal((8, n))
+    _same_when_short(lambda: _grm(n, m, cs.PREC_FP32), lambda g: g.mat_vec(v), 30 * MB)
