@@ -286,8 +286,8 @@ __global__ void __launch_bounds__(kLiveRows)
 // row): z^2 of the four codes (00 -> 2, 10 -> 1, 11 -> 0, 01 missing -> 0) sits in shared
 // memory for kDiagChunk rows at a time, so an entry costs a
 // bit-field extract, one 8-byte lookup (four addresses per row: no bank conflicts)
-// and one FP64 add.  Block y sums the live rows [y per, (y + 1) per) into row y of partial;
-// grm_diag_finish adds the rows in order.  The ranges count live rows, so that a handle with
+// and one FP64 add.  Block y sums the (first + y)-th range of `per` live rows into row y of
+// partial; grm_diag_finish adds the rows in order.  The ranges count live rows, so that a handle with
 // markers left out forms the sums of a handle without them, to the bit.  Bound: the lookups.
 // One thread per sample over all markers (a 4-byte load per 2-bit code, one serial chain) took
 // 22.9 ms at n = 60,013, m = 39,000; this takes 0.62 ms (0.64 with the 51 registers that the
@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(kDiagThreads, 4)
     grm_diag_kernel(const uint32_t* __restrict__ geno, int64_t wpr,
                     const double* __restrict__ two_p, const double* __restrict__ inv_s,
                     const int32_t* __restrict__ rows, const int32_t* __restrict__ n_live,
-                    int64_t per, double* __restrict__ partial) {
+                    int64_t per, int64_t first, double* __restrict__ partial) {
   __shared__ double tab[kDiagChunk][4];
   __shared__ int64_t at[kDiagChunk];  // the rows' first words
   const int64_t w = (int64_t)blockIdx.x * kDiagThreads + threadIdx.x;
-  const int64_t lo = (int64_t)blockIdx.y * per;
+  const int64_t lo = (first + blockIdx.y) * per;
   const int64_t n_rows = *n_live, hi = lo + per < n_rows ? lo + per : n_rows;
   double acc[16];
 #pragma unroll
@@ -349,11 +349,12 @@ __global__ void __launch_bounds__(kDiagThreads, 4)
   for (int e = 0; e < 8; ++e) o[e] = make_double2(acc[2 * e], acc[2 * e + 1]);
 }
 
+// (more: after the ranges that out already has)
 __global__ void grm_diag_finish(const double* __restrict__ partial, int splits, int64_t n_pad,
-                                int64_t n, double scale, double* __restrict__ out) {
+                                int64_t n, bool more, double scale, double* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double s = 0.0;
+  double s = more ? out[i] : 0.0;
 #pragma unroll 4
   for (int k = 0; k < splits; ++k) s += partial[(int64_t)k * n_pad + i];
   out[i] = s * scale;
@@ -456,8 +457,16 @@ Status grm_diag(saige_grm* h, double* out, cudaStream_t st) {
   const int64_t splits = std::max<int64_t>(1, ceil_div(m_used, per));
   const int64_t blocks = std::max<int64_t>(1, ceil_div(h->m, (int64_t)kLiveRows));
   DevBuf partial, list;
-  SG_TRY(partial.reserve((size_t)splits * h->n_pad * sizeof(double)));
   SG_TRY(list.reserve((size_t)(h->m + blocks + 1) * sizeof(int32_t)));
+  // all ranges at once; when memory is short, as many at a time as fit
+  int64_t at_once = splits;
+  Status room = partial.reserve((size_t)at_once * h->n_pad * sizeof(double));
+  while (room.code == SAIGE_ENOMEM && at_once > 1) {
+    at_once = ceil_div(at_once, (int64_t)2);
+    set_error("");
+    room = partial.reserve((size_t)at_once * h->n_pad * sizeof(double));
+  }
+  SG_TRY(room);
   int32_t *rows = list.as<int32_t>(), *counts = rows + h->m, *n_live = counts + blocks;
   const uint8_t* excl = h->masked ? h->excl.as<uint8_t>() : nullptr;
   // the buffers are used on st only
@@ -465,11 +474,15 @@ Status grm_diag(saige_grm* h, double* out, cudaStream_t st) {
   live_count_kernel<<<(unsigned)blocks, kLiveRows, 0, st>>>(h->inv_s, excl, h->m, counts);
   live_list_kernel<<<(unsigned)blocks, kLiveRows, 0, st>>>(h->inv_s, excl, h->m, counts, rows,
                                                            n_live);
-  grm_diag_kernel<<<dim3((unsigned)windows, (unsigned)splits), kDiagThreads, 0, st>>>(
-      h->geno, h->wpr, h->two_p, h->inv_s, rows, n_live, per, partial.as<double>());
-  grm_diag_finish<<<(unsigned)ceil_div(h->n, 256), 256, 0, st>>>(
-      partial.as<double>(), (int)splits, h->n_pad, h->n, scale, out);
-  count_launches(4);
+  for (int64_t s0 = 0; s0 < splits; s0 += at_once) {
+    const int64_t k = std::min(at_once, splits - s0);
+    grm_diag_kernel<<<dim3((unsigned)windows, (unsigned)k), kDiagThreads, 0, st>>>(
+        h->geno, h->wpr, h->two_p, h->inv_s, rows, n_live, per, s0, partial.as<double>());
+    grm_diag_finish<<<(unsigned)ceil_div(h->n, 256), 256, 0, st>>>(
+        partial.as<double>(), (int)k, h->n_pad, h->n, s0 > 0, s0 + k == splits ? scale : 1.0, out);
+    count_launches(2);
+  }
+  count_launches(2);
   SG_CHECK_LAUNCH();
   partial.release();
   list.release();

@@ -85,3 +85,9 @@ def test_fp32_columns_without_room_for_a_shared_decode():
     n, m = 100000, 2000
     v = np.random.default_rng(3).standard_normal((8, n))
     _same_when_short(lambda: _grm(n, m, cs.PREC_FP32), lambda g: g.mat_vec(v), 30 * MB)
+
+
+def test_diagonal_without_room_for_all_ranges():
+    # 23 MB for the sums of all 47 ranges of markers
+    n, m = 60000, 6000
+    _same_when_short(lambda: _grm(n, m, cs.PREC_FP32), lambda g: g.diag(), 8 * MB)
