@@ -325,9 +325,10 @@ struct SyrkPlan {
   std::vector<SyrkItem> items;  // the first launch's, then one per slot
   int64_t first = 0, slots = 0;
 };
+// sms 0: one launch
 SyrkPlan syrk_plan(int64_t nb, int64_t nch, int sms) {
   SyrkPlan p;
-  const int64_t tiles = nb * (nb + 1) / 2, w = tiles / sms, rest = tiles % sms;
+  const int64_t tiles = nb * (nb + 1) / 2, w = sms ? tiles / sms : 0, rest = sms ? tiles % sms : 0;
   // (sms - rest): the SMs that the last of w + 1 waves would leave idle
   int64_t k = w >= 1 && rest > 0 ? ceil_div((int64_t)sms, sms - rest) : 0;
   // one launch where two would save less than a twentieth of the waves
@@ -361,15 +362,24 @@ Status run_syrk(SyrkArgs a, int64_t n, int64_t n_pad, bool packed, int32_t arith
   int dev = 0, sms = 0;
   SG_CUDA(cudaGetDevice(&dev));
   SG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const SyrkPlan plan = syrk_plan(nb, a.m_pad / kKc, sms);
+  SyrkPlan plan = syrk_plan(nb, a.m_pad / kKc, sms);
   DevBuf d_items, d_carry;
   std::vector<int2> tiles;
+  if (plan.slots > 0) {
+    const Status cs = d_carry.reserve((size_t)plan.slots * kT * kT * sizeof(double));
+    if (cs.ok()) {
+      a.carry = d_carry.as<double>();
+    } else if (cs.code == SAIGE_ENOMEM) {  // one launch, for the same sums
+      set_error("");
+      plan = syrk_plan(nb, 0, 0);
+    } else {
+      return cs;
+    }
+  }
   if (plan.slots > 0) {
     SG_TRY(d_items.reserve(plan.items.size() * sizeof(SyrkItem)));
     SG_CUDA(cudaMemcpyAsync(d_items.ptr, plan.items.data(), plan.items.size() * sizeof(SyrkItem),
                             cudaMemcpyHostToDevice, st));
-    SG_TRY(d_carry.reserve((size_t)plan.slots * kT * kT * sizeof(double)));
-    a.carry = d_carry.as<double>();
   } else {
     for (const SyrkItem& t : plan.items) tiles.push_back(make_int2(t.bi, t.bj));
     SG_TRY(d_items.reserve(tiles.size() * sizeof(int2)));

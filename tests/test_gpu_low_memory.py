@@ -91,3 +91,15 @@ def test_diagonal_without_room_for_all_ranges():
     # 23 MB for the sums of all 47 ranges of markers
     n, m = 60000, 6000
     _same_when_short(lambda: _grm(n, m, cs.PREC_FP32), lambda g: g.diag(), 8 * MB)
+
+
+def test_explicit_grm_without_room_for_shared_tiles():
+    # 528 tiles on 148 SMs: two launches, between which 148 tiles' sums take 19 MB
+    n, m = 4001, 600
+    bed = cs.gen_bed(cs.CohortSpec(n=n, m=m, seed=4, missing_rate=0.01))
+    want, used = cs.compute_sparse_grm(bed, n, m)
+    with _Taken(12 * MB):
+        got, used_short = cs.compute_sparse_grm(bed, n, m)
+    assert used_short == used
+    for a, b in ((got.rows, want.rows), (got.cols, want.cols), (got.vals, want.vals)):
+        assert np.array_equal(a, b)
