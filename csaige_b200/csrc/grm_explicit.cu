@@ -322,7 +322,8 @@ struct Events {
 // tiles' first 1/k in the time that w waves leave: w + 1 - 1/k waves in place of w + 1.
 // n = 4,001, m = 6,007 (528 tiles on 148 SMs): 4 waves in 7.15 ms, 3 2/3 in 6.71.
 struct SyrkPlan {
-  std::vector<SyrkItem> items;  // the first launch's, then one per slot
+  std::vector<int2> tiles;      // one launch, or
+  std::vector<SyrkItem> items;  // two: the first one's, then one per slot
   int64_t first = 0, slots = 0;
 };
 // sms 0: one launch
@@ -333,8 +334,15 @@ SyrkPlan syrk_plan(int64_t nb, int64_t nch, int sms) {
   int64_t k = w >= 1 && rest > 0 ? ceil_div((int64_t)sms, sms - rest) : 0;
   // one launch where two would save less than a twentieth of the waves
   if (nch < 4 * k || k * (w + 1) > 20) k = 0;
-  const int64_t whole = k ? tiles - sms : tiles;
-  const int c = k ? (int)(nch / k) : 0;
+  if (!k) {
+    p.tiles.reserve((size_t)tiles);
+    for (int64_t bi = 0; bi < nb; ++bi)
+      for (int64_t bj = bi; bj < nb; ++bj) p.tiles.push_back(make_int2((int)bi, (int)bj));
+    p.first = tiles;
+    return p;
+  }
+  const int64_t whole = tiles - sms;
+  const int c = (int)(nch / k);
   std::vector<SyrkItem> head, tail;
   for (int64_t bi = 0, at = 0; bi < nb; ++bi)
     for (int64_t bj = bi; bj < nb; ++bj, ++at) {
@@ -364,7 +372,6 @@ Status run_syrk(SyrkArgs a, int64_t n, int64_t n_pad, bool packed, int32_t arith
   SG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   SyrkPlan plan = syrk_plan(nb, a.m_pad / kKc, sms);
   DevBuf d_items, d_carry;
-  std::vector<int2> tiles;
   if (plan.slots > 0) {
     const Status cs = d_carry.reserve((size_t)plan.slots * kT * kT * sizeof(double));
     if (cs.ok()) {
@@ -381,9 +388,8 @@ Status run_syrk(SyrkArgs a, int64_t n, int64_t n_pad, bool packed, int32_t arith
     SG_CUDA(cudaMemcpyAsync(d_items.ptr, plan.items.data(), plan.items.size() * sizeof(SyrkItem),
                             cudaMemcpyHostToDevice, st));
   } else {
-    for (const SyrkItem& t : plan.items) tiles.push_back(make_int2(t.bi, t.bj));
-    SG_TRY(d_items.reserve(tiles.size() * sizeof(int2)));
-    SG_CUDA(cudaMemcpyAsync(d_items.ptr, tiles.data(), tiles.size() * sizeof(int2),
+    SG_TRY(d_items.reserve(plan.tiles.size() * sizeof(int2)));
+    SG_CUDA(cudaMemcpyAsync(d_items.ptr, plan.tiles.data(), plan.tiles.size() * sizeof(int2),
                             cudaMemcpyHostToDevice, st));
     a.tiles = d_items.as<int2>();
   }
