@@ -1230,30 +1230,44 @@ __global__ void __launch_bounds__(256)
 }
 
 // How a one-column pass divides the columns of its code tiles: `tiles` per block, `blocks`
-// blocks per row block, chosen for the shortest sum of waves x (tiles + ends), ends being what
-// a block's first loads and last sums cost in tiles (more where partial sums meet), fitted to
-// the times below.  A cohort's row blocks alone neither fill the SMs (n = 9,001: 36 in pass B)
-// nor come in whole waves.  us undivided / with pass B divided into 12 blocks per SM / now:
-//                         pass A        pass B
-//   200,000 x 148,979     1808 / -  / 1823   -  / 1847 / 1788
-//   100,000 x  49,000      348 / -  /  324   -  /  320 /  305
-//     9,001 x  21,011     20.0 / -  / 20.4   -  / 27.6 / 18.3
-//    30,000 x   9,033     23.3 / -  / 24.8   -  / 35.9 / 25.0
-//     2,000 x   4,077      4.0 / -  /  4.1   -  /  5.8 /  6.0
+// blocks per row block, chosen for the shortest sum of waves x (tiles + ends), plus `meet` where
+// partial sums meet; ends is what a block's first loads and last sums cost, in tiles.  A cohort's
+// row blocks alone neither fill the SMs (n = 9,001: 36 in pass B) nor come in whole waves.
+// `resident`, blocks that an SM takes in the time of one: in pass A two take as long as one after
+// the other, since the eight warps of one block keep the integer pipe busy; in pass B, where a
+// warp has every second column tile, two take less.  Fitted to every division of 30 sizes from
+// 1,000 x 108 to 200,000 x 19,022: within 0.4 % (A, 3 % at most) and 0.9 % (B, 7.5 % at most) of the
+// best division on average, against 2.5 % and 3.8 % (31 % and 68 % at most) with waves of two blocks per
+// SM in both passes and nothing for the meeting.  us undivided / that rule / this one:
+//                        pass A              pass B
+//   100,000 x 49,000   352 / 326 / 327     343 / 309 / 309
+//    20,000 x 48,995  77.3 / 77.4 / 77.4   122 / 72.3 / 70.5
+//     9,001 x 21,010  20.4 / 20.6 / 20.6  53.9 / 18.3 / 18.5
+//     5,000 x  7,053   6.1 /  8.3 /  6.3  20.0 /  7.5 /  7.5
+//    30,000 x  2,138  21.4 / 10.2 / 10.1   8.3 / 10.8 /  8.4
+//     3,000 x    750   4.6 /  5.6 /  4.7   4.5 /  5.1 /  4.6
+//     2,000 x  4,081   4.0 /  4.0 /  4.0  12.4 /  5.9 /  5.9
 struct SrSplit {
   int64_t tiles;
   unsigned blocks;
 };
 
-SrSplit sr_split(int64_t row_blocks, int64_t n_kt, int sms, int64_t ends, int64_t ends_split) {
-  const int64_t slots = 2 * (int64_t)sms;  // two blocks per SM are resident
+struct SrCost {
+  int resident;
+  int64_t ends, ends_divided, meet;
+};
+constexpr SrCost kSrCostA{1, 2, 10, 16}, kSrCostB{2, 4, 4, 8};
+
+SrSplit sr_split(int64_t row_blocks, int64_t n_kt, int sms, const SrCost& cost) {
+  const int64_t slots = (int64_t)cost.resident * sms;
   SrSplit best{n_kt, 1};
-  int64_t least = ceil_div(row_blocks, slots) * (n_kt + ends);
+  int64_t least = ceil_div(row_blocks, slots) * (n_kt + cost.ends);
   for (int64_t b = 2; b <= std::min<int64_t>(n_kt, 64); ++b) {
     const int64_t tiles = ceil_div(n_kt, b), blocks = ceil_div(n_kt, tiles);
-    const int64_t cost = ceil_div(row_blocks * blocks, slots) * (tiles + ends_split);
-    if (cost < least) {
-      least = cost;
+    const int64_t c =
+        ceil_div(row_blocks * blocks, slots) * (tiles + cost.ends_divided) + cost.meet;
+    if (c < least) {
+      least = c;
       best = SrSplit{tiles, (unsigned)blocks};
     }
   }
@@ -1951,9 +1965,9 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     const unsigned blocks_a = (unsigned)(h->m_pad / kSrRowsA);
     const unsigned blocks_b = (unsigned)(h->n_pad / kSrRowsB);  // (n_pad: a multiple of 512)
     SrArgs a{};
-    a.split = sr_split(blocks_a, n_stages_a, p->sms, 12, 26);
+    a.split = sr_split(blocks_a, n_stages_a, p->sms, kSrCostA);
     SrArgs b{};
-    b.split = sr_split(blocks_b, n_stages_b, p->sms, 5, 5);
+    b.split = sr_split(blocks_b, n_stages_b, p->sms, kSrCostB);
     if ((a.split.blocks > 1 || b.split.blocks > 1) && !p->sr_sums.ptr) {
       const size_t bytes = (size_t)std::max(h->n_pad, h->m_pad) * 16 +
                            (size_t)std::max(blocks_a, blocks_b) * 4;
