@@ -186,8 +186,8 @@ class ClockSampler:
 
 def single_column_modes(grm, n: int, reps: int = 4) -> dict:
     """Device ms per one-column product on the bench's handle (after its timed fits) with
-    the dense missing-flag sums (SAIGE_SR_LISTS=0) and by the library's own rule (the
-    missing-call lists, where they are the cheaper): the same products to the bit."""
+    the dense missing-flag sums (SAIGE_SR_LISTS=0) and by the library's own rule (which lists
+    the missing calls of small handles only): the same products to the bit."""
     import numpy as np
 
     v = np.random.default_rng(3).standard_normal((1, n))

@@ -899,8 +899,7 @@ __global__ void __launch_bounds__(128)
 // one column costs nearly what 42 do.  These kernels form the same exact integer sums and
 // apply the same FP64 epilogue, so their results are bit-identical to the block path's.
 // With the missing-call lists of the handle (miss_lists.cuh) the flag sums give way to int64
-// sums over the ~1 % missing calls, a third fewer instructions per entry for the same
-// integers.
+// sums over the missing calls, for the same integers.
 //
 // What bounds it: the unpack (four masks and four byte permutes per 16 entries, and four
 // more for the flags), then HBM (7.5 GB of codes at 200,000 x 150,000: 1.15 ms per pass).
@@ -1488,19 +1487,30 @@ struct TcPlan {
 // Bytes of the counts of the tiles that CTAs share.
 static size_t part_counts(const TcPlan* p) { return (size_t)round_up((int64_t)p->sms * 4, 256); }
 
-// The missing-call lists cost about two products' time to build (four passes over the
-// codes) and 8 bytes per missing call, while a fit runs four or five one-column products:
-// a handle counts its missing calls at the first one-column product of its second AI-REML
-// fit, and lists them if the lists are then the cheaper of the two.  The flags cost about
-// 0.5 ms per pass at 200,000 x 148,979 whatever the calls; the lists 1.1-1.4 ms at 1 %
-// missing, in proportion to the calls (9,001 x 21,011: 28 and 25 us against 20 and 18): the
-// line is 0.3 %.  In handles of a few million entries the launch is most of either (3,000 x
-// 779 at 1 %: 5.6 + 6.4 us against 4.7 + 5.1), and the lists are kept, as their statistics
-// report them.
-// SAIGE_SR_LISTS: 0 keeps the dense missing-flag sums, 2 builds the lists at a handle's
-// first one-column product, otherwise (default) by the rule above.
+// When a handle lists its missing calls.  The lists take about two products' time to build (four
+// passes over the codes) and 8 bytes per missing call, and the products with them are not the
+// faster ones.  us per pass, A + B, with the flags / with the lists of that many missing calls:
+//                        flags          0.1 %          1 %
+//   200,000 x 148,988  1831 + 1802   2157 + 2111   2634 + 2672
+//    50,000 x  98,979   325 +  312    385 +  367
+//     9,001 x  21,010  20.7 + 18.5   25.9 + 20.9   32.9 + 25.1
+//     3,000 x   3,105   4.7 +  5.9    5.1 +  6.2
+//     3,000 x     750   4.7 +  4.6    5.2 +  4.9    6.0 +  6.0
+// (with no call missing at all 1978 + 1920 at the first size: the staging of the values and the
+// barriers around it.)  So large handles keep the flags.  Small ones, where a product loses at
+// most 3 us, list their calls from the second AI-REML fit on, at its first one-column product, as
+// they always have and as their statistics say (saige_grm_stats: missing_listed).
+// SAIGE_SR_LISTS: 0 keeps the flag sums, 2 builds the lists at a handle's first one-column
+// product (up to kMissListMaxFrac missing), otherwise (default) by this rule.
+constexpr int64_t kSrListSmall = (int64_t)1 << 22;  // entries: up to kMissListMaxFrac missing
+constexpr int64_t kSrListMost = (int64_t)1 << 24;   // up to kSrListFrac; above, none
 constexpr double kSrListFrac = 0.003;
-constexpr int64_t kSrListSmall = (int64_t)1 << 22;
+
+// The largest fraction of missing calls that the default lists (0: none).
+static double sr_list_frac(const saige_grm* h) {
+  const int64_t entries = h->m_pad * h->n_pad;
+  return entries <= kSrListSmall ? kMissListMaxFrac : (entries <= kSrListMost ? kSrListFrac : 0.0);
+}
 
 static int sr_lists_mode() {
   const char* e = getenv("SAIGE_SR_LISTS");
@@ -1938,13 +1948,12 @@ Status tc_product(saige_grm* h, const double* v, double* kp, int q, const int32_
     int8_t* planes_b = p->img_w.as<int8_t>();  // 6 x m_pad limb planes of qw, qc
     double* u = p->u.as<double>();
     const int lmode = sr_lists_mode();
-    if ((p->miss.state == 0 && (lmode == 2 || (lmode == 1 && h->n_fits >= 2))) ||
+    const double frac = lmode == 2 ? kMissListMaxFrac : (lmode == 1 ? sr_list_frac(h) : 0.0);
+    if ((p->miss.state == 0 && (lmode == 2 || (frac > 0.0 && h->n_fits >= 2))) ||
         (p->miss.state == kMissListsLeft && lmode == 2))
       SG_TRY(miss_lists_build(
           h, p->tiles_s.as<uint8_t>(), p->s_ld,
-          MissShape{kSrRowsA, kSrChunkA / 16, kSrRowsB, kSrChunkB},
-          lmode == 2 || h->m_pad * h->n_pad <= kSrListSmall ? kMissListMaxFrac : kSrListFrac,
-          &p->miss, st));
+          MissShape{kSrRowsA, kSrChunkA / 16, kSrRowsB, kSrChunkB}, frac, &p->miss, st));
     const bool lists = p->miss.state == 1 && lmode != 0;
     int32_t *qv32 = nullptr, *qc32 = nullptr;
     if (lists) {

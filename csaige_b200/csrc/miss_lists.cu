@@ -5,9 +5,9 @@
 // (kernels_tc.cu).  The dense missing-flag sums cost a second unpack and a second set of
 // matrix instructions for a sum over a few entries.  With these lists the one-column kernels
 // form Mi instead as an exact int64 sum of the quantised vector over each row's missing
-// calls, read from the chunk of the vector they hold in shared memory: cheaper up to about
-// 0.3 % of the calls missing.  The integer is the one the dense sums form, so the products
-// do not change by a bit.
+// calls, read from the chunk of the vector they hold in shared memory.  The integer is the one
+// the dense sums form, so the products do not change by a bit.  They are no longer faster (see the
+// rule in kernels_tc.cu); small handles build them by default.
 #include <algorithm>
 #include <vector>
 

@@ -465,10 +465,10 @@ typedef struct {
                               /* over the missing calls in place of dense    */
                               /* flag sums, the same integers; built at the  */
                               /* first such product of the handle's second   */
-                              /* fit, where at most 0.3 % of the calls are   */
-                              /* missing or the handle is small (env         */
-                              /* SAIGE_SR_LISTS=2: at its first product,     */
-                              /* =0: never)                                  */
+                              /* fit, where the handle is small (up to 2^22  */
+                              /* entries; up to 2^24 with at most 0.3 % of   */
+                              /* the calls missing; env SAIGE_SR_LISTS=2: in */
+                              /* any handle at its first product, =0: never) */
   int64_t missing_listed;     /* missing calls in the handle's lists; -1     */
                               /* while none are built or when declined       */
                               /* (over 3 % of the calls missing, or too      */
