@@ -164,7 +164,7 @@ __global__ void combo_kernel(const double* __restrict__ V, int m, const double* 
     if (c0 + c < q) Y[(int64_t)(c0 + c) * ld + i] = acc[c];
 }
 
-// out may be kv (each element is read before it is written by the same thread)
+// out = tau0 v / wmax + tau1 kv, and v and kv copied beside it; no output overlaps an input.
 __global__ void sigma_image_kernel(const double* __restrict__ v, const double* __restrict__ kv,
                                    const double* __restrict__ wmax, double tau0, double tau1,
                                    double* __restrict__ v_out, double* __restrict__ kv_out,
