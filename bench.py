@@ -55,9 +55,9 @@ REF_KV_PER_FIT = 929
 CPU_SAMPLE_MARKERS = 32768
 # DRAM bytes read per marker row by one tensor-core launch (packed genotype tile rows
 # plus the vector-limb tiles), from the ncu capture at N=200,000, m_pad=17,280:
-# pass A 923.9 MB, pass B 904.8 MB.  Reads scale with m_pad; the output writes
+# pass A 926.1 MB, pass B 905.4 MB.  Reads scale with m_pad; the output writes
 # (pass A: m_pad*R*8 bytes, pass B: N*R*8 bytes) are added per launch.
-TC_READ_PER_MARKER_ROW = {"A": 923.9e6 / 17280, "B": 904.8e6 / 17280}
+TC_READ_PER_MARKER_ROW = {"A": 926.1e6 / 17280, "B": 905.4e6 / 17280}
 
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # The plain CPU-scale fit-null cohort (the reference's own benchmark size): N = 2,000,

@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(128)
 // The unpacked bytes stay in registers: they are the A fragments of mma.m16n8k32 over the
 // three limb columns of q (one instruction for 16 x 32 entries), which a tcgen05.mma would
 // want stored to TMEM or shared memory first.  Formed with dp4a (three per four entries and
-// accumulator) the sums took 2.7 and 3.1 ms per pass at 200,000 x 148,979; now 1.82 and 1.79
+// accumulator) the sums took 2.7 and 3.1 ms per pass at 200,000 x 148,979; now 1.83 and 1.80
 // (1.31 without the flags).
 // ---------------------------------------------------------------------------
 // prmt tables of the NEGATED genotype (codes 00, 01, 10, 11 -> -2, 0, -1, 0) and of
